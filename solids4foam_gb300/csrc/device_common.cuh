@@ -53,6 +53,9 @@ struct MeshView {
   // doubles in, followed by the groups' arrival counters (unsigned)
   long locGrpOff;
   int locGroups;
+  // row -> its position in the PCG vectors x and r (the cluster-resident
+  // PCG's order); null: the storage order
+  const int* pcgPos;
 };
 
 // Batched launches: the case's boundary values (bval [case][nB][3],

@@ -106,6 +106,13 @@ struct EventTimer : LaunchTimer {
   }
 };
 
+// Largest meshes of the cluster-resident PCG, in rows per CTA of a full cluster,
+// by where the separate kernels are as fast.  Exact DIC: as many as the row
+// vector's memory holds.
+template <typename T>
+constexpr int kResMaxRows(bool local) { return !local ? 16000 : sizeof(T) == 4 ? 2048 : 1280; }
+constexpr int kResMaxDiagRows = 16384;
+
 struct Engine {
   Ctx* ctx = nullptr;
   HostPrep hp;
@@ -144,6 +151,24 @@ struct Engine {
   bool tuned64 = false, tuned32 = false;
   bool autotune = true;
   double tuneUs[2][kLocNumNT + kLocNumU] = {};  // last timings (us), for perf
+  // cluster-resident PCG (kernels_resident.cu), per value type: the plan, made
+  // at the first solve of that type, and its tables
+  template <typename T>
+  struct Resident {
+    bool tried = false, ok = false, valid = false;
+    int precond = -1;
+    int placeMany = 0;  // ResView::place when several solves run at once
+    int* pos = nullptr;
+    ResView rv{};
+    ResPtrs<T> rp{};
+  };
+  Resident<double> res64;
+  Resident<float> res32;
+  template <typename T>
+  Resident<T>& resident() {
+    if constexpr (sizeof(T) == 4) return res32;
+    else return res64;
+  }
   DevState* dState = nullptr;  // one per load case ([caseCap])
   DevState* hState = nullptr;  // pinned mirror
   int caseCap = 1;             // load cases the per-case arrays hold
@@ -605,8 +630,226 @@ struct Engine {
     matrixValid = true;
     matrixPrecond = pre;
     fp32Valid = false;
+    res64.valid = res32.valid = false;
     return S4G_OK;
   }
+
+  // The cluster-resident PCG of value type T: true if this mesh runs it.
+  // Rows of at most kResW neighbours and a row vector that fits the cluster's
+  // shared memory; the profiled context keeps the separate kernels, whose
+  // times it reports.
+  template <typename T>
+  s4g_status ensureResident() {
+    Resident<T>& q = resident<T>();
+    if (ctx->profile) return S4G_OK;
+    cudaStream_t s = ctx->stream;
+    if (!q.tried) {
+      q.tried = true;
+      S4G_TRY(planResident<T>(q));
+    }
+    const int pre = lin.preconditioner == S4G_PRECOND_DIC ? 0 : 1;
+    if (!q.ok || (q.valid && q.precond == pre)) return S4G_OK;
+    launchResTables<T>(mv, q.rv, q.pos, dVal, dDiag, dRD, dRDa, pre != 0, q.rp, s);
+    launches++;
+    S4G_CUDA(cudaGetLastError());
+    q.valid = true;
+    q.precond = pre;
+    return S4G_OK;
+  }
+
+  template <typename T>
+  s4g_status planResident(Resident<T>& q) {
+    const int nC = hp.nC;
+    for (int r = 0; r < nC; ++r)
+      if (hp.rowptr[r + 1] - hp.rowptr[r] > kResW) return S4G_OK;
+    int maxSmem = 0;
+    S4G_CUDA(cudaDeviceGetAttribute(&maxSmem, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+    const size_t limit = (size_t)maxSmem - 1024;  // beside the kernel's static shared memory
+    ResView& rv = q.rv;
+    rv.local = mv.subdomains;
+    rv.C = 1;
+    rv.nLev = hp.globalLevels;
+    rv.maxRows = 4;
+    rv.uRows = (nC + 3) / 4 * 4 + 4;
+    rv.ring = kResThreads;
+    // Exact DIC: the substitutions inside one CTA where all rows fit its memory
+    // (a level costs the CTA's barrier, not the cluster's).  Rows per CTA: a
+    // level's cost hardly depends on them, the other phases' time does, and
+    // FP64 arithmetic (2 multiply-adds per cycle and SM) more than FP32's.
+    rv.single = !rv.local && resSmemBytes<T>(rv, 0) <= limit;
+    const int rows = sizeof(T) == 8 || !rv.local ? 256 : 1024;
+    rv.C = std::max(1, std::min({kResMaxCtas, (nC + rows - 1) / rows,
+                                 rv.local ? hp.nParts : kResMaxCtas}));
+    if (nC > kResMaxCtas * kResMaxRows<T>(rv.local)) return S4G_OK;
+    // rows by CTA and level
+    std::vector<int> chunk(rv.C + 1, 0), lvl, pos(nC);
+    if (rv.local) {
+      rv.nLev = hp.maxLocalLevels;
+      std::vector<int> first(rv.C + 1, hp.nParts);  // first part of each CTA
+      first[0] = 0;
+      for (int c = 1, p = 0; c < rv.C; ++c) {
+        // the part boundary nearest an even share, one part at least each
+        const long want = (long)nC * c / rv.C;
+        p = std::max(p + 1, first[c - 1] + 1);
+        while (p < hp.nParts - (rv.C - c) &&
+               std::labs(hp.partStart[p + 1] - want) <= std::labs(hp.partStart[p] - want))
+          ++p;
+        first[c] = p;
+      }
+      for (int c = 0, at = 0; c < rv.C; ++c) {
+        chunk[c] = at;
+        for (int l = 0; l < rv.nLev; ++l) {
+          lvl.push_back(at - chunk[c]);
+          for (int p = first[c]; p < first[c + 1]; ++p) {
+            const int q0 = hp.lvlOff[p] + l;
+            if (q0 >= hp.lvlOff[p + 1]) continue;
+            for (int r = hp.lvlStart[q0]; r < hp.lvlStart[q0 + 1]; ++r) pos[r] = at++;
+          }
+        }
+        lvl.push_back(at - chunk[c]);
+      }
+    } else {
+      // levels of the whole lower-triangular DAG; each split evenly
+      std::vector<int> lev(nC, 0);
+      int nLev = 1;
+      for (int r = 0; r < nC; ++r) {
+        int l = 0;
+        for (int e = hp.rowptr[r]; e < hp.rowptr[r + 1] && hp.col[e] < r; ++e)
+          l = std::max(l, lev[hp.col[e]] + 1);
+        lev[r] = l;
+        nLev = std::max(nLev, l + 1);
+      }
+      rv.nLev = nLev;
+      std::vector<int> start(nLev + 1, 0), rows(nC);
+      for (int r = 0; r < nC; ++r) ++start[lev[r] + 1];
+      for (int l = 0; l < nLev; ++l) start[l + 1] += start[l];
+      std::vector<int> fill(start.begin(), start.end() - 1);
+      for (int r = 0; r < nC; ++r) rows[fill[lev[r]]++] = r;
+      if (!rv.single) {
+        // each level in the order of where its rows' lower neighbours stand in
+        // theirs, so that most of them are in the same CTA
+        std::vector<float> at(nC, 0.0f);
+        for (int l = 0; l < nLev; ++l) {
+          const int n = start[l + 1] - start[l];
+          auto b = rows.begin() + start[l];
+          if (l > 0) {
+            for (int k = 0; k < n; ++k) {
+              const int r = b[k];
+              float sum = 0;
+              int m = 0;
+              for (int e = hp.rowptr[r]; e < hp.rowptr[r + 1] && hp.col[e] < r; ++e, ++m) sum += at[hp.col[e]];
+              at[r] = sum / (float)m;
+            }
+            std::sort(b, b + n, [&](int x, int y) { return at[x] != at[y] ? at[x] < at[y] : x < y; });
+          }
+          for (int k = 0; k < n; ++k) at[b[k]] = ((float)k + 0.5f) / (float)n;
+        }
+      }
+      if (rv.single) {
+        for (int k = 0; k < nC; ++k) pos[rows[k]] = k;
+        for (int c = 0; c < rv.C; ++c) chunk[c] = (int)((long)nC * c / rv.C);
+        lvl = start;
+      }
+      for (int c = 0, at = 0; c < rv.C && !rv.single; ++c) {
+        chunk[c] = at;
+        for (int l = 0; l < nLev; ++l) {
+          lvl.push_back(at - chunk[c]);
+          const long n = start[l + 1] - start[l];
+          for (long k = n * c / rv.C; k < n * (c + 1) / rv.C; ++k) pos[rows[start[l] + k]] = at++;
+        }
+        lvl.push_back(at - chunk[c]);
+      }
+    }
+    chunk[rv.C] = nC;
+    rv.maxRows = 0;
+    for (int c = 0; c < rv.C; ++c) rv.maxRows = std::max(rv.maxRows, chunk[c + 1] - chunk[c]);
+    rv.maxRows = (rv.maxRows + 3) / 4 * 4;
+    if (!rv.single) rv.uRows = rv.maxRows + 4;
+    // more than three lower or three upper entries of a sweep in some row
+    bool more = false;
+    for (int r = 0; r < nC && !more; ++r) {
+      int lo = 0, hi = nC, n[2] = {0, 0};
+      if (rv.local) {
+        if (hp.locSlots) break;
+        const int part = (int)(std::upper_bound(hp.partStart.begin(), hp.partStart.end(), r) -
+                               hp.partStart.begin()) - 1;
+        lo = hp.partStart[part];
+        hi = hp.partStart[part + 1];
+      }
+      for (int e = hp.rowptr[r]; e < hp.rowptr[r + 1]; ++e)
+        if (hp.col[e] >= lo && hp.col[e] < hi) ++n[hp.col[e] > r];
+      more = n[0] > 3 || n[1] > 3;
+    }
+    // the widest level of a CTA decides how many threads walk the levels, and
+    // whether the short forms of the substitutions do
+    int wide = 1;
+    for (size_t l = 0; l + 1 < lvl.size(); ++l) wide = std::max(wide, lvl[l + 1] - lvl[l]);
+    const bool inside = rv.local || rv.single;  // the levels end with a CTA's barrier
+    rv.more = more ? 1 : 0;
+    rv.wide = wide > kResThreads ? 1 : 0;
+    if (rv.wide) rv.more = 1;  // (the form for wide levels reads the second entries' flag)
+    rv.split = sizeof(T) == 8 && 3 * wide <= kResThreads ? 1 : 0;
+    rv.walk = inside ? (std::min(kResThreads, (rv.split ? 3 : 1) * wide) + 31) / 32 * 32 : kResThreads;
+    rv.ring = ((rv.split ? rv.walk / 3 : rv.walk) + 3) / 4 * 4;
+    rv.place = resPlacement<T>(rv, limit);
+    if (rv.place < 0) return S4G_OK;
+    // with others at the same time: room for a second CTA on the SM, if that
+    // leaves the sweep tables in shared memory
+    q.placeMany = resPlacement<T>(rv, limit / 2 - 1024);
+    if (!(q.placeMany & 2)) q.placeMany = rv.place;
+    int clusters = 0;
+    const cudaError_t e = resPrepare<T>(rv, &clusters);
+    if (e != cudaSuccess || clusters < 1) {
+      cudaGetLastError();
+      return S4G_OK;
+    }
+    int *dChunk, *dLvl;
+    uint32_t *col, *cnt;
+    T *val, *dg, *rd;
+    const size_t nE = (size_t)kResW * nC;
+    S4G_TRY(upload(&dChunk, chunk));
+    S4G_TRY(upload(&dLvl, lvl));
+    S4G_TRY(upload(&q.pos, pos));
+    S4G_TRY(alloc(&col, nE)); S4G_TRY(alloc(&cnt, (size_t)nC)); S4G_TRY(alloc(&val, nE));
+    S4G_TRY(alloc(&dg, (size_t)nC)); S4G_TRY(alloc(&rd, (size_t)nC));
+    q.rp.val = val; q.rp.diag = dg; q.rp.rD = rd;
+    for (int k = 0; k < (rv.more ? 4 : 2); ++k) {
+      ResSweepTab<T>& tb = k < 2 ? q.rp.sweep[k] : q.rp.more[k - 2];
+      typename ResSweepTab<T>::Q* a;
+      typename ResSweepTab<T>::R* b;
+      S4G_TRY(alloc(&a, (size_t)nC)); S4G_TRY(alloc(&b, (size_t)nC));
+      tb.q = a; tb.r = b;
+    }
+    S4G_CUDA(cudaStreamSynchronize(ctx->stream));  // the host arrays end here
+    rv.chunk = dChunk; rv.lvl = dLvl; rv.col = col; rv.cnt = cnt;
+    q.ok = true;
+    return S4G_OK;
+  }
+
+  // The mesh as the field passes of a solve of type T see it: with the
+  // resident PCG's row order, where that runs.
+  template <typename T>
+  MeshView fieldView() {
+    MeshView v = mv;
+    if (runsResident<T>()) v.pcgPos = resident<T>().pos;
+    return v;
+  }
+  // The diagonal preconditioner's iteration has no levels to walk: past some
+  // rows the whole device's row kernels are faster than one cluster.
+  template <typename T>
+  bool runsResident() {
+    return !ctx->profile && resident<T>().ok &&
+           (lin.preconditioner == S4G_PRECOND_DIC || hp.nC <= kResMaxDiagRows);
+  }
+  template <typename T>
+  cudaError_t resPcg(const Controls& c, const PcgPtrs<T>& p) {
+    const Resident<T>& q = resident<T>();
+    ResView rv = q.rv;
+    const bool many = nRun > 1 || batched;
+    if (many) rv.place = q.placeMany;
+    return launchResPcg<T>(mv, c, rv, q.rp, p, dState, ctx->stream, nRun, many);
+  }
+  bool batched = false;  // capturing this mesh's loop into a batch's graph
 
   // FP32 copies of the matrix, factor and work vectors (mixed precision).
   s4g_status ensureFp32() {
@@ -778,6 +1021,7 @@ struct Engine {
     S4G_TRY(ensureMatrix());
     const bool mixed = precision == S4G_FP32_REFINE;
     if (mixed) S4G_TRY(ensureFp32());
+    S4G_TRY(mixed ? ensureResident<float>() : ensureResident<double>());
     {
       const Controls ct = controls(0);
       if (mixed) S4G_TRY(tuneLocal<float>(ct, pc32));
@@ -883,6 +1127,7 @@ struct Engine {
   template <typename T>
   s4g_status tuneLocal(const Controls& c, const PcgPtrs<T>& p) {
     bool& done = sizeof(T) == 4 ? tuned32 : tuned64;
+    if (runsResident<T>()) return S4G_OK;  // nothing to choose
     if (done || !autotune) { done = true; return S4G_OK; }
     cudaStream_t s = ctx->stream;
     const size_t n3 = 3 * (size_t)hp.nC;
@@ -1003,6 +1248,7 @@ struct Engine {
   //   loop count = 0; cond(correctors) = any case live
   //   WHILE correctors: right-hand side; cond(pcg) = any component active
   //                     WHILE pcg: one PCG iteration; cond(pcg)
+  //                       (or the cluster-resident PCG in one launch)
   //                     post-solve pass; cond(correctors)
   // Each loop is also bounded on the device (nCorrectors + 4 correctors,
   // maxIter + 4 PCG iterations per corrector).
@@ -1010,8 +1256,10 @@ struct Engine {
   bool buildLoopGraph(cudaGraph_t g, const Controls& c, int tl, const PcgPtrs<T>& p, int grid) {
     cudaStream_t s = ctx->stream;
     const cudaStreamCaptureMode mode = cudaStreamCaptureModeThreadLocal;
-    cudaGraphConditionalHandle hOut, hPcg;
-    if (cudaGraphConditionalHandleCreate(&hOut, g, 0, cudaGraphCondAssignDefault) != cudaSuccess ||
+    cudaGraphConditionalHandle hOut, hPcg{};
+    if (cudaGraphConditionalHandleCreate(&hOut, g, 0, cudaGraphCondAssignDefault) != cudaSuccess)
+      return false;
+    if (!runsResident<T>() &&
         cudaGraphConditionalHandleCreate(&hPcg, g, 0, cudaGraphCondAssignDefault) != cudaSuccess)
       return false;
     const unsigned outerLimit = (unsigned)c.nCorr + 4, pcgLimit = (unsigned)c.maxIter + 4;
@@ -1023,12 +1271,20 @@ struct Engine {
     ok = cudaStreamEndCapture(s, &ended) == cudaSuccess && ok;
     if (!ok || cudaStreamBeginCaptureToGraph(s, outerBody, nullptr, nullptr, 0, mode) != cudaSuccess)
       return false;
-    launchRhs<T>(mv, c, f, p.x, p.r, dState, dPartials, s, nullptr, nRun);
-    launchSetLoopCond(hPcg, dState, nRun, 0, 1, pcgLimit, s);
-    ok = addWhile(s, hPcg, &pcgBody);
-    launchPost<T>(mv, c, f, p.x, dState, dPartials, 1, s, nullptr, nRun, p.p, p.p2);
+    const MeshView fv = fieldView<T>();
+    const bool res = runsResident<T>();
+    launchRhs<T>(fv, c, f, p.x, p.r, dState, dPartials, s, nullptr, nRun);
+    if (res) {
+      // the PCG loop of the corrector is one launch
+      ok = resPcg<T>(c, p) == cudaSuccess;
+    } else {
+      launchSetLoopCond(hPcg, dState, nRun, 0, 1, pcgLimit, s);
+      ok = addWhile(s, hPcg, &pcgBody);
+    }
+    launchPost<T>(fv, c, f, p.x, dState, dPartials, 1, s, nullptr, nRun, p.p, p.p2);
     launchSetLoopCond(hOut, dState, nRun, 1, 0, outerLimit, s);
     ok = cudaStreamEndCapture(s, &ended) == cudaSuccess && ok;
+    if (res) return ok && cudaGetLastError() == cudaSuccess;
     if (!ok || cudaStreamBeginCaptureToGraph(s, pcgBody, nullptr, nullptr, 0, mode) != cudaSuccess)
       return false;
     long long dummy = 0;
@@ -1072,6 +1328,11 @@ struct Engine {
   s4g_status pcgLoop(const Controls& c, const PcgPtrs<T>& p, int grid) {
     // Iterations are launched in growing batches; the launches after the
     // device's stop decision return at once.
+    if (runsResident<T>()) {
+      S4G_CUDA(resPcg<T>(c, p));
+      launches++;
+      return readState();
+    }
     int chunk = 2, launched = 0;
     pcgBase.resize(nRun);
     for (int cs = 0; cs < nRun; ++cs) pcgBase[cs] = hState[cs].pcgIter;
@@ -1125,18 +1386,20 @@ struct Engine {
         S4G_TRY(readState());
         const bool local = mv.subdomains && c.precond == 0;
         const long long perIt = local ? (tuning<T>().uIdx == 2 ? 3 : 2) : (c.precond == 0 ? 5 : 4);
+        const bool res = runsResident<T>();
         launches += 1 + (long long)(hState->nCorrDone - corr0) * (tl ? 6 : 5) +
-                    (long long)(hState->pcgIter - it0) * (perIt + 1);
+                    (res ? 0 : (long long)(hState->pcgIter - it0) * (perIt + 1));
         ranOnDevice = true;
         return S4G_OK;
       }
     }
+    const MeshView fv = fieldView<T>();
     for (;;) {
-      launchRhs<T>(mv, c, f, p.x, p.r, dState, dPartials, s, tm(), nRun);
+      launchRhs<T>(fv, c, f, p.x, p.r, dState, dPartials, s, tm(), nRun);
       launches += 2;
       S4G_TRY(readState());
       if (anyCase(&DevState::pcgContinue)) S4G_TRY(pcgLoop<T>(c, p, grid));
-      launchPost<T>(mv, c, f, p.x, dState, dPartials, 1, s, tm(), nRun, p.p, p.p2);
+      launchPost<T>(fv, c, f, p.x, dState, dPartials, 1, s, tm(), nRun, p.p, p.p2);
       launches += tl ? 3 : 2;
       S4G_CUDA(cudaGetLastError());
       S4G_TRY(readState());
@@ -1175,6 +1438,7 @@ struct Engine {
     S4G_TRY(ensureMatrix());
     const bool mixed = precision == S4G_FP32_REFINE;
     if (mixed) S4G_TRY(ensureFp32());
+    S4G_TRY(mixed ? ensureResident<float>() : ensureResident<double>());
     cudaEvent_t e0, e1;
     S4G_CUDA(cudaEventCreate(&e0));
     S4G_CUDA(cudaEventCreate(&e1));
@@ -1305,6 +1569,7 @@ struct Engine {
     S4G_TRY(ensureMatrix());
     const bool mixed = precision == S4G_FP32_REFINE;
     if (mixed) S4G_TRY(ensureFp32());
+    S4G_TRY(mixed ? ensureResident<float>() : ensureResident<double>());
     if (mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC) {
       const Controls ct = controls(0);
       if (mixed) S4G_TRY(tuneLocal<float>(ct, pc32));
@@ -1326,8 +1591,11 @@ struct Engine {
   }
   bool batchCapture(cudaGraph_t g) {
     const Controls c = controls(0);
-    return precision == S4G_FP32_REFINE ? buildLoopGraph<float>(g, c, 0, pc32, sweepGrid32)
-                                        : buildLoopGraph<double>(g, c, 0, pc, sweepGrid);
+    batched = true;
+    const bool ok = precision == S4G_FP32_REFINE ? buildLoopGraph<float>(g, c, 0, pc32, sweepGrid32)
+                                                 : buildLoopGraph<double>(g, c, 0, pc, sweepGrid);
+    batched = false;
+    return ok;
   }
   s4g_status batchFinish(double* Dout, double* sigOut, s4g_perf* perf, float ms) {
     cudaStream_t s = ctx->stream;
@@ -1336,7 +1604,9 @@ struct Engine {
     const bool local = mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC;
     const long long perIt = local ? (tuning32or64().uIdx == 2 ? 3 : 2)
                                   : (lin.preconditioner == S4G_PRECOND_DIC ? 5 : 4);
-    launches += 1 + (long long)hState->nCorrDone * 5 + (long long)hState->pcgIter * (perIt + 1);
+    const bool res = precision == S4G_FP32_REFINE ? runsResident<float>() : runsResident<double>();
+    launches += 1 + (long long)hState->nCorrDone * 5 +
+                (res ? 0 : (long long)hState->pcgIter * (perIt + 1));
     if (Dout) {
       launchGather(hp.nC, 3, dC2s, f.D[hState->dcur], dOut, s);
       S4G_CUDA(cudaMemcpyAsync(Dout, dOut, sizeof(double) * 3 * hp.nC, cudaMemcpyDeviceToHost, s));

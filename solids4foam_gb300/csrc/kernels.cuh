@@ -212,6 +212,80 @@ size_t localSmemBytes(const MeshView& mv);
 template <typename T>
 cudaError_t localPrepare(const MeshView& mv, int* blocksPerSM);
 
+// ---- cluster-resident PCG (kernels_resident.cu) ------------------------------
+constexpr int kResW = 6;         // most neighbours of a row
+constexpr int kResThreads = 256;  // threads of a CTA
+constexpr int kResMaxCtas = 16;  // most CTAs of a cluster
+// Plan of a mesh: the rows' PCG order, split over the CTAs of a cluster.
+struct ResView {
+  int C;               // CTAs of the cluster
+  int local;           // 1: processor-local DIC (levels of whole parts in a CTA)
+  int single;          // 1: exact DIC, the substitutions run in CTA 0 (all rows in its memory)
+  int wide;            // 1: levels of more rows than threads walk them
+  int more;            // 1: rows with more than three entries of a sweep
+  int split;           // 1: a thread per component of a row walks the levels
+  int walk;            // threads that run the substitutions (inside a CTA)
+  int ring;            // rows of a level whose entries are copied ahead
+  int nLev;            // levels of the substitutions
+  int maxRows;         // rows of the largest chunk, rounded up to 4
+  int uRows;           // rows of the shared vector, the last one zero
+  int place;           // kept in shared memory: 1 vectors, 2 sweep tables, 4 product tables
+  const int* chunk;    // [C + 1] first PCG row of each CTA
+  const int* lvl;      // [C][nLev + 1] first row (in the chunk) of each level; single: [nLev + 1]
+  const uint32_t* col;   // [kResW][nC] product columns: CTA << 24 | row in its chunk
+  const uint32_t* cnt;   // [nC] entries of the product
+};
+// One sweep's table, by row: three coefficients and a word of packed columns
+// (kernels_resident.cu).
+template <typename T> struct ResSweepTab;
+template <> struct ResSweepTab<float> {
+  using Q = float4;    // a0, a1, a2, word bits 0-31
+  using R = uint32_t;  // word bits 32-63
+  const Q* q; const R* r;
+  __device__ __forceinline__ void put(int i, const float (&a)[3], unsigned long long w) const {
+    const_cast<Q*>(q)[i] = make_float4(a[0], a[1], a[2], __uint_as_float((uint32_t)w));
+    const_cast<R*>(r)[i] = (uint32_t)(w >> 32);
+  }
+};
+template <> struct ResSweepTab<double> {
+  using Q = double2;  // a0, a1
+  using R = double2;  // a2, word
+  const Q* q; const R* r;
+  __device__ __forceinline__ void put(int i, const double (&a)[3], unsigned long long w) const {
+    const_cast<Q*>(q)[i] = make_double2(a[0], a[1]);
+    const_cast<R*>(r)[i] = make_double2(a[2], __longlong_as_double((long long)w));
+  }
+};
+// The same for the parts of kernels_part.cu: 16 bytes a row in FP32.
+template <typename T> struct PartTab;
+template <> struct PartTab<float> {
+  const float4* q;
+};
+// Its coefficients in the PCG value type, by PCG row.
+template <typename T>
+struct ResPtrs {
+  const T* val; const T* diag; const T* rD;
+  ResSweepTab<T> sweep[2];  // forward, backward
+  ResSweepTab<T> more[2];   // entries 3..5 of the rows that have them; null: none has
+};
+template <typename T>
+size_t resSmemBytes(const ResView& rv, int place);
+template <typename T>
+int resPlacement(const ResView& rv, size_t limit);
+// Sets the kernels' attributes; clusters: how many fit the device at once.
+template <typename T>
+cudaError_t resPrepare(const ResView& rv, int* clusters);
+template <typename T>
+void launchResTables(const MeshView& mv, const ResView& rv, const int* pos, const double* val,
+                     const double* diag, const double* rD, const double* rDa, bool diagOnly,
+                     const ResPtrs<T>& out, cudaStream_t s);
+// The PCG loop of a corrector for nCases load cases (a cluster each).  many:
+// several meshes or cases run at once (two CTAs per SM).
+template <typename T>
+cudaError_t launchResPcg(const MeshView& mv, const Controls& c, const ResView& rv,
+                         const ResPtrs<T>& rp, const PcgPtrs<T>& p, DevState* st, cudaStream_t s,
+                         int nCases, bool many);
+
 // ---- operator product without allocation (noalloc.cu) ------------------------
 // y = A x and x.Ax for k columns of host vectors in caller order, through the
 // work vectors work0/work1 ([nC][3] doubles each) and a static scratch block;

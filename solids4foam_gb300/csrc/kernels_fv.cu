@@ -45,6 +45,11 @@ __device__ __forceinline__ S6 neoHookean(const Controls& c, const T9& F) {
   return (1.0 / J) * addI(sdev, sigmaHyd);
 }
 
+// The position of row s in the PCG vectors x and r.
+__device__ __forceinline__ int pcgRow(const MeshView& mv, int s) {
+  return mv.pcgPos ? mv.pcgPos[s] : s;
+}
+
 // ------------------------------------------------------------- geometry ---
 
 __global__ void kGeomCells(MeshView mv, GeomInputs in, GeomOutputs out) {
@@ -282,15 +287,15 @@ kApplyX(MeshView mv, Controls c, FieldPtrs f, T* __restrict__ x, const T* pA, co
     const bool first = st->iCorr == 0;
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < mv.nC; s += gridDim.x * blockDim.x) {
       const V3 uo = ldV(Uold, s);
-      const V3 us = uo + ldVT(x, s);
+      const V3 us = uo + ldVT(x, pcgRow(mv, s));
       stV(Unew, s, aitkenRelax(c, first, f.aitA + s, f.aitR + 3 * (size_t)s, uo, us, true));
     }
   } else if (fr == 1.0)
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < mv.nC; s += gridDim.x * blockDim.x)
-      stV(Unew, s, ldV(Uold, s) + ldVT(x, s));
+      stV(Unew, s, ldV(Uold, s) + ldVT(x, pcgRow(mv, s)));
   else
     for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < mv.nC; s += gridDim.x * blockDim.x)
-      stV(Unew, s, ldV(Uold, s) + fr * ldVT(x, s));
+      stV(Unew, s, ldV(Uold, s) + fr * ldVT(x, pcgRow(mv, s)));
 }
 
 // mode 0 (constructor): gradient only, from the current field.
@@ -333,7 +338,7 @@ kPost(MeshView mv, Controls c, FieldPtrs f, const T* __restrict__ x, DevState* s
       acc = acc + outer(ldV(mv.lsv, e), ldV(U, mv.col[e]) - Up);
     // relaxed: the boundary values come from the field as solved, then
     // relax against their previous values (the cells were relaxed already)
-    const V3 UpSolved = (relax && apply) ? ldV(f.D[dc], s) + ldVT(x, s) : Up;
+    const V3 UpSolved = (relax && apply) ? ldV(f.D[dc], s) + ldVT(x, pcgRow(mv, s)) : Up;
     for (int b = mv.browptr[s]; b < mv.browptr[s + 1]; ++b) {
       V3 Ub = boundaryValue(mv, c, f, b, UpSolved, Gold);
       if (relax) {
@@ -398,7 +403,7 @@ kPost(MeshView mv, Controls c, FieldPtrs f, const T* __restrict__ x, DevState* s
     if (apply) {
       // maxima of squared magnitudes; the square root is taken once at the end
       // max|D - D.prevIter|: the correction, or its relaxed part
-      const V3 xs = relax ? Up - ldV(f.D[dc], s) : ldVT(x, s);
+      const V3 xs = relax ? Up - ldV(f.D[dc], s) : ldVT(x, pcgRow(mv, s));
       mx[0] = fmax(mx[0], magSqr(xs));
       mx[1] = fmax(mx[1], c.tl == 1 ? magSqr(Up) : magSqr(Up - ldV(f.D0, s)));
       mx[2] = fmax(mx[2], magSqr(Up));
@@ -587,8 +592,9 @@ kRhs(MeshView mv, Controls c, FieldPtrs f, T* __restrict__ x, T* __restrict__ r,
     if (mv.emptyDir == 1) R.x = 0.0;
     else if (mv.emptyDir == 2) R.y = 0.0;
     else if (mv.emptyDir == 3) R.z = 0.0;
-    stVT(r, s, R);
-    stVT(x, s, V3{0, 0, 0});
+    const int ps = pcgRow(mv, s);
+    stVT(r, ps, R);
+    stVT(x, ps, V3{0, 0, 0});
     const double xb[3] = {st->xbar[0], st->xbar[1], st->xbar[2]};
     const double md[3] = {MD.x, MD.y, MD.z}, rr[3] = {R.x, R.y, R.z};
     for (int k = 0; k < 3; ++k) {
