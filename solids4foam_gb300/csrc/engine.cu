@@ -112,6 +112,7 @@ struct EventTimer : LaunchTimer {
 template <typename T>
 constexpr int kResMaxRows(bool local) { return !local ? 16000 : sizeof(T) == 4 ? 2048 : 1280; }
 constexpr int kResMaxDiagRows = 16384;
+constexpr int kPartUnroll = 8;  // PCG iterations of a pass of the device loop (part kernels)
 
 struct Engine {
   Ctx* ctx = nullptr;
@@ -164,6 +165,22 @@ struct Engine {
   };
   Resident<double> res64;
   Resident<float> res32;
+  // part kernels of the processor-local PCG (kernels_part.cu), per value type
+  template <typename T>
+  struct Parts {
+    bool tried = false, ok = false, valid = false;
+    PartView pv{};
+    PartPtrs<T> pt{};
+  };
+  Parts<double> parts64;
+  Parts<float> parts32;
+  int *dHaloCnt = nullptr, *dHalo = nullptr, haloCap = 0;
+  unsigned short* dSlot = nullptr;
+  template <typename T>
+  Parts<T>& parts() {
+    if constexpr (sizeof(T) == 4) return parts32;
+    else return parts64;
+  }
   template <typename T>
   Resident<T>& resident() {
     if constexpr (sizeof(T) == 4) return res32;
@@ -631,6 +648,7 @@ struct Engine {
     matrixPrecond = pre;
     fp32Valid = false;
     res64.valid = res32.valid = false;
+    parts64.valid = parts32.valid = false;
     return S4G_OK;
   }
 
@@ -824,6 +842,90 @@ struct Engine {
     rv.chunk = dChunk; rv.lvl = dLvl; rv.col = col; rv.cnt = cnt;
     q.ok = true;
     return S4G_OK;
+  }
+
+  // The part kernels of value type T (kernels_part.cu): true if they run this
+  // mesh's processor-local PCG where the resident one does not.
+  template <typename T>
+  s4g_status ensureParts() {
+    Parts<T>& q = parts<T>();
+    if (!mv.subdomains || lin.preconditioner != S4G_PRECOND_DIC || runsResident<T>()) return S4G_OK;
+    if (!q.tried) {
+      q.tried = true;
+      S4G_TRY(planParts<T>(q));
+    }
+    if (!q.ok || q.valid) return S4G_OK;
+    S4G_CUDA(launchPartTables<T>(mv, q.pv, dVal, dRDa, q.pt, ctx->stream));
+    launches++;
+    q.valid = true;
+    return S4G_OK;
+  }
+
+  template <typename T>
+  s4g_status planParts(Parts<T>& q) {
+    const int nC = hp.nC;
+    cudaStream_t s = ctx->stream;
+    PartView& pv = q.pv;
+    pv.capRows = (hp.maxRows + 3) / 4 * 4;
+    pv.zeroRow = pv.capRows;
+    if (pv.capRows > partMaxRows<T>()) return S4G_OK;
+    for (int r = 0; r < nC; ++r)
+      if (hp.rowptr[r + 1] - hp.rowptr[r] > kResW) return S4G_OK;
+    int wide = 1;
+    for (size_t l = 0; l + 1 < hp.lvlStart.size(); ++l)
+      wide = std::max(wide, hp.lvlStart[l + 1] - hp.lvlStart[l]);
+    pv.wide = wide > partWalkRows<T>() ? 1 : 0;
+    pv.more = (pv.wide || !hp.locSlots) ? 1 : 0;  // (the form for wide levels reads the flag)
+    if (!dHalo) {
+      // the entries that lead out of a part: counted, then placed
+      int* most;
+      S4G_TRY(alloc(&dHaloCnt, (size_t)hp.nParts));
+      S4G_TRY(alloc(&most, 1));
+      S4G_CUDA(cudaMemsetAsync(most, 0, sizeof(int), s));
+      S4G_CUDA(launchPartCount(mv, dHaloCnt, most, s));
+      S4G_TRY(copySync(&haloCap, most, sizeof(int), cudaMemcpyDeviceToHost));
+      S4G_TRY(alloc(&dHalo, (size_t)hp.nParts * std::max(haloCap, 1)));
+      S4G_TRY(alloc(&dSlot, (size_t)kResW * nC));
+      PartView all = pv;
+      all.haloCap = haloCap; all.halo = dHalo; all.slot = dSlot;
+      S4G_CUDA(launchPartSlots(mv, all, s));
+      launches += 2;
+    }
+    pv.haloCap = haloCap; pv.haloCnt = dHaloCnt; pv.halo = dHalo; pv.slot = dSlot;
+    if (pv.capRows + haloCap > 65535) return S4G_OK;
+    int blocks[2] = {0, 0};
+    const cudaError_t e = partPrepare<T>(mv, pv, blocks);
+    if (e != cudaSuccess || blocks[0] < 1 || blocks[1] < 1) {
+      cudaGetLastError();
+      return S4G_OK;
+    }
+    // the smallest grid that gives every CTA the same number of parts
+    for (int k = 0; k < 2; ++k) {
+      const int most = std::min(hp.nParts, blocks[k] * ctx->numSMs);
+      const int waves = (hp.nParts + most - 1) / most;
+      pv.grid[k] = (hp.nParts + waves - 1) / waves;
+    }
+    T* val;
+    S4G_TRY(alloc(&val, (size_t)kResW * nC));
+    q.pt.val = val;
+    for (int k = 0; k < (pv.more ? 4 : 2); ++k) {
+      auto& tb = k < 2 ? q.pt.sweep[k] : q.pt.more[k - 2];
+      if constexpr (sizeof(T) == 4) {
+        float4* a;
+        S4G_TRY(alloc(&a, (size_t)nC));
+        tb.q = a;
+      } else {
+        double2 *a, *b;
+        S4G_TRY(alloc(&a, (size_t)nC)); S4G_TRY(alloc(&b, (size_t)nC));
+        tb.q = a; tb.r = b;
+      }
+    }
+    q.ok = true;
+    return S4G_OK;
+  }
+  template <typename T>
+  bool runsParts() {
+    return mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC && !runsResident<T>() && parts<T>().ok;
   }
 
   // The mesh as the field passes of a solve of type T see it: with the
@@ -1022,6 +1124,7 @@ struct Engine {
     const bool mixed = precision == S4G_FP32_REFINE;
     if (mixed) S4G_TRY(ensureFp32());
     S4G_TRY(mixed ? ensureResident<float>() : ensureResident<double>());
+    S4G_TRY(mixed ? ensureParts<float>() : ensureParts<double>());
     {
       const Controls ct = controls(0);
       if (mixed) S4G_TRY(tuneLocal<float>(ct, pc32));
@@ -1127,7 +1230,7 @@ struct Engine {
   template <typename T>
   s4g_status tuneLocal(const Controls& c, const PcgPtrs<T>& p) {
     bool& done = sizeof(T) == 4 ? tuned32 : tuned64;
-    if (runsResident<T>()) return S4G_OK;  // nothing to choose
+    if (runsResident<T>() || runsParts<T>()) return S4G_OK;  // nothing to choose
     if (done || !autotune) { done = true; return S4G_OK; }
     cudaStream_t s = ctx->stream;
     const size_t n3 = 3 * (size_t)hp.nC;
@@ -1288,12 +1391,18 @@ struct Engine {
     if (!ok || cudaStreamBeginCaptureToGraph(s, pcgBody, nullptr, nullptr, 0, mode) != cudaSuccess)
       return false;
     long long dummy = 0;
-    if (mv.subdomains && c.precond == 0)
+    if (runsParts<T>()) {
+      // several iterations per pass of the loop (a pass costs about 5 us, the
+      // launches after the stop decision about 1 us each)
+      for (int k = 0; k < kPartUnroll; ++k)
+        ok = launchPartIteration<T>(mv, c, parts<T>().pv, parts<T>().pt, p, dState, dPartials, s, nullptr,
+                                    nRun) == cudaSuccess && ok;
+    } else if (mv.subdomains && c.precond == 0)
       launchLocalIteration<T>(mv, c, p, dState, dPartials, tuning<T>(), s, &dummy, nullptr, nRun);
     else
       launchPcgIteration<T>(mv, c, p, dState, dPartials, grid, s, &dummy, nullptr);
     launchSetLoopCond(hPcg, dState, nRun, 0, 0, pcgLimit, s);
-    ok = cudaStreamEndCapture(s, &ended) == cudaSuccess;
+    ok = cudaStreamEndCapture(s, &ended) == cudaSuccess && ok;
     (void)tl;
     return ok && cudaGetLastError() == cudaSuccess;
   }
@@ -1339,7 +1448,11 @@ struct Engine {
     auto launchBatch = [&](int n, long long* count) {
       for (int i = 0; i < n; ++i) {
         if (tm()) timer.tag = launched++;
-        if (mv.subdomains && c.precond == 0)
+        if (runsParts<T>()) {
+          launchPartIteration<T>(mv, c, parts<T>().pv, parts<T>().pt, p, dState, dPartials, ctx->stream,
+                                 tm(), nRun);
+          *count += 2;
+        } else if (mv.subdomains && c.precond == 0)
           launchLocalIteration<T>(mv, c, p, dState, dPartials, tuning<T>(), ctx->stream,
                                   count, tm(), nRun);
         else
@@ -1370,6 +1483,15 @@ struct Engine {
     return setErr(S4G_TIMEOUT, "PCG loop did not end");
   }
 
+  // Kernels that a device loop launched for `it` PCG iterations.
+  template <typename T>
+  long long pcgLaunches(const Controls& c, bool local, long long it) {
+    if (runsResident<T>()) return 0;  // (one per corrector, counted there)
+    if (runsParts<T>()) return 2 * it + (it + kPartUnroll - 1) / kPartUnroll;
+    const int perIt = local ? (tuning<T>().uIdx == 2 ? 3 : 2) : (c.precond == 0 ? 5 : 4);
+    return it * (perIt + 1);
+  }
+
   // One evolve(): correctors until converged() or nCorrectors.  The inner
   // PCG runs in T; the right-hand side, the correction of D and every
   // convergence test stay in FP64.
@@ -1385,10 +1507,8 @@ struct Engine {
         S4G_CUDA(cudaGetLastError());
         S4G_TRY(readState());
         const bool local = mv.subdomains && c.precond == 0;
-        const long long perIt = local ? (tuning<T>().uIdx == 2 ? 3 : 2) : (c.precond == 0 ? 5 : 4);
-        const bool res = runsResident<T>();
         launches += 1 + (long long)(hState->nCorrDone - corr0) * (tl ? 6 : 5) +
-                    (res ? 0 : (long long)(hState->pcgIter - it0) * (perIt + 1));
+                    pcgLaunches<T>(c, local, hState->pcgIter - it0);
         ranOnDevice = true;
         return S4G_OK;
       }
@@ -1439,6 +1559,7 @@ struct Engine {
     const bool mixed = precision == S4G_FP32_REFINE;
     if (mixed) S4G_TRY(ensureFp32());
     S4G_TRY(mixed ? ensureResident<float>() : ensureResident<double>());
+    S4G_TRY(mixed ? ensureParts<float>() : ensureParts<double>());
     cudaEvent_t e0, e1;
     S4G_CUDA(cudaEventCreate(&e0));
     S4G_CUDA(cudaEventCreate(&e1));
@@ -1570,6 +1691,7 @@ struct Engine {
     const bool mixed = precision == S4G_FP32_REFINE;
     if (mixed) S4G_TRY(ensureFp32());
     S4G_TRY(mixed ? ensureResident<float>() : ensureResident<double>());
+    S4G_TRY(mixed ? ensureParts<float>() : ensureParts<double>());
     if (mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC) {
       const Controls ct = controls(0);
       if (mixed) S4G_TRY(tuneLocal<float>(ct, pc32));
@@ -1602,11 +1724,10 @@ struct Engine {
     S4G_TRY(readState());
     ranOnDevice = true;
     const bool local = mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC;
-    const long long perIt = local ? (tuning32or64().uIdx == 2 ? 3 : 2)
-                                  : (lin.preconditioner == S4G_PRECOND_DIC ? 5 : 4);
-    const bool res = precision == S4G_FP32_REFINE ? runsResident<float>() : runsResident<double>();
+    const Controls c = controls(0);
     launches += 1 + (long long)hState->nCorrDone * 5 +
-                (res ? 0 : (long long)hState->pcgIter * (perIt + 1));
+                (precision == S4G_FP32_REFINE ? pcgLaunches<float>(c, local, hState->pcgIter)
+                                              : pcgLaunches<double>(c, local, hState->pcgIter));
     if (Dout) {
       launchGather(hp.nC, 3, dC2s, f.D[hState->dcur], dOut, s);
       S4G_CUDA(cudaMemcpyAsync(Dout, dOut, sizeof(double) * 3 * hp.nC, cudaMemcpyDeviceToHost, s));

@@ -286,6 +286,44 @@ cudaError_t launchResPcg(const MeshView& mv, const Controls& c, const ResView& r
                          const ResPtrs<T>& rp, const PcgPtrs<T>& p, DevState* st, cudaStream_t s,
                          int nCases, bool many);
 
+// ---- processor-local DIC PCG, a CTA per part (kernels_part.cu) ---------------
+// Plan of a mesh for a value type.
+struct PartView {
+  int capRows;     // rows of the largest part, rounded up to 4
+  int zeroRow;     // the zero row of the substitutions' padding
+  int more, wide;  // rows of more than three entries; levels of more rows than threads
+  int grid[2];     // CTAs of the preconditioner and of the product
+  int haloCap;     // most entries of a part that lead out of it
+  const int* haloCnt;          // [nParts]
+  const int* halo;             // [nParts][haloCap] their rows
+  const unsigned short* slot;  // [kResW][nC] product columns: row of the part, or rows + place
+};
+template <typename T> struct PartTabOf { using Tab = PartTab<float>; };
+template <> struct PartTabOf<double> { using Tab = ResSweepTab<double>; };
+template <typename T>
+struct PartPtrs {
+  const T* val;                        // [kResW][nC] product coefficients
+  typename PartTabOf<T>::Tab sweep[2]; // forward, backward
+  typename PartTabOf<T>::Tab more[2];  // entries 3..5
+};
+template <typename T>
+int partMaxRows();
+template <typename T>
+int partWalkRows();
+cudaError_t launchPartCount(const MeshView& mv, int* cnt, int* most, cudaStream_t s);
+cudaError_t launchPartSlots(const MeshView& mv, const PartView& pv, cudaStream_t s);
+template <typename T>
+cudaError_t launchPartTables(const MeshView& mv, const PartView& pv, const double* val,
+                             const double* rDa, const PartPtrs<T>& out, cudaStream_t s);
+// Sets the kernels' attributes; blocks[2]: resident CTAs per SM of each.
+template <typename T>
+cudaError_t partPrepare(const MeshView& mv, const PartView& pv, int* blocks);
+// One PCG iteration (two kernels).
+template <typename T>
+cudaError_t launchPartIteration(const MeshView& mv, const Controls& c, const PartView& pv,
+                                const PartPtrs<T>& pt, const PcgPtrs<T>& p, DevState* st,
+                                double* partials, cudaStream_t s, LaunchTimer* tm, int nCases);
+
 // ---- operator product without allocation (noalloc.cu) ------------------------
 // y = A x and x.Ax for k columns of host vectors in caller order, through the
 // work vectors work0/work1 ([nC][3] doubles each) and a static scratch block;

@@ -331,28 +331,18 @@ __device__ __forceinline__ void locFinish(const MeshView& mv, const Controls& c,
   if (!lastBlockDone(&st->counter[5], gridDim.x)) return;
   double S[6];
   locGroupsTotal<6>(grec, mv.locGroups, S, red);
-  if (t != 0) return;
-  st->counter[5] = 0;
-  st->locTicket = 0;
-  int any = 0;
-  for (int k = 0; k < 3; ++k) {
-    if (st->pending[k]) {
-      st->pending[k] = 0;
-      const double fr = S[3 + k] / st->normFactor[k];
-      st->finalRes[k] = fr;
-      st->nIter[k] += 1;
-      const bool conv = fr < c.tol || (c.relTol > 1e-20 && fr < c.relTol * st->initRes[k]);
-      if (!isfinite(fr)) atomicOr(&st->status, kErrNaN);
-      st->active[k] = (!conv && st->nIter[k] < c.maxIter && isfinite(fr)) ? 1 : 0;
-    }
-    if (st->active[k]) {
-      st->beta[k] = st->nIter[k] == 0 ? 0.0 : S[k] / st->wArA[k];
-      st->wArA[k] = S[k];
-    }
-    any |= st->active[k];
+  if (t >= 32) return;
+  double mine = 0;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    const double v = __shfl_sync(0xffffffffu, S[k], 0);
+    if (t == k) mine = v;
   }
-  if (anyPend) st->pcgIter += 1;
-  st->pcgContinue = any;
+  if (t == 0) {
+    st->counter[5] = 0;
+    st->locTicket = 0;
+  }
+  pcgDecideBeta(c, st, mine, anyPend);
 }
 
 // Resident blocks the register budget is set for (NT threads, RPT rows per
@@ -790,25 +780,15 @@ kLocSpmv(MeshView mv, PcgPtrs<T> p, DevState* st, double* partials) {
   if (!lastBlockDone(&st->counter[6], gridDim.x)) return;
   double sum[3];
   reducePartials<3>(partials, 8, gridDim.x, sum, red);
-  if (threadIdx.x != 0) return;
-  st->counter[6] = 0;
-  int any = 0;
+  if (threadIdx.x >= 32) return;
+  double mine = 0;
+#pragma unroll
   for (int k = 0; k < 3; ++k) {
-    st->xPend[k] = 0;  // applied by this pass
-    if (!st->active[k]) continue;
-    st->wApA[k] = sum[k];
-    if (fabs(sum[k]) / st->normFactor[k] < 1e-300) {  // checkSingularity: stop this component
-      st->active[k] = 0;
-      continue;
-    }
-    if (sum[k] <= 0) atomicOr(&st->status, kErrIndefinite);
-    st->alpha[k] = st->wArA[k] / sum[k];
-    st->pending[k] = 1;
-    st->xPend[k] = 1;
-    any = 1;
+    const double v = __shfl_sync(0xffffffffu, sum[k], 0);
+    if (threadIdx.x == k) mine = v;
   }
-  st->pbuf = pb ^ 1;
-  st->pcgContinue = any;
+  if (threadIdx.x == 0) st->counter[6] = 0;
+  pcgDecideAlpha(st, mine, pb);
 }
 
 // Split form of the second kernel (FP64 favours it: a neighbour's p_new is
@@ -884,25 +864,15 @@ kLocSpmvSplit(MeshView mv, PcgPtrs<T> p, DevState* st, double* partials) {
   if (!lastBlockDone(&st->counter[6], gridDim.x)) return;
   double sum[3];
   reducePartials<3>(partials, 8, gridDim.x, sum, red);
-  if (threadIdx.x != 0) return;
-  st->counter[6] = 0;
-  int any = 0;
+  if (threadIdx.x >= 32) return;
+  double mine = 0;
+#pragma unroll
   for (int k = 0; k < 3; ++k) {
-    st->xPend[k] = 0;  // applied by this pass
-    if (!st->active[k]) continue;
-    st->wApA[k] = sum[k];
-    if (fabs(sum[k]) / st->normFactor[k] < 1e-300) {  // checkSingularity: stop this component
-      st->active[k] = 0;
-      continue;
-    }
-    if (sum[k] <= 0) atomicOr(&st->status, kErrIndefinite);
-    st->alpha[k] = st->wArA[k] / sum[k];
-    st->pending[k] = 1;
-    st->xPend[k] = 1;
-    any = 1;
+    const double v = __shfl_sync(0xffffffffu, sum[k], 0);
+    if (threadIdx.x == k) mine = v;
   }
-  st->pbuf = pb ^ 1;
-  st->pcgContinue = any;
+  if (threadIdx.x == 0) st->counter[6] = 0;
+  pcgDecideAlpha(st, mine, pb);
 }
 
 // Generic tables: kLocPrecond with NT threads and RPT rows per thread in

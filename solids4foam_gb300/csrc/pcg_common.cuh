@@ -2,6 +2,7 @@
 #pragma once
 
 #include "device_common.cuh"
+#include "kernels.cuh"
 
 namespace s4g {
 
@@ -35,6 +36,74 @@ template <> struct Acc<float> {
   }
   __device__ __forceinline__ double value() const { return (double)s + (double)c; }
 };
+
+// End of a processor-local preconditioner launch, by warp 0 of its last CTA:
+// S = w.r of the components, then sum|r| (S[k] in lane k and k + 3 for lanes
+// 0 .. 5 of `mine`).  Per component the residual test of the pending iteration,
+// beta and wArA, and whether the loop goes on.  A lane per component with its
+// state read at once: one thread going through the three with their dependent
+// loads and divisions (564 cycles each) took about 6 us of every iteration.
+__device__ __forceinline__ void pcgDecideBeta(const Controls& c, DevState* st, double mine, bool anyPend) {
+  const int l = threadIdx.x & 31;
+  const double rs = __shfl_down_sync(0xffffffffu, mine, 3);
+  int act = 0;
+  if (l < 3) {
+    const int pend = st->pending[l], it0 = st->nIter[l], a0 = st->active[l];
+    const double nf = st->normFactor[l], ir = st->initRes[l], wa = st->wArA[l];
+    act = a0;
+    int it = it0;
+    if (pend) {
+      st->pending[l] = 0;
+      st->nIter[l] = ++it;
+      // sum|r| / normFactor < tolerance, or relTol * the initial one
+      const bool conv = rs < c.tol * nf || (c.relTol > 1e-20 && rs < c.relTol * ir * nf);
+      const bool fin = isfinite(rs);
+      if (!fin) atomicOr(&st->status, kErrNaN);
+      act = (!conv && it < c.maxIter && fin) ? 1 : 0;
+      st->active[l] = act;
+      if (!act) st->finalRes[l] = rs / nf;
+    }
+    if (act) {
+      st->beta[l] = it == 0 ? 0.0 : mine / wa;
+      st->wArA[l] = mine;
+    }
+  }
+  const unsigned any = __ballot_sync(0xffffffffu, act != 0);
+  if (l == 0) {
+    if (anyPend) st->pcgIter += 1;
+    st->pcgContinue = any != 0;
+  }
+}
+
+// End of the product's launch, by warp 0 of its last CTA: mine = p.q of the
+// component in lanes 0 .. 2.  alpha, and which components have an iteration
+// pending; pb: the p buffer the launch read.
+__device__ __forceinline__ void pcgDecideAlpha(DevState* st, double mine, int pb) {
+  const int l = threadIdx.x & 31;
+  int on = 0;
+  if (l < 3) {
+    const int act = st->active[l];
+    const double nf = st->normFactor[l], wa = st->wArA[l];
+    st->xPend[l] = 0;  // applied by this pass
+    if (act) {
+      st->wApA[l] = mine;
+      if (fabs(mine) < 1e-300 * nf) {  // checkSingularity: stop this component
+        st->active[l] = 0;
+      } else {
+        if (mine <= 0) atomicOr(&st->status, kErrIndefinite);
+        st->alpha[l] = wa / mine;
+        st->pending[l] = 1;
+        st->xPend[l] = 1;
+        on = 1;
+      }
+    }
+  }
+  const unsigned any = __ballot_sync(0xffffffffu, on != 0);
+  if (l == 0) {
+    st->pbuf = pb ^ 1;
+    st->pcgContinue = any != 0;
+  }
+}
 
 // 16-byte asynchronous global->shared copy that bypasses L1 (data read once).
 __device__ __forceinline__ void cpAsync16(void* sm, const void* gm) {

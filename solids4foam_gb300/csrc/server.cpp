@@ -102,7 +102,7 @@ long long estimateFootprint(const Request& r) {
   b += N * (8 * 3 + 24 * 3 + 72 + 48 + 72) + F * (48) + B * (24 + 72 + 48 + 24);
   b += N * 24 * 6;
   if (r.precision == S4G_FP32_REFINE) b += N * (8 + 12 * 6) + F * 16;
-  b += N * 240;  // the PCG's own tables (cluster-resident)
+  b += N * 240;  // the PCG's own tables (cluster-resident or by part)
   if (r.meshOpts.dic_subdomains) b += F * 2 * 18 + N * 8;
   if (r.model != S4G_LIN_GEOM_TOTAL_DISP) b += N * (72 * 6 + 48 + 8) + B * (72 * 6 + 48 + 8);
   return (long long)(b * 1.15) + (16ll << 20);

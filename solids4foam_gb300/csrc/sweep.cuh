@@ -253,7 +253,7 @@ constexpr int kResAhead = 8;
 // shared addresses of a sweep's tables, or of its ring (m: the second entries)
 struct ResAddr { unsigned q, r, mq, mr; };
 template <int DIR, bool CROSS, bool RING, bool SPLIT, bool MORE, bool WIDE, typename E>
-__device__ __noinline__ void resSweep(const typename E::Tab tb, const typename E::Tab more,
+__device__ __forceinline__ void resSweepBody(const typename E::Tab tb, const typename E::Tab more,
                                       const ResAddr ad, unsigned uBase, unsigned rank,
                                       unsigned lva, int nL, int walk, int rs) {
   using T = typename E::T;
@@ -350,6 +350,14 @@ __device__ __noinline__ void resSweep(const typename E::Tab tb, const typename E
   }
 }
 
+// The same as a function of its own (the resident kernel's many forms).
+template <int DIR, bool CROSS, bool RING, bool SPLIT, bool MORE, bool WIDE, typename E>
+__device__ __noinline__ void resSweep(const typename E::Tab tb, const typename E::Tab more,
+                                      const ResAddr ad, unsigned uBase, unsigned rank,
+                                      unsigned lva, int nL, int walk, int rs) {
+  resSweepBody<DIR, CROSS, RING, SPLIT, MORE, WIDE, E>(tb, more, ad, uBase, rank, lva, nL, walk, rs);
+}
+
 // ---- sums ------------------------------------------------------------------------
 // A thread's partial sum and its addition: FP64, or (FP32 values) the
 // compensated pair s + c, added with the error of s (two-sum) kept in c.
@@ -358,6 +366,7 @@ template <> struct Part<double> {
   using V = double;
   static __device__ __forceinline__ V of(const Acc<double>& a) { return a.s; }
   static __device__ __forceinline__ V zero() { return 0.0; }
+  static __device__ __forceinline__ V ldcg(const V* a) { return __ldcg(a); }
   static __device__ __forceinline__ V add(V a, V b) { return a + b; }
   static __device__ __forceinline__ V shfl(V a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
   static __device__ __forceinline__ double value(V a) { return a; }
@@ -366,6 +375,7 @@ template <> struct Part<float> {
   using V = float2;
   static __device__ __forceinline__ V of(const Acc<float>& a) { return make_float2(a.s, a.c); }
   static __device__ __forceinline__ V zero() { return make_float2(0.0f, 0.0f); }
+  static __device__ __forceinline__ V ldcg(const V* a) { return __ldcg(a); }
   static __device__ __forceinline__ V add(V a, V b) {
     const float s = __fadd_rn(a.x, b.x), z = __fsub_rn(s, a.x);
     const float e = __fadd_rn(__fsub_rn(a.x, __fsub_rn(s, z)), __fsub_rn(b.x, z));
