@@ -38,6 +38,10 @@ struct MeshView {
   const int* lowCnt;   // lower entries per row
   int maxRows, maxHalo, maxEntries, maxLevels;
   int rowGrid;         // blocks of the grid-stride row kernels
+  // the corrector's field passes: threads per block (few on a small mesh, so that
+  // its FP64 work spreads over the SMs), blocks over cells, most over faces
+  int fvBlock, fvGrid, fvFaceGrid;
+  const int* bcell;    // cell of each boundary face
   int spinLimit;       // polls of a bounded wait before it gives up (kErrTimeout)
   // processor-local DIC tables (see HostPrep)
   const int* locEntStart; const int* locSrc; const uint16_t* locIdx;
@@ -254,8 +258,20 @@ __device__ __forceinline__ T9 fromS(const S6& s) {
 }
 __device__ __forceinline__ double trS(const S6& s) { return s.xx + s.yy + s.zz; }
 __device__ __forceinline__ double trT(const T9& t) { return t.xx + t.yy + t.zz; }
+// x / 3, correctly rounded, in three operations instead of a division (some
+// fifteen FP64 ones): the product with the rounded reciprocal, corrected by its
+// exact remainder (Markstein 1990).
+__device__ __forceinline__ double third(double x) {
+  const double y = 1.0 / 3.0, q = __dmul_rn(x, y), r = __fma_rn(-3.0, q, x);
+  return isfinite(x) ? __fma_rn(r, y, q) : q;
+}
 __device__ __forceinline__ S6 devS(const S6& s) {
   double m = trS(s) / 3.0;
+  return {s.xx - m, s.xy, s.xz, s.yy - m, s.yz, s.zz - m};
+}
+// devS with third(): the same values, without the division
+__device__ __forceinline__ S6 devThird(const S6& s) {
+  const double m = third(trS(s));
   return {s.xx - m, s.xy, s.xz, s.yy - m, s.yz, s.zz - m};
 }
 __device__ __forceinline__ S6 operator+(const S6& a, const S6& b) {

@@ -328,11 +328,16 @@ struct Engine {
     mv.emptyDir = o ? o->empty_direction : 0;
     mv.rowGrid = std::max(1, std::min((nC + kRowBlock - 1) / kRowBlock,
                                       ctx->numSMs * kRowBlocksPerSM));
+    // 64-thread blocks until they fill the SMs four times over (measured on a
+    // 8^3 .. 40^3 mesh: 256-thread blocks leave most SMs without work)
+    mv.fvBlock = nC < ctx->numSMs * 256 ? 64 : kRowBlock;
+    mv.fvGrid = std::max(1, std::min((nC + mv.fvBlock - 1) / mv.fvBlock, ctx->numSMs * kRowBlocksPerSM));
+    mv.fvFaceGrid = ctx->numSMs * kRowBlocksPerSM * (kRowBlock / mv.fvBlock);
     mv.spinLimit = ctx->spinLimit;
     mv.rowptr = dRow; mv.col = dCol; mv.fidx = dFidx; mv.fown = dFown; mv.fnei = dFnei;
     mv.fS = geo.fS; mv.fmagS = geo.fmagS; mv.fw = geo.fw; mv.fdelta = geo.fdelta;
     mv.C = geo.C; mv.invDd = geo.invDd;
-    mv.browptr = dBrow; mv.btype = dBtype;
+    mv.browptr = dBrow; mv.btype = dBtype; mv.bcell = dBcell;
     mv.bS = geo.bS; mv.bmagS = geo.bmagS; mv.bn = geo.bn; mv.bk = geo.bk;
     mv.bdelta = geo.bdelta; mv.bls = geo.bls; mv.bval = dBval; mv.bpress = dBpress;
     mv.brelax = dBrelax;
@@ -386,6 +391,8 @@ struct Engine {
     S4G_TRY(alloc(&f.sigb, 6 * (size_t)nB));
     S4G_TRY(alloc(&f.g, 3 * (size_t)nB));
     S4G_TRY(alloc(&f.gPrev, 3 * (size_t)nB));
+    S4G_TRY(alloc(&f.Ub, 3 * (size_t)nB));
+    S4G_TRY(alloc(&f.sgB, 3 * (size_t)nB));
     S4G_TRY(alloc(&f.Ubr, 3 * (size_t)nB));
     S4G_TRY(alloc(&f.flux, 6 * (size_t)nI));
     S4G_TRY(alloc(&pc.x, 3 * (size_t)nC));
@@ -398,7 +405,9 @@ struct Engine {
     pc.val = dVal; pc.diag = dDiag; pc.rD = dRD; pc.rDa = dRDa;
     S4G_TRY(alloc(&dState, 1));
     S4G_CUDA(cudaMallocHost((void**)&hState, sizeof(DevState)));
-    const size_t rowBlocks = (nC + kRowBlock - 1) / kRowBlock;
+    // records of the row kernels; of the post pass: 8 per cell block, 2 per face block
+    const size_t rowBlocks = std::max<size_t>((nC + kRowBlock - 1) / kRowBlock,
+                                              mv.fvGrid + ((nB + mv.fvBlock - 1) / mv.fvBlock + 4) / 4);
     // per case: block or part records, then the preconditioner's group
     // records and group counters (zero between launches)
     mv.locGroups = (hp.nParts + 31) / 32;
@@ -1066,6 +1075,8 @@ struct Engine {
     S4G_TRY(regrow(f.Gb, 9 * nB * o, 9 * nB * n));
     S4G_TRY(regrow(f.sigb, 6 * nB * o, 6 * nB * n));
     S4G_TRY(regrow(f.g, 3 * nB * o, 3 * nB * n));
+    S4G_TRY(regrow(f.Ub, 3 * nB * o, 3 * nB * n));
+    S4G_TRY(regrow(f.sgB, 3 * nB * o, 3 * nB * n));
     S4G_TRY(regrow(f.Ubr, 3 * nB * o, 3 * nB * n));
     S4G_TRY(regrow(f.gPrev, 3 * nB * o, 3 * nB * n));
     if (f.aitA) {
@@ -1376,16 +1387,19 @@ struct Engine {
       return false;
     const MeshView fv = fieldView<T>();
     const bool res = runsResident<T>();
-    launchRhs<T>(fv, c, f, p.x, p.r, dState, dPartials, s, nullptr, nRun);
+    // of one case, the kernels that decide a loop set its condition
+    const bool one = nRun == 1;
+    LoopCond cOut{one ? 1 : 0, outerLimit, hOut}, cPcg{one && !res ? 1 : 0, pcgLimit, hPcg};
+    launchRhs<T>(fv, c, f, p.x, p.r, dState, dPartials, s, nullptr, nRun, cPcg);
     if (res) {
       // the PCG loop of the corrector is one launch
       ok = resPcg<T>(c, p) == cudaSuccess;
     } else {
-      launchSetLoopCond(hPcg, dState, nRun, 0, 1, pcgLimit, s);
+      if (!one) launchSetLoopCond(hPcg, dState, nRun, 0, 1, pcgLimit, s);
       ok = addWhile(s, hPcg, &pcgBody);
     }
-    launchPost<T>(fv, c, f, p.x, dState, dPartials, 1, s, nullptr, nRun, p.p, p.p2);
-    launchSetLoopCond(hOut, dState, nRun, 1, 0, outerLimit, s);
+    launchPost<T>(fv, c, f, p.x, dState, dPartials, 1, s, nullptr, nRun, p.p, p.p2, cOut);
+    if (!one) launchSetLoopCond(hOut, dState, nRun, 1, 0, outerLimit, s);
     ok = cudaStreamEndCapture(s, &ended) == cudaSuccess && ok;
     if (res) return ok && cudaGetLastError() == cudaSuccess;
     if (!ok || cudaStreamBeginCaptureToGraph(s, pcgBody, nullptr, nullptr, 0, mode) != cudaSuccess)
@@ -1486,7 +1500,7 @@ struct Engine {
   // Kernels that a device loop launched for `it` PCG iterations.
   template <typename T>
   long long pcgLaunches(const Controls& c, bool local, long long it) {
-    if (runsResident<T>()) return 0;  // (one per corrector, counted there)
+    if (runsResident<T>()) return 0;  // (one per corrector)
     if (runsParts<T>()) return 2 * it + (it + kPartUnroll - 1) / kPartUnroll;
     const int perIt = local ? (tuning<T>().uIdx == 2 ? 3 : 2) : (c.precond == 0 ? 5 : 4);
     return it * (perIt + 1);
@@ -1507,7 +1521,7 @@ struct Engine {
         S4G_CUDA(cudaGetLastError());
         S4G_TRY(readState());
         const bool local = mv.subdomains && c.precond == 0;
-        launches += 1 + (long long)(hState->nCorrDone - corr0) * (tl ? 6 : 5) +
+        launches += 1 + (long long)(hState->nCorrDone - corr0) * ((tl ? 7 : 6) + (runsResident<T>() ? 1 : 0)) +
                     pcgLaunches<T>(c, local, hState->pcgIter - it0);
         ranOnDevice = true;
         return S4G_OK;
@@ -1520,7 +1534,7 @@ struct Engine {
       S4G_TRY(readState());
       if (anyCase(&DevState::pcgContinue)) S4G_TRY(pcgLoop<T>(c, p, grid));
       launchPost<T>(fv, c, f, p.x, dState, dPartials, 1, s, tm(), nRun, p.p, p.p2);
-      launches += tl ? 3 : 2;
+      launches += tl ? 5 : 4;
       S4G_CUDA(cudaGetLastError());
       S4G_TRY(readState());
       if (ctx->verbose && outer.info_frequency > 0 &&
@@ -1725,7 +1739,7 @@ struct Engine {
     ranOnDevice = true;
     const bool local = mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC;
     const Controls c = controls(0);
-    launches += 1 + (long long)hState->nCorrDone * 5 +
+    launches += 1 + (long long)hState->nCorrDone * 6 +
                 (precision == S4G_FP32_REFINE ? pcgLaunches<float>(c, local, hState->pcgIter)
                                               : pcgLaunches<double>(c, local, hState->pcgIter));
     if (Dout) {

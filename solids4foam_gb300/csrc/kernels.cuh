@@ -52,6 +52,8 @@ struct FieldPtrs {
   double* sigb;  // [nB][6]
   double* g;     // [nB][3] traction snGrad
   double* gPrev; // [nB][3] the g the last corrector used (before its update)
+  double* Ub;    // [nB][3] boundary values of the solved field, this corrector's
+  double* sgB;   // [nB][3] their normal gradient on fixed-value faces
   double* Ubr;   // [nB][3] field relaxation: the boundary values of the solved
                  // field after the last relaxation (D.prevIter on the boundary)
   double* aitA;  // [nC + nB] Aitken factor of each cell, then of each boundary face
@@ -73,11 +75,19 @@ __host__ __device__ inline FieldPtrs caseFields(FieldPtrs f, int cs, int nC, int
   if (f.D0b) f.D0b += c * 3 * nB;
   f.G += c * 9 * nC; f.sig += c * 6 * nC;
   f.Gb += c * 9 * nB; f.sigb += c * 6 * nB; f.g += c * 3 * nB;
-  f.Ubr += c * 3 * nB; f.gPrev += c * 3 * nB;
+  f.Ubr += c * 3 * nB; f.gPrev += c * 3 * nB; f.Ub += c * 3 * nB; f.sgB += c * 3 * nB;
   if (f.aitA) { f.aitA += c * (nC + nB); f.aitR += c * 3 * (nC + nB); }
   f.flux += c * 6 * nI;
   return f;
 }
+
+// The condition of a device-resident loop of one case, set by the kernel that
+// decides it (instead of launchSetLoopCond's).
+struct LoopCond {
+  int on = 0;
+  unsigned limit = 0;
+  cudaGraphConditionalHandle h{};
+};
 
 // g = tractionBoundarySnGrad with the current sigma_b / grad_b (constructor).
 void launchTractionInit(const MeshView& mv, const Controls& c, const FieldPtrs& f,
@@ -91,13 +101,13 @@ template <typename T>
 void launchPost(const MeshView& mv, const Controls& c, const FieldPtrs& f, const T* x,
                 DevState* st, double* partials, int mode, cudaStream_t s,
                 LaunchTimer* tm = nullptr, int nCases = 1, const T* pA = nullptr,
-                const T* pB = nullptr);
+                const T* pB = nullptr, LoopCond loop = LoopCond());
 // RHS pass (FP64): R = div(sigma) + RhieChow + boundary terms, M*D_old for the
 // residual normalisation; zeroes x, sets r = R rounded to the PCG type.
 template <typename T>
 void launchRhs(const MeshView& mv, const Controls& c, const FieldPtrs& f, T* x, T* r,
                DevState* st, double* partials, cudaStream_t s, LaunchTimer* tm = nullptr,
-               int nCases = 1);
+               int nCases = 1, LoopCond loop = LoopCond());
 // pointD [nP][3] (caller point order) from the storage-order cell centres C,
 // field U and gradient G, over the points' cells pcc (caller cell ids,
 // CSR pcs); see kPointInterp.

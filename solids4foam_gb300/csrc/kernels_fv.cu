@@ -27,13 +27,16 @@
 // negatives of each other; there are no atomics and sums run in a fixed order.
 
 #include "kernels.cuh"
+#include "sweep.cuh"
+
+#include <algorithm>
 
 namespace s4g {
 namespace {
 
 __device__ __forceinline__ S6 hooke(const Controls& c, const T9& g) {
   S6 eps = symmT(g);
-  return addI((2.0 * c.mu) * devS(eps), c.K * trS(eps));
+  return addI((2.0 * c.mu) * devThird(eps), c.K * trS(eps));
 }
 
 __device__ __forceinline__ S6 neoHookean(const Controls& c, const T9& F) {
@@ -298,85 +301,118 @@ kApplyX(MeshView mv, Controls c, FieldPtrs f, T* __restrict__ x, const T* pA, co
       stV(Unew, s, ldV(Uold, s) + fr * ldVT(x, pcgRow(mv, s)));
 }
 
-// mode 0 (constructor): gradient only, from the current field.
-// mode 1 (corrector): apply the correction x, gradient, law, boundary, g.
-// With field relaxation the boundary values are relaxed too (the forced
-// assignment of GeometricField::relax): Ub = Ub.prevIter + f (Ub_new -
+// The boundary values of the solved field and, on fixed-value faces, the normal
+// gradient they give with the previous cell gradient: a thread per face (a cell
+// with three boundary faces would walk them one after the other, FP64 work of
+// some 10 us).  mode 0 (constructor): from the current field.  mode 1
+// (corrector): from the corrected field of kApplyX.  With field relaxation the
+// boundary values come from the field as solved and are relaxed themselves (the
+// forced assignment of GeometricField::relax): Ub = Ub.prevIter + f (Ub_new -
 // Ub.prevIter), Ub.prevIter kept in f.Ubr (mode 0 stores the constructor's).
-// For the TL model the law needs the global J check first, so mode 1 stops
-// after the kinematics (F, F^-1, J) and kPostLawTL finishes the pass.
+template <typename T>
+__global__ void __launch_bounds__(kRowBlock)
+kBoundaryValues(MeshView mv, Controls c, FieldPtrs f, const T* __restrict__ x, const DevState* st, int mode) {
+  const int cs = blockIdx.y;
+  f = caseFields(f, cs, mv.nC, mv.nB, mv.nI);
+  caseView(mv, cs);
+  x += (size_t)cs * 3 * mv.nC;
+  st += cs;
+  const bool apply = mode == 1;
+  if (apply && !st->caseLive) return;
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= mv.nB) return;
+  const int s = mv.bcell[b], dc = st->dcur;
+  const V3 Up = ldV(f.D[apply ? dc ^ 1 : dc], s);
+  const T9 Gold = ldT(f.G, s);
+  const bool relax = c.fieldRelax != 1.0 || c.aitken;
+  const V3 UpSolved = (relax && apply) ? ldV(f.D[dc], s) + ldVT(x, pcgRow(mv, s)) : Up;
+  V3 Ub = boundaryValue(mv, c, f, b, UpSolved, Gold);
+  if (relax) {
+    if (apply) {
+      const V3 pb = ldV(f.Ubr, b);
+      if (c.aitken)
+        Ub = aitkenRelax(c, st->iCorr == 0, f.aitA + mv.nC + b, f.aitR + 3 * ((size_t)mv.nC + b),
+                         pb, Ub, mv.btype[b] == 1);
+      else
+        Ub = pb + c.fieldRelax * (Ub - pb);
+    }
+    stV(f.Ubr, b, Ub);
+  }
+  stV(f.Ub, b, Ub);
+  if (mv.btype[b] != 1) stV(f.sgB, b, mv.bdelta[b] * (Ub - (Up + dotVT(ldV(mv.bk, b), Gold))));
+}
 
+// Records of the corrector pass, one per block: 8 values {sum U (3), maxima of
+// |x|^2, |U - D0|^2, |U|^2, -min J, max J}, the cell blocks' first, then the
+// face blocks' (the last two values).
+constexpr int kPostRec = 8;
+
+// Sums and maxima of a block of any size (a multiple of 32): the sums by the
+// spread tree (6 FP64 additions a lane instead of 15), the maxima only where
+// asked for.  Results in warp 0: sum k in lane 8 k, maximum k in every lane.
+template <int NM>
+__device__ __forceinline__ double blockSumsMaxima(double (&sums)[4], double (&mx)[NM], int nm, double* smem) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  constexpr int R = 4 + NM;
+  double v = warpSpreadSum<double, 4>(sums);
+#pragma unroll
+  for (int k = 0; k < NM; ++k)
+    if (k < nm)
+      for (int o = 16; o > 0; o >>= 1) mx[k] = fmax(mx[k], __shfl_xor_sync(0xffffffffu, mx[k], o));
+  if (lane % 8 == 0) smem[wid * R + lane / 8] = v;
+  if (lane == 0)
+#pragma unroll
+    for (int k = 0; k < NM; ++k) smem[wid * R + 4 + k] = mx[k];
+  __syncthreads();
+  if (wid == 0) {
+    // lane 8 k + j: records j of sum k
+    v = 0;
+    for (int j = lane % 8; j < nw; j += 8) v += smem[j * R + lane / 8];
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+#pragma unroll
+    for (int k = 0; k < NM; ++k)
+      if (k < nm) {
+        double m = lane < nw ? smem[lane * R + 4 + k] : smem[4 + k];
+        for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+        mx[k] = m;
+      }
+  }
+  __syncthreads();
+  return v;
+}
+
+// Cells of the post-solve pass: leastSquares gradient with the boundary values of
+// kBoundaryValues, and the law (linear geometry) or the kinematics F, F^-1, J
+// (total Lagrangian; kPostLawTL finishes that pass, the law needs the global J
+// check first).  mode 0 (constructor): the gradient only.
 template <typename T>
 __global__ void __launch_bounds__(kRowBlock)
 kPost(MeshView mv, Controls c, FieldPtrs f, const T* __restrict__ x, DevState* st,
       double* partials, int mode) {
-  __shared__ double smem[32 * 6];
+  __shared__ double smem[(kRowBlock / 32) * 9];
   {
     const int cs = blockIdx.y;
     f = caseFields(f, cs, mv.nC, mv.nB, mv.nI);
-    caseView(mv, cs);
     x += (size_t)cs * 3 * mv.nC;
     st += cs;
     partials += (size_t)cs * mv.caseRec;
   }
-  if (mode == 1 && !st->caseLive) return;
+  const bool apply = mode == 1;
+  if (apply && !st->caseLive) return;
   const int dc = st->dcur;
-  const bool apply = (mode == 1);
-  // the corrected field D + x, written by kApplyX (mode 1), or D (mode 0)
   const double* U = f.D[apply ? dc ^ 1 : dc];
   const bool relax = c.fieldRelax != 1.0 || c.aitken;
-  double red[6] = {0, 0, 0, 0, 0, 0};  // sum U
-  double mx[3] = {0, 0, 0};            // max|x|, max|U-D0|, max|U|
-  double minJ = 1e300, maxJ = -1e300;
+  double sums[4] = {0, 0, 0, 0};              // sum U
+  double mx[5] = {0, 0, 0, -1e300, -1e300};   // max |x|^2, |U-D0|^2, |U|^2, -min J, max J
   for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < mv.nC; s += gridDim.x * blockDim.x) {
     const V3 Up = ldV(U, s);
-    const bool hasB = mv.browptr[s + 1] > mv.browptr[s];
-    T9 Gold = hasB ? ldT(f.G, s) : zeroT();
-    // leastSquares gradient with the precomputed vectors of the cell's faces
     T9 acc = zeroT();
     for (int e = mv.rowptr[s]; e < mv.rowptr[s + 1]; ++e)
       acc = acc + outer(ldV(mv.lsv, e), ldV(U, mv.col[e]) - Up);
-    // relaxed: the boundary values come from the field as solved, then
-    // relax against their previous values (the cells were relaxed already)
-    const V3 UpSolved = (relax && apply) ? ldV(f.D[dc], s) + ldVT(x, pcgRow(mv, s)) : Up;
-    for (int b = mv.browptr[s]; b < mv.browptr[s + 1]; ++b) {
-      V3 Ub = boundaryValue(mv, c, f, b, UpSolved, Gold);
-      if (relax) {
-        if (apply) {
-          const V3 pb = ldV(f.Ubr, b);
-          if (c.aitken)
-            Ub = aitkenRelax(c, st->iCorr == 0, f.aitA + mv.nC + b, f.aitR + 3 * ((size_t)mv.nC + b),
-                             pb, Ub, mv.btype[b] == 1);
-          else
-            Ub = pb + c.fieldRelax * (Ub - pb);
-        }
-        stV(f.Ubr, b, Ub);
-      }
-      acc = acc + outer(ldV(mv.bls, b), Ub - Up);
-    }
+    for (int b = mv.browptr[s]; b < mv.browptr[s + 1]; ++b)
+      acc = acc + outer(ldV(mv.bls, b), ldV(f.Ub, b) - Up);
     const T9 G = acc;
     stT(f.G, s, G);
-    // boundary gradient: Gb = G + n (snGrad - n.G)
-    for (int b = mv.browptr[s]; b < mv.browptr[s + 1]; ++b) {
-      V3 n = ldV(mv.bn, b);
-      V3 sg;
-      if (mv.btype[b] == 1) {
-        sg = ldV(f.g, b);
-      } else {
-        const V3 Ub = relax ? ldV(f.Ubr, b) : boundaryValue(mv, c, f, b, Up, Gold);
-        sg = mv.bdelta[b] * (Ub - (Up + dotVT(ldV(mv.bk, b), Gold)));
-      }
-      T9 Gb = G + outer(n, sg - dotVT(n, G));
-      stT(f.Gb, b, Gb);
-      if (!c.tl) {
-        S6 sb = mode == 1 ? hooke(c, Gb) : ldS(f.sigb, b);
-        if (mode == 1) stS(f.sigb, b, sb);
-        if (mv.btype[b] == 1) {
-          stV(f.gPrev, b, sg);
-          stV(f.g, b, relaxG(mv, b, tractionSnGrad(mv, c, b, sb, Gb, nullptr, 0), sg));
-        }
-      }
-    }
     if (!c.tl) {
       if (mode == 1) stS(f.sig, s, hooke(c, G));
     } else if (mode == 1) {
@@ -388,17 +424,7 @@ kPost(MeshView mv, Controls c, FieldPtrs f, const T* __restrict__ x, DevState* s
       stT(f.Finv, s, invT(F));
       double J = detT(F);
       f.J[s] = J;
-      minJ = fmin(minJ, J); maxJ = fmax(maxJ, J);
-      for (int b = mv.browptr[s]; b < mv.browptr[s + 1]; ++b) {
-        T9 GDb = ldT(f.GD0b, b) + ldT(f.Gb, b);
-        stT(f.GDb, b, GDb);
-        T9 Fb = transposeT(GDb);
-        Fb.xx += 1.0; Fb.yy += 1.0; Fb.zz += 1.0;
-        stT(f.Finvb, b, invT(Fb));
-        double Jb = detT(Fb);
-        f.Jb[b] = Jb;
-        minJ = fmin(minJ, Jb); maxJ = fmax(maxJ, Jb);
-      }
+      mx[3] = fmax(mx[3], -J); mx[4] = fmax(mx[4], J);
     }
     if (apply) {
       // maxima of squared magnitudes; the square root is taken once at the end
@@ -407,51 +433,161 @@ kPost(MeshView mv, Controls c, FieldPtrs f, const T* __restrict__ x, DevState* s
       mx[0] = fmax(mx[0], magSqr(xs));
       mx[1] = fmax(mx[1], c.tl == 1 ? magSqr(Up) : magSqr(Up - ldV(f.D0, s)));
       mx[2] = fmax(mx[2], magSqr(Up));
-      red[0] += Up.x; red[1] += Up.y; red[2] += Up.z;
+      sums[0] += Up.x; sums[1] += Up.y; sums[2] += Up.z;
       if (!(isfinite(Up.x) && isfinite(Up.y) && isfinite(Up.z))) atomicOr(&st->status, kErrNaN);
     }
   }
   if (mode == 0) return;
-  double sums[3] = {red[0], red[1], red[2]};
-  blockSum<3>(sums, smem);
-  double mxs[5] = {mx[0], mx[1], mx[2], -minJ, maxJ};
-  blockMax<5>(mxs, smem);
-  if (threadIdx.x == 0) {
-    double* p = partials + 8 * (size_t)blockIdx.x;
-    p[0] = sums[0]; p[1] = sums[1]; p[2] = sums[2];
-    p[3] = mxs[0]; p[4] = mxs[1]; p[5] = mxs[2]; p[6] = mxs[3]; p[7] = mxs[4];
+  const double v = blockSumsMaxima<5>(sums, mx, c.tl ? 5 : 3, smem);
+  if (threadIdx.x < 32) {
+    double* p = partials + kPostRec * (size_t)blockIdx.x;
+    const int lane = threadIdx.x;
+    if (lane % 8 == 0 && lane < 24) p[lane / 8] = v;
+    if (lane == 0)
+#pragma unroll
+      for (int k = 0; k < 5; ++k) p[3 + k] = mx[k];
+  }
+}
+
+// The loop condition of the device-resident loops (launchSetLoopCond), by one
+// thread.
+__device__ __forceinline__ void setLoopCond(cudaGraphConditionalHandle h, DevState* st, int nRun,
+                                            int which, int first, unsigned limit) {
+  unsigned* count = which == 0 ? &st[0].loopPcg : &st[0].loopOuter;
+  if (first) *count = 0;
+  else *count += 1;
+  int any = 0;
+  for (int cs = 0; cs < nRun; ++cs) {
+    // a case whose wait gave up or whose field is not finite stops here
+    if (st[cs].status & (kErrTimeout | kErrNaN)) {
+      st[cs].pcgContinue = 0;
+      if (which == 1) st[cs].caseLive = 0;
+      continue;
+    }
+    any |= which == 0 ? st[cs].pcgContinue : st[cs].caseLive;
+  }
+  if (any && *count >= limit) {
+    for (int cs = 0; cs < nRun; ++cs) {
+      st[cs].status |= kErrTimeout;
+      st[cs].pcgContinue = 0;
+      if (which == 1) st[cs].caseLive = 0;
+    }
+    any = 0;
+  }
+  cudaGraphSetConditional(h, any ? 1u : 0u);
+}
+
+// Faces of the post-solve pass, a thread per boundary face: boundary gradient Gb =
+// G + n (snGrad - n.G), then stress and next traction gradient (linear geometry)
+// or kinematics (total Lagrangian).  The block that finishes last adds up the
+// records of the cells and the faces and decides converged(); in a device
+// loop of one case it also sets the corrector loop's condition.
+__global__ void __launch_bounds__(kRowBlock)
+kPostFace(MeshView mv, Controls c, FieldPtrs f, DevState* st, double* partials, int mode, int cellBlocks,
+          LoopCond loop) {
+  __shared__ double smem[(kRowBlock / 32) * 9];
+  {
+    const int cs = blockIdx.y;
+    f = caseFields(f, cs, mv.nC, mv.nB, mv.nI);
+    caseView(mv, cs);
+    st += cs;
+    partials += (size_t)cs * mv.caseRec;
+  }
+  if (mode == 1 && !st->caseLive) return;
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  double mx[5] = {0, 0, 0, -1e300, -1e300};
+  if (b < mv.nB) {
+    const T9 G = ldT(f.G, mv.bcell[b]);
+    const V3 n = ldV(mv.bn, b);
+    const V3 sg = mv.btype[b] == 1 ? ldV(f.g, b) : ldV(f.sgB, b);
+    const T9 Gb = G + outer(n, sg - dotVT(n, G));
+    stT(f.Gb, b, Gb);
+    if (!c.tl) {
+      S6 sb = mode == 1 ? hooke(c, Gb) : ldS(f.sigb, b);
+      if (mode == 1) stS(f.sigb, b, sb);
+      if (mv.btype[b] == 1) {
+        stV(f.gPrev, b, sg);
+        stV(f.g, b, relaxG(mv, b, tractionSnGrad(mv, c, b, sb, Gb, nullptr, 0), sg));
+      }
+    } else if (mode == 1) {
+      T9 GDb = ldT(f.GD0b, b) + Gb;
+      stT(f.GDb, b, GDb);
+      T9 Fb = transposeT(GDb);
+      Fb.xx += 1.0; Fb.yy += 1.0; Fb.zz += 1.0;
+      stT(f.Finvb, b, invT(Fb));
+      double Jb = detT(Fb);
+      f.Jb[b] = Jb;
+      mx[3] = -Jb; mx[4] = Jb;
+    }
+  }
+  if (mode == 0) return;
+  double sums[4] = {0, 0, 0, 0};
+  double* faceRec = partials + kPostRec * (size_t)cellBlocks;
+  if (c.tl) {
+    double m2[2] = {mx[3], mx[4]};
+    blockSumsMaxima<2>(sums, m2, 2, smem);
+    if (threadIdx.x == 0) {
+      faceRec[2 * (size_t)blockIdx.x] = m2[0];
+      faceRec[2 * (size_t)blockIdx.x + 1] = m2[1];
+    }
   }
   if (!lastBlockDone(&st->counter[0], gridDim.x)) return;
-  double S[3], M[5];
-  reducePartials<3>(partials, 8, gridDim.x, S, smem);
-  reducePartialsMax<5>(partials + 3, 8, gridDim.x, M, smem);
-  if (threadIdx.x != 0) return;
-  for (int k = 0; k < 3; ++k) M[k] = sqrt(M[k]);
+  // sums and maxima over the records
+  sums[0] = sums[1] = sums[2] = sums[3] = 0;
+  mx[3] = mx[4] = -1e300;
+  mx[0] = mx[1] = mx[2] = 0;
+  const int nm = c.tl ? 5 : 3;
+  for (int j = threadIdx.x; j < cellBlocks; j += blockDim.x) {
+    double r[kPostRec];
+#pragma unroll
+    for (int k = 0; k < kPostRec; ++k) r[k] = __ldcg(partials + kPostRec * (size_t)j + k);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) { sums[k] += r[k]; mx[k] = fmax(mx[k], r[3 + k]); }
+    if (c.tl) { mx[3] = fmax(mx[3], r[6]); mx[4] = fmax(mx[4], r[7]); }
+  }
+  if (c.tl)
+    for (int j = threadIdx.x; j < (int)gridDim.x; j += blockDim.x) {
+      mx[3] = fmax(mx[3], __ldcg(faceRec + 2 * (size_t)j));
+      mx[4] = fmax(mx[4], __ldcg(faceRec + 2 * (size_t)j + 1));
+    }
+  const double total = blockSumsMaxima<5>(sums, mx, nm, smem);
+  if (threadIdx.x >= 32) return;
+  // lanes 0 .. 2: a maximum's square root; lanes 0, 8, 16: the mean of a component
+  const int lane = threadIdx.x;
+  const double root = sqrt(lane == 0 ? mx[0] : lane == 1 ? mx[1] : mx[2]);
+  if (lane % 8 == 0 && lane < 24) st->xbar[lane / 8] = total / mv.nC;
+  const double m0 = __shfl_sync(0xffffffffu, root, 0), m1 = __shfl_sync(0xffffffffu, root, 1),
+               m2 = __shfl_sync(0xffffffffu, root, 2);
+  if (lane != 0) return;
   st->counter[0] = 0;
-  st->dcur = dc ^ 1;
+  st->dcur = st->dcur ^ 1;
   // converged(): relative displacement residual
-  double denom = M[1];
-  if (denom < 1e-15) denom = fmax(M[2], 1e-15);
-  double relRes = M[0] / denom;
+  double denom = m1;
+  if (denom < 1e-15) denom = fmax(m2, 1e-15);
+  const double relRes = m0 / denom;
   double r2 = 0;
   int maxIt = 0;
+  long long its = 0;
   for (int k = 0; k < 3; ++k) {
-    r2 += st->initRes[k] * st->initRes[k];
-    maxIt = max(maxIt, st->nIter[k]);
-    st->totalLinIters += st->nIter[k];
+    const double ir = st->initRes[k];
+    const int n = st->nIter[k];
+    r2 += ir * ir;
+    maxIt = max(maxIt, n);
+    its += n;
   }
-  double initResMag = sqrt(r2);
+  st->totalLinIters += its;
+  const double initResMag = sqrt(r2);
   st->relRes = relRes;
   st->initResMag = initResMag;
   st->lastMaxIters = maxIt;
-  for (int k = 0; k < 3; ++k) st->xbar[k] = S[k] / mv.nC;
   if (c.tl) {
-    st->minJ = -M[3]; st->maxJ = M[4];
+    const double minJ = -mx[3], maxJ = mx[4];
+    st->minJ = minJ; st->maxJ = maxJ;
     // only the incremental form checks J (nonLinGeomTotalLagSolid.C:203-207)
-    if (c.tl == 1 && !st->enforceLinear && (st->minJ < 0.01 || st->maxJ > 100))
-      st->enforceLinear = 1;
+    if (c.tl == 1 && !st->enforceLinear && (minJ < 0.01 || maxJ > 100)) st->enforceLinear = 1;
   }
   const int iCorr = st->iCorr;
+  const unsigned status = st->status;
   const double materialResidual = 0.0;
   bool conv = false;
   if (iCorr > 1 && materialResidual < c.matTol) {
@@ -461,33 +597,43 @@ kPost(MeshView mv, Controls c, FieldPtrs f, const T* __restrict__ x, DevState* s
   }
   // fmax drops NaN, so a non-finite field can pass the test above: the
   // NaN flag (set by any block's isfinite check) overrides it
-  st->converged = (conv && !(st->status & kErrNaN)) ? 1 : 0;
+  st->converged = (conv && !(status & kErrNaN)) ? 1 : 0;
   st->nCorrDone += 1;
   st->iCorr = iCorr + 1;
-  st->outerContinue = (!conv && iCorr + 1 < c.nCorr) ? 1 : 0;
-  if (st->status & kErrNaN) st->outerContinue = 0;
-  st->caseLive = st->outerContinue;
+  const int go = (!conv && iCorr + 1 < c.nCorr && !(status & kErrNaN)) ? 1 : 0;
+  st->outerContinue = go;
+  st->caseLive = go;
+  if (loop.on) setLoopCond(loop.h, st, 1, 1, 0, loop.limit);
 }
 
 // TL second half: law (with the enforceLinear decision of this corrector),
-// boundary stress and the next traction snGrad.
+// boundary stress and the next traction snGrad; a thread per cell, then (blocks
+// from cellBlocks on) per boundary face.  The faces keep the form of a loop:
+// the compiler then contracts their multiply-adds as it always has, and the
+// loop over the correctors amplifies a last bit of a traction gradient.
 __global__ void __launch_bounds__(kRowBlock)
-kPostLawTL(MeshView mv, Controls c, FieldPtrs f, const DevState* st) {
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= mv.nC) return;
+kPostLawTL(MeshView mv, Controls c, FieldPtrs f, const DevState* st, int cellBlocks) {
   const int el = st->enforceLinear;
-  T9 G = ldT(f.G, s);
-  T9 FL = ldT(f.FL0, s) + transposeT(G);
-  stT(f.FL, s, FL);
-  S6 sg;
-  if (el) {
-    S6 s0 = ldS(f.sig0, s);
-    sg = addI(s0 + (2.0 * c.mu) * devS(symmT(G)), c.K * trT(G));
+  int b0 = 0, b1 = 0;
+  if ((int)blockIdx.x < cellBlocks) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= mv.nC) return;
+    T9 G = ldT(f.G, s);
+    T9 FL = ldT(f.FL0, s) + transposeT(G);
+    stT(f.FL, s, FL);
+    S6 sg;
+    if (el) {
+      S6 s0 = ldS(f.sig0, s);
+      sg = addI(s0 + (2.0 * c.mu) * devS(symmT(G)), c.K * trT(G));
+    } else {
+      sg = neoHookean(c, FL);
+    }
+    stS(f.sig, s, sg);
   } else {
-    sg = neoHookean(c, FL);
+    b0 = (blockIdx.x - cellBlocks) * blockDim.x + threadIdx.x;
+    b1 = b0 < mv.nB ? b0 + 1 : b0;
   }
-  stS(f.sig, s, sg);
-  for (int b = mv.browptr[s]; b < mv.browptr[s + 1]; ++b) {
+  for (int b = b0; b < b1; ++b) {
     T9 Gb = ldT(f.Gb, b);
     T9 FLb = ldT(f.FL0b, b) + transposeT(Gb);
     stT(f.FLb, b, FLb);
@@ -545,8 +691,8 @@ kRhsFace(MeshView mv, Controls c, FieldPtrs f, const DevState* st) {
 template <typename T>
 __global__ void __launch_bounds__(kRowBlock)
 kRhs(MeshView mv, Controls c, FieldPtrs f, T* __restrict__ x, T* __restrict__ r,
-     DevState* st, double* partials) {
-  __shared__ double smem[32 * 6];
+     DevState* st, double* partials, LoopCond loop) {
+  __shared__ double smem[(kRowBlock / 32) * 6];
   {
     const int cs = blockIdx.y;
     f = caseFields(f, cs, mv.nC, mv.nB, mv.nI);
@@ -603,56 +749,65 @@ kRhs(MeshView mv, Controls c, FieldPtrs f, T* __restrict__ x, T* __restrict__ r,
       part[3 + k] += fabs(rr[k]);
     }
   }
-  blockSum<6>(part, smem);
-  if (threadIdx.x == 0) {
-    double* p = partials + 8 * (size_t)blockIdx.x;
-    for (int k = 0; k < 6; ++k) p[k] = part[k];
+  // six sums: a record per block, then over the records by the last block
+  constexpr int NV = 6;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  auto blockTotal = [&](double (&v)[8]) {  // value k in the lanes 4 k .. of warp 0
+    double a = warpSpreadSum<double, 8>(v);
+    if (lane % 4 == 0 && lane / 4 < NV) smem[wid * NV + lane / 4] = a;
+    __syncthreads();
+    if (wid == 0) {
+      a = 0;
+      if (lane / 4 < NV)
+        for (int j = lane % 4; j < nw; j += 4) a += smem[j * NV + lane / 4];
+      for (int o = 2; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    }
+    __syncthreads();
+    return a;
+  };
+  {
+    double v[8] = {part[0], part[1], part[2], part[3], part[4], part[5], 0, 0};
+    const double a = blockTotal(v);
+    if (wid == 0 && lane % 4 == 0 && lane / 4 < NV) partials[8 * (size_t)blockIdx.x + lane / 4] = a;
   }
   if (!lastBlockDone(&st->counter[1], gridDim.x)) return;
-  double S[6];
-  reducePartials<6>(partials, 8, gridDim.x, S, smem);
-  if (threadIdx.x != 0) return;
-  st->counter[1] = 0;
-  int any = 0;
-  for (int k = 0; k < 3; ++k) {
-    double nf = S[k] + 1e-20;
-    st->normFactor[k] = nf;
-    st->initRes[k] = S[3 + k] / nf;
-    st->finalRes[k] = st->initRes[k];
-    st->nIter[k] = 0;
-    st->pending[k] = 0;
-    st->xPend[k] = 0;
-    st->active[k] = (st->initRes[k] < c.tol) ? 0 : 1;
-    st->wArA[k] = 1e20;
-    any |= st->active[k];
+  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (int j = threadIdx.x; j < (int)gridDim.x; j += blockDim.x) {
+    double q[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) q[k] = __ldcg(partials + 8 * (size_t)j + k);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] += q[k];
   }
-  st->pcgContinue = (any && c.maxIter > 0) ? 1 : 0;
+  const double total = blockTotal(v);
+  if (wid != 0) return;
+  // lane k of 3: the component's normFactor and initial residual
+  const double nf = __shfl_sync(0xffffffffu, total, 4 * lane % 32) + 1e-20,
+               sr = __shfl_sync(0xffffffffu, total, (4 * lane + 12) % 32);
+  int act = 0;
+  if (lane < 3) {
+    const double ir = sr / nf;
+    st->normFactor[lane] = nf;
+    st->initRes[lane] = ir;
+    st->finalRes[lane] = ir;
+    st->nIter[lane] = 0;
+    st->pending[lane] = 0;
+    st->xPend[lane] = 0;
+    act = (ir < c.tol) ? 0 : 1;
+    st->active[lane] = act;
+    st->wArA[lane] = 1e20;
+  }
+  const unsigned any = __ballot_sync(0xffffffffu, act != 0);
+  if (lane == 0) {
+    st->counter[1] = 0;
+    st->pcgContinue = (any && c.maxIter > 0) ? 1 : 0;
+    if (loop.on) setLoopCond(loop.h, st, 1, 0, 1, loop.limit);
+  }
 }
 
 __global__ void kSetLoopCond(cudaGraphConditionalHandle h, DevState* st, int nRun, int which,
                              int first, unsigned limit) {
-  unsigned* count = which == 0 ? &st[0].loopPcg : &st[0].loopOuter;
-  if (first) *count = 0;
-  else *count += 1;
-  int any = 0;
-  for (int cs = 0; cs < nRun; ++cs) {
-    // a case whose wait gave up or whose field is not finite stops here
-    if (st[cs].status & (kErrTimeout | kErrNaN)) {
-      st[cs].pcgContinue = 0;
-      if (which == 1) st[cs].caseLive = 0;
-      continue;
-    }
-    any |= which == 0 ? st[cs].pcgContinue : st[cs].caseLive;
-  }
-  if (any && *count >= limit) {
-    for (int cs = 0; cs < nRun; ++cs) {
-      st[cs].status |= kErrTimeout;
-      st[cs].pcgContinue = 0;
-      if (which == 1) st[cs].caseLive = 0;
-    }
-    any = 0;
-  }
-  cudaGraphSetConditional(h, any ? 1u : 0u);
+  setLoopCond(h, st, nRun, which, first, limit);
 }
 
 // pointD after the loop (enhancedVolPointInterpolate.C:351-423 via
@@ -756,34 +911,42 @@ void launchTractionInit(const MeshView& mv, const Controls& c, const FieldPtrs& 
 template <typename T>
 void launchPost(const MeshView& mv, const Controls& c, const FieldPtrs& f, const T* x,
                 DevState* st, double* partials, int mode, cudaStream_t s, LaunchTimer* tm,
-                int nCases, const T* pA, const T* pB) {
-  const int grid = (mv.nC + kRowBlock - 1) / kRowBlock;
+                int nCases, const T* pA, const T* pB, LoopCond loop) {
   TimeScope ts(tm, S4G_K_POST, s);
-  const dim3 g(mv.rowGrid, nCases);
-  if (mode == 1) kApplyX<T><<<g, kRowBlock, 0, s>>>(mv, c, f, const_cast<T*>(x), pA, pB, st);
-  kPost<T><<<g, kRowBlock, 0, s>>>(mv, c, f, x, st, partials, mode);
-  if (c.tl && mode == 1) kPostLawTL<<<grid, kRowBlock, 0, s>>>(mv, c, f, st);
+  const int bd = mv.fvBlock, bB = (mv.nB + bd - 1) / bd;
+  const dim3 g(mv.fvGrid, nCases);
+  if (mode == 1) kApplyX<T><<<g, bd, 0, s>>>(mv, c, f, const_cast<T*>(x), pA, pB, st);
+  if (mv.nB > 0) kBoundaryValues<T><<<dim3(bB, nCases), bd, 0, s>>>(mv, c, f, x, st, mode);
+  kPost<T><<<g, bd, 0, s>>>(mv, c, f, x, st, partials, mode);
+  if (mode == 1 || mv.nB > 0)
+    kPostFace<<<dim3(std::max(1, bB), nCases), bd, 0, s>>>(mv, c, f, st, partials, mode, mv.fvGrid, loop);
+  if (c.tl && mode == 1) {
+    const int cb = (mv.nC + bd - 1) / bd;
+    kPostLawTL<<<cb + bB, bd, 0, s>>>(mv, c, f, st, cb);
+  }
 }
 
 template <typename T>
 void launchRhs(const MeshView& mv, const Controls& c, const FieldPtrs& f, T* x, T* r,
-               DevState* st, double* partials, cudaStream_t s, LaunchTimer* tm, int nCases) {
+               DevState* st, double* partials, cudaStream_t s, LaunchTimer* tm, int nCases,
+               LoopCond loop) {
   TimeScope ts(tm, S4G_K_RHS, s);
-  const dim3 g(mv.rowGrid, nCases);
-  if (mv.nI > 0) kRhsFace<<<g, kRowBlock, 0, s>>>(mv, c, f, st);
-  kRhs<T><<<g, kRowBlock, 0, s>>>(mv, c, f, x, r, st, partials);
+  const int bd = mv.fvBlock;
+  const int fg = std::max(mv.fvGrid, std::min((mv.nI + bd - 1) / bd, mv.fvFaceGrid));
+  if (mv.nI > 0) kRhsFace<<<dim3(fg, nCases), bd, 0, s>>>(mv, c, f, st);
+  kRhs<T><<<dim3(mv.fvGrid, nCases), bd, 0, s>>>(mv, c, f, x, r, st, partials, loop);
 }
 
 template void launchPost<double>(const MeshView&, const Controls&, const FieldPtrs&, const double*,
                                  DevState*, double*, int, cudaStream_t, LaunchTimer*, int,
-                                 const double*, const double*);
+                                 const double*, const double*, LoopCond);
 template void launchPost<float>(const MeshView&, const Controls&, const FieldPtrs&, const float*,
                                 DevState*, double*, int, cudaStream_t, LaunchTimer*, int,
-                                const float*, const float*);
+                                const float*, const float*, LoopCond);
 template void launchRhs<double>(const MeshView&, const Controls&, const FieldPtrs&, double*, double*,
-                                DevState*, double*, cudaStream_t, LaunchTimer*, int);
+                                DevState*, double*, cudaStream_t, LaunchTimer*, int, LoopCond);
 template void launchRhs<float>(const MeshView&, const Controls&, const FieldPtrs&, float*, float*,
-                               DevState*, double*, cudaStream_t, LaunchTimer*, int);
+                               DevState*, double*, cudaStream_t, LaunchTimer*, int, LoopCond);
 
 void launchGather(int n, int width, const int* c2s, const double* in, double* out, cudaStream_t s) {
   long tot = (long)n * width;
