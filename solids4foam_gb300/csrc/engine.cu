@@ -109,10 +109,9 @@ struct EventTimer : LaunchTimer {
 // Largest meshes of the cluster-resident PCG, in rows per CTA of a full cluster,
 // by where the separate kernels are as fast.  Exact DIC: as many as the row
 // vector's memory holds.
-template <typename T>
-constexpr int kResMaxRows(bool local) { return !local ? 16000 : sizeof(T) == 4 ? 2048 : 1280; }
+constexpr int kResMaxRows(bool local) { return !local ? 16000 : 2048; }
 constexpr int kResMaxDiagRows = 16384;
-constexpr int kPartUnroll = 8;  // PCG iterations of a pass of the device loop (part kernels)
+constexpr int kPcgUnroll = 8;  // PCG iterations of a pass of the device loop
 
 struct Engine {
   Ctx* ctx = nullptr;
@@ -668,7 +667,7 @@ struct Engine {
   template <typename T>
   s4g_status ensureResident() {
     Resident<T>& q = resident<T>();
-    if (ctx->profile) return S4G_OK;
+    if (ctx->profile || !residentForm<T>()) return S4G_OK;
     cudaStream_t s = ctx->stream;
     if (!q.tried) {
       q.tried = true;
@@ -701,13 +700,12 @@ struct Engine {
     rv.ring = kResThreads;
     // Exact DIC: the substitutions inside one CTA where all rows fit its memory
     // (a level costs the CTA's barrier, not the cluster's).  Rows per CTA: a
-    // level's cost hardly depends on them, the other phases' time does, and
-    // FP64 arithmetic (2 multiply-adds per cycle and SM) more than FP32's.
+    // level's cost hardly depends on them, the other phases' time does.
     rv.single = !rv.local && resSmemBytes<T>(rv, 0) <= limit;
-    const int rows = sizeof(T) == 8 || !rv.local ? 256 : 1024;
+    const int rows = rv.local ? 1024 : 256;
     rv.C = std::max(1, std::min({kResMaxCtas, (nC + rows - 1) / rows,
                                  rv.local ? hp.nParts : kResMaxCtas}));
-    if (nC > kResMaxCtas * kResMaxRows<T>(rv.local)) return S4G_OK;
+    if (nC > kResMaxCtas * kResMaxRows(rv.local)) return S4G_OK;
     // rows by CTA and level
     std::vector<int> chunk(rv.C + 1, 0), lvl, pos(nC);
     if (rv.local) {
@@ -885,7 +883,7 @@ struct Engine {
       wide = std::max(wide, hp.lvlStart[l + 1] - hp.lvlStart[l]);
     pv.wide = wide > partWalkRows<T>() ? 1 : 0;
     pv.more = (pv.wide || !hp.locSlots) ? 1 : 0;  // (the form for wide levels reads the flag)
-    if (!dHalo) {
+    if (sizeof(T) == 4 && !dHalo) {
       // the entries that lead out of a part: counted, then placed
       int* most;
       S4G_TRY(alloc(&dHaloCnt, (size_t)hp.nParts));
@@ -901,7 +899,7 @@ struct Engine {
       launches += 2;
     }
     pv.haloCap = haloCap; pv.haloCnt = dHaloCnt; pv.halo = dHalo; pv.slot = dSlot;
-    if (pv.capRows + haloCap > 65535) return S4G_OK;
+    if (sizeof(T) == 4 && pv.capRows + haloCap > 65535) return S4G_OK;
     int blocks[2] = {0, 0};
     const cudaError_t e = partPrepare<T>(mv, pv, blocks);
     if (e != cudaSuccess || blocks[0] < 1 || blocks[1] < 1) {
@@ -914,9 +912,11 @@ struct Engine {
       const int waves = (hp.nParts + most - 1) / most;
       pv.grid[k] = (hp.nParts + waves - 1) / waves;
     }
-    T* val;
-    S4G_TRY(alloc(&val, (size_t)kResW * nC));
-    q.pt.val = val;
+    if (sizeof(T) == 4) {
+      T* val;
+      S4G_TRY(alloc(&val, (size_t)kResW * nC));
+      q.pt.val = val;
+    }
     for (int k = 0; k < (pv.more ? 4 : 2); ++k) {
       auto& tb = k < 2 ? q.pt.sweep[k] : q.pt.more[k - 2];
       if constexpr (sizeof(T) == 4) {
@@ -948,9 +948,16 @@ struct Engine {
   // The diagonal preconditioner's iteration has no levels to walk: past some
   // rows the whole device's row kernels are faster than one cluster.
   template <typename T>
-  bool runsResident() {
-    return !ctx->profile && resident<T>().ok &&
-           (lin.preconditioner == S4G_PRECOND_DIC || hp.nC <= kResMaxDiagRows);
+  bool runsResident() { return !ctx->profile && resident<T>().ok && residentForm<T>(); }
+  // The forms it has.  In FP64 the exact DIC only: the corrector loop of the
+  // processor-local DIC (and, less, of the diagonal preconditioner) amplifies a
+  // last bit of a sum over many correctors, and the separate kernels' sums are
+  // the ones results are compared with.
+  template <typename T>
+  bool residentForm() const {
+    const bool dic = lin.preconditioner == S4G_PRECOND_DIC;
+    if (sizeof(T) == 8) return dic && !mv.subdomains;
+    return dic || hp.nC <= kResMaxDiagRows;
   }
   template <typename T>
   cudaError_t resPcg(const Controls& c, const PcgPtrs<T>& p) {
@@ -1241,7 +1248,7 @@ struct Engine {
   template <typename T>
   s4g_status tuneLocal(const Controls& c, const PcgPtrs<T>& p) {
     bool& done = sizeof(T) == 4 ? tuned32 : tuned64;
-    if (runsResident<T>() || runsParts<T>()) return S4G_OK;  // nothing to choose
+    if (runsResident<T>() || (sizeof(T) == 4 && runsParts<T>())) return S4G_OK;  // nothing to choose
     if (done || !autotune) { done = true; return S4G_OK; }
     cudaStream_t s = ctx->stream;
     const size_t n3 = 3 * (size_t)hp.nC;
@@ -1405,16 +1412,16 @@ struct Engine {
     if (!ok || cudaStreamBeginCaptureToGraph(s, pcgBody, nullptr, nullptr, 0, mode) != cudaSuccess)
       return false;
     long long dummy = 0;
-    if (runsParts<T>()) {
-      // several iterations per pass of the loop (a pass costs about 5 us, the
-      // launches after the stop decision about 1 us each)
-      for (int k = 0; k < kPartUnroll; ++k)
-        ok = launchPartIteration<T>(mv, c, parts<T>().pv, parts<T>().pt, p, dState, dPartials, s, nullptr,
-                                    nRun) == cudaSuccess && ok;
-    } else if (mv.subdomains && c.precond == 0)
-      launchLocalIteration<T>(mv, c, p, dState, dPartials, tuning<T>(), s, &dummy, nullptr, nRun);
-    else
-      launchPcgIteration<T>(mv, c, p, dState, dPartials, grid, s, &dummy, nullptr);
+    // several iterations per pass of the loop (a pass costs about 5 us, the
+    // launches after the stop decision about 1 us each)
+    for (int k = 0; k < kPcgUnroll; ++k)
+      if (runsParts<T>())
+        ok = launchPartIteration<T>(mv, c, parts<T>().pv, parts<T>().pt, p, dState, dPartials, tuning<T>(),
+                                    s, nullptr, nRun) == cudaSuccess && ok;
+      else if (mv.subdomains && c.precond == 0)
+        launchLocalIteration<T>(mv, c, p, dState, dPartials, tuning<T>(), s, &dummy, nullptr, nRun);
+      else
+        launchPcgIteration<T>(mv, c, p, dState, dPartials, grid, s, &dummy, nullptr);
     launchSetLoopCond(hPcg, dState, nRun, 0, 0, pcgLimit, s);
     ok = cudaStreamEndCapture(s, &ended) == cudaSuccess && ok;
     (void)tl;
@@ -1463,9 +1470,9 @@ struct Engine {
       for (int i = 0; i < n; ++i) {
         if (tm()) timer.tag = launched++;
         if (runsParts<T>()) {
-          launchPartIteration<T>(mv, c, parts<T>().pv, parts<T>().pt, p, dState, dPartials, ctx->stream,
-                                 tm(), nRun);
-          *count += 2;
+          launchPartIteration<T>(mv, c, parts<T>().pv, parts<T>().pt, p, dState, dPartials, tuning<T>(),
+                                 ctx->stream, tm(), nRun);
+          *count += sizeof(T) == 8 && tuning<T>().uIdx == 2 ? 3 : 2;
         } else if (mv.subdomains && c.precond == 0)
           launchLocalIteration<T>(mv, c, p, dState, dPartials, tuning<T>(), ctx->stream,
                                   count, tm(), nRun);
@@ -1501,9 +1508,8 @@ struct Engine {
   template <typename T>
   long long pcgLaunches(const Controls& c, bool local, long long it) {
     if (runsResident<T>()) return 0;  // (one per corrector)
-    if (runsParts<T>()) return 2 * it + (it + kPartUnroll - 1) / kPartUnroll;
     const int perIt = local ? (tuning<T>().uIdx == 2 ? 3 : 2) : (c.precond == 0 ? 5 : 4);
-    return it * (perIt + 1);
+    return it * perIt + (it + kPcgUnroll - 1) / kPcgUnroll;
   }
 
   // One evolve(): correctors until converged() or nCorrectors.  The inner

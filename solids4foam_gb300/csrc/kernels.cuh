@@ -328,11 +328,13 @@ cudaError_t launchPartTables(const MeshView& mv, const PartView& pv, const doubl
 // Sets the kernels' attributes; blocks[2]: resident CTAs per SM of each.
 template <typename T>
 cudaError_t partPrepare(const MeshView& mv, const PartView& pv, int* blocks);
-// One PCG iteration (two kernels).
+// One PCG iteration (two kernels; in FP64 the product is kernels_local.cu's in the
+// form t names).
 template <typename T>
 cudaError_t launchPartIteration(const MeshView& mv, const Controls& c, const PartView& pv,
                                 const PartPtrs<T>& pt, const PcgPtrs<T>& p, DevState* st,
-                                double* partials, cudaStream_t s, LaunchTimer* tm, int nCases);
+                                double* partials, const LocalTuning& t, cudaStream_t s,
+                                LaunchTimer* tm, int nCases);
 
 // ---- operator product without allocation (noalloc.cu) ------------------------
 // y = A x and x.Ax for k columns of host vectors in caller order, through the

@@ -51,6 +51,7 @@
 
 #include "kernels.cuh"
 #include "pcg_common.cuh"
+#include "part_sums.cuh"
 
 namespace s4g {
 namespace {
@@ -255,94 +256,6 @@ template <typename T>
 __global__ void kLocGather(int n, const int* src, const double* rDa, T* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] = src[i] >= 0 ? (T)rDa[src[i]] : T(0);
-}
-
-// Part records in groups of kLocGroup parts: the CTA whose part completes a
-// group (the last to arrive on the group's counter) sums the group's records
-// in part order by a fixed shuffle tree, and the last CTA of the launch sums
-// the group records -- one round trip each instead of one CTA reading every
-// part record at the end of the launch.
-constexpr int kLocGroup = 32;
-
-__device__ __forceinline__ int locGroupSize(int g, int nParts) {
-  const int n = nParts - g * kLocGroup;
-  return n < kLocGroup ? n : kLocGroup;
-}
-
-// Thread 0: the arrival of `part`'s record (written by this thread) on its
-// group's counter; true if it completes the group.
-__device__ __forceinline__ bool locArrive(unsigned* gcnt, int part, int nParts) {
-  __threadfence();
-  const int g = part / kLocGroup;
-  return atomicAdd(&gcnt[g], 1u) + 1u == (unsigned)locGroupSize(g, nParts);
-}
-
-// One warp: the record (N values) of group g (lane j holds part g*32 + j),
-// and the group's counter back to zero for the next launch.
-template <int N = 6>
-__device__ __forceinline__ void locGroupSum(const double* rec, double* grec, unsigned* gcnt, int g,
-                                            int nParts) {
-  const int lane = threadIdx.x & 31;
-  const int part = g * kLocGroup + lane;
-  __threadfence();
-  double v[N];
-#pragma unroll
-  for (int k = 0; k < N; ++k) v[k] = part < nParts ? __ldcg(rec + 8 * (size_t)part + k) : 0.0;
-#pragma unroll
-  for (int k = 0; k < N; ++k)
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) grec[8 * (size_t)g + k] = v[k];
-    gcnt[g] = 0;
-  }
-}
-
-// The last CTA: the sum of the group records in group order -- lane v of
-// 64 sums groups v, v + 64, ..., then a fixed tree.  Result in thread 0.
-template <int N>
-__device__ __forceinline__ void locGroupsTotal(const double* grec, int nGroups, double (&S)[N],
-                                               double* red) {
-#pragma unroll
-  for (int k = 0; k < N; ++k) S[k] = 0;
-  if (threadIdx.x < 64)
-    for (int g = threadIdx.x; g < nGroups; g += 64)
-#pragma unroll
-      for (int k = 0; k < N; ++k) S[k] += __ldcg(grec + 8 * (size_t)g + k);
-  sum64<N>(S, red);
-}
-
-// End of a preconditioner launch, after the CTA's last part: thread 0
-// reports that part on its group counter (warp 0 sums the group if that
-// completes it); the last CTA sums the group records in group order -- lane
-// v of 64 sums groups v, v + 64, ..., then a fixed tree -- and decides, per
-// component, the residual test of the pending iteration, beta and wArA, and
-// whether the loop goes on.  Block size >= 64.
-__device__ __forceinline__ void locFinish(const MeshView& mv, const Controls& c, DevState* st,
-                                          double* partials, int lastPart, bool anyPend,
-                                          double* red, int* sGroup) {
-  double* grec = partials + mv.locGrpOff;
-  unsigned* gcnt = reinterpret_cast<unsigned*>(grec + 8 * (size_t)mv.locGroups);
-  const int t = (int)threadIdx.x;
-  if (t == 0)
-    *sGroup = (lastPart >= 0 && locArrive(gcnt, lastPart, mv.nParts)) ? lastPart / kLocGroup : -1;
-  __syncthreads();
-  if (*sGroup >= 0 && t < 32) locGroupSum(partials, grec, gcnt, *sGroup, mv.nParts);
-  if (!lastBlockDone(&st->counter[5], gridDim.x)) return;
-  double S[6];
-  locGroupsTotal<6>(grec, mv.locGroups, S, red);
-  if (t >= 32) return;
-  double mine = 0;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const double v = __shfl_sync(0xffffffffu, S[k], 0);
-    if (t == k) mine = v;
-  }
-  if (t == 0) {
-    st->counter[5] = 0;
-    st->locTicket = 0;
-  }
-  pcgDecideBeta(c, st, mine, anyPend);
 }
 
 // Resident blocks the register budget is set for (NT threads, RPT rows per

@@ -16,6 +16,12 @@
 // once, at the end, and the last CTA adds the CTAs' records in order: the order
 // of the sums depends on the mesh, the value type and the device only.
 //
+// In FP64 the corrector loop of some processor-local runs amplifies a last bit of
+// a sum a thousandfold every ten correctors (measured: 1e-13 after 60, 2e-6
+// after 100).  There the preconditioner keeps the sums of kernels_local.cu in
+// their order -- 64 lanes over a part's rows, parts in groups of 32
+// (part_sums.cuh) -- and the product and its sums stay with kernels_local.cu.
+//
 // Parts of rows with at most six neighbours that fit shared memory (in FP32
 // at most 1022 rows: 10-bit columns); others run kernels_local.cu.
 
@@ -23,6 +29,7 @@
 
 #include "kernels.cuh"
 #include "pcg_common.cuh"
+#include "part_sums.cuh"
 #include "sweep.cuh"
 
 namespace s4g {
@@ -34,12 +41,12 @@ template <typename T> struct PartCfg;
 template <> struct PartCfg<float> {
   using Ent = PartEnt;
   static constexpr int kNT = 64, kKeep = 8, kOcc = 6;
-  static constexpr bool kSplit = false;
+  static constexpr bool kSplit = false, kOrdered = false;
 };
 template <> struct PartCfg<double> {
   using Ent = ResEnt<double>;
   static constexpr int kNT = 192, kKeep = 3, kOcc = 3;
-  static constexpr bool kSplit = true;
+  static constexpr bool kSplit = true, kOrdered = true;
 };
 constexpr int kPartSpmvThreads = 128;
 
@@ -116,7 +123,8 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ __align__(16) int4 sDesc[2][2];
   __shared__ V wrec[6 * (NT / 32)];
-  __shared__ double sum[8];
+  __shared__ double sum[12];
+  __shared__ int sGroup;
   const int t = (int)threadIdx.x, cap = pv.capRows;
   // w and its zero row | tables forward, backward | level bounds
   const unsigned uBase = (unsigned)__cvta_generic_to_shared(smraw);
@@ -132,6 +140,11 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
     }
   }
   const unsigned lva = at + 16;  // two empty levels before the first
+  // (ordered sums) the part's residual
+  T* const sr = (T*)(smraw + (at - uBase) + 8 * (mv.maxLevels + 5));
+  double* grec = partials + mv.locGrpOff;
+  unsigned* gcnt = reinterpret_cast<unsigned*>(grec + 8 * (size_t)mv.locGroups);
+  int prev = -1;
   const T* __restrict__ qg = p.q;
   const T* __restrict__ rDg = p.rD;
   T* __restrict__ rg = p.r;
@@ -161,6 +174,9 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
       cpAsync16(&sDesc[buf ^ 1][0], mv.locDesc + 2 * next);
       cpAsync16(&sDesc[buf ^ 1][1], mv.locDesc + 2 * next + 1);
     }
+    // the previous part's record is reported on its group's counter
+    bool done = false;
+    if (C::kOrdered && t == 0 && prev >= 0) done = locArrive(gcnt, prev, nParts);
     // the part's tables in flight while the vectors stream
     for (int i = t; i < nR; i += NT)
 #pragma unroll
@@ -205,6 +221,7 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
               rg[g + k] = rK[j][k];
             }
             w[k] = mulT(rd[j], rK[j][k]);
+            if (C::kOrdered) sr[3 * i + k] = rK[j][k];
           }
           URow<T>::store(uBase + kU * (unsigned)i, w);
         }
@@ -222,6 +239,7 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
           rg[g + k] = rv;
         }
         w[k] = mulT(rd, rv);
+        if (C::kOrdered) sr[3 * i + k] = rv;
       }
       URow<T>::store(uBase + kU * (unsigned)i, w);
     }
@@ -242,7 +260,7 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
         URow<T>::load(uBase + kU * (unsigned)i, w);
         stRow(p.w, (size_t)(pLo + i), w);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
+        for (int k = 0; k < 3 && !C::kOrdered; ++k) {
           wr[k].add(mulT(w[k], rK[j][k]));
           ar[k].add(fabs(rK[j][k]));
         }
@@ -253,13 +271,41 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
       URow<T>::load(uBase + kU * (unsigned)i, w);
       stRow(p.w, (size_t)(pLo + i), w);
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
+      for (int k = 0; k < 3 && !C::kOrdered; ++k) {
         const T r = rg[3 * (size_t)(pLo + i) + k];  // written by this thread
         wr[k].add(mulT(w[k], r));
         ar[k].add(fabs(r));
       }
     }
+    if (C::kOrdered) {
+      // lane l of 64 sums rows l, l + 64, ..., then a fixed tree
+      double d6[6] = {0, 0, 0, 0, 0, 0};
+      if (t < 64)
+        for (int i = t; i < nR; i += 64) {
+          T w[3];
+          URow<T>::load(uBase + kU * (unsigned)i, w);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const T r = sr[3 * i + k];
+            d6[k] = fma((double)w[k], (double)r, d6[k]);
+            d6[3 + k] += fabs((double)r);
+          }
+        }
+      if (t == 0) sGroup = done ? prev / kLocGroup : -1;
+      sum64<6>(d6, sum);
+      if (t == 0) {
+        double* q = partials + 8 * (size_t)part;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) q[k] = d6[k];
+      }
+      if (sGroup >= 0 && t < 32) locGroupSum(partials, grec, gcnt, sGroup, nParts);
+      prev = part;
+    }
     __syncthreads();  // the next part reuses the shared memory
+  }
+  if (C::kOrdered) {
+    locFinish(mv, c, st, partials, prev, anyPend, sum, &sGroup);
+    return;
   }
   V v[8] = {P::of(wr[0]), P::of(wr[1]), P::of(wr[2]), P::of(ar[0]),
             P::of(ar[1]), P::of(ar[2]), P::zero(), P::zero()};
@@ -269,9 +315,9 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
   pcgDecideBeta(c, st, t < 6 ? sum[t] : 0.0, anyPend);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kPartSpmvThreads, (sizeof(T) == 4 ? 8 : 6))
-kPartSpmv(MeshView mv, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p, DevState* st, double* partials) {
+__global__ void __launch_bounds__(kPartSpmvThreads, 8)
+kPartSpmv(MeshView mv, PartView pv, PartPtrs<float> pt, PcgPtrs<float> p, DevState* st, double* partials) {
+  using T = float;
   using P = Part<T>;
   using V = typename P::V;
   constexpr int NT = kPartSpmvThreads, RP = 1, KH = 4;
@@ -490,8 +536,9 @@ __global__ void kPartTables(MeshView mv, PartView pv, const double* val, const d
   const int lo = mv.partStart[part], hi = mv.partStart[part + 1];
   for (int s = lo + threadIdx.x; s < hi; s += blockDim.x) {
     const int e0 = mv.rowptr[s], n = mv.rowptr[s + 1] - e0;
-    for (int k = 0; k < kResW; ++k)
-      const_cast<T*>(out.val)[(size_t)k * mv.nC + s] = k < n ? (T)val[e0 + k] : T(0);
+    if (out.val)
+      for (int k = 0; k < kResW; ++k)
+        const_cast<T*>(out.val)[(size_t)k * mv.nC + s] = k < n ? (T)val[e0 + k] : T(0);
     for (int dir = 0; dir < 2; ++dir) {
       T a[6] = {T(0), T(0), T(0), T(0), T(0), T(0)};
       const unsigned z = (unsigned)pv.zeroRow;
@@ -518,11 +565,10 @@ template <typename T>
 size_t precondSmem(const MeshView& mv, const PartView& pv) {
   const size_t ent = 16 + PartCfg<T>::Ent::kB;
   return URow<T>::kBytes * (size_t)(pv.capRows + 4) + 2 * (pv.more ? 2 : 1) * ent * pv.capRows +
-         8 * (size_t)(mv.maxLevels + 5);
+         8 * (size_t)(mv.maxLevels + 5) + (PartCfg<T>::kOrdered ? 3 * sizeof(T) * pv.capRows : 0);
 }
-template <typename T>
 size_t spmvSmem(const PartView& pv) {
-  return URow<T>::kBytes * (size_t)(pv.capRows + pv.haloCap);
+  return URow<float>::kBytes * (size_t)(pv.capRows + pv.haloCap);
 }
 
 }  // namespace
@@ -536,10 +582,11 @@ int partWalkRows() { return PartCfg<T>::kSplit ? PartCfg<T>::kNT / 3 : PartCfg<T
 
 template <typename T>
 cudaError_t partPrepare(const MeshView& mv, const PartView& pv, int* blocks) {
-  const void* k[2] = {precondKernel<T>(pv), (const void*)kPartSpmv<T>};
-  const size_t sm[2] = {precondSmem<T>(mv, pv), spmvSmem<T>(pv)};
+  const void* k[2] = {precondKernel<T>(pv), (const void*)kPartSpmv};
+  const size_t sm[2] = {precondSmem<T>(mv, pv), spmvSmem(pv)};
   const int nt[2] = {PartCfg<T>::kNT, kPartSpmvThreads};
-  for (int j = 0; j < 2; ++j) {
+  blocks[1] = 1;
+  for (int j = 0; j < (PartCfg<T>::kOrdered ? 1 : 2); ++j) {
     cudaError_t e = setMaxDynamicSmem(k[j]);
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[j], k[j], nt[j], sm[j]);
@@ -566,7 +613,8 @@ cudaError_t launchPartTables(const MeshView& mv, const PartView& pv, const doubl
 template <typename T>
 cudaError_t launchPartIteration(const MeshView& mv, const Controls& c, const PartView& pv,
                                 const PartPtrs<T>& pt, const PcgPtrs<T>& p, DevState* st,
-                                double* partials, cudaStream_t s, LaunchTimer* tm, int nCases) {
+                                double* partials, const LocalTuning& t, cudaStream_t s,
+                                LaunchTimer* tm, int nCases) {
   {
     TimeScope ts(tm, S4G_K_LOC_PRECOND, s);
     void* args[] = {(void*)&mv, (void*)&c, (void*)&pv, (void*)&pt, (void*)&p, (void*)&st, (void*)&partials};
@@ -576,8 +624,9 @@ cudaError_t launchPartIteration(const MeshView& mv, const Controls& c, const Par
   }
   {
     TimeScope ts(tm, S4G_K_LOC_SPMV, s);
-    kPartSpmv<T><<<dim3(pv.grid[1], nCases), kPartSpmvThreads, spmvSmem<T>(pv), s>>>(mv, pv, pt, p, st,
-                                                                                  partials);
+    if constexpr (PartCfg<T>::kOrdered) launchLocalSpmv<T>(mv, p, st, partials, t, s, nCases);
+    else
+      kPartSpmv<<<dim3(pv.grid[1], nCases), kPartSpmvThreads, spmvSmem(pv), s>>>(mv, pv, pt, p, st, partials);
   }
   return cudaGetLastError();
 }
@@ -590,7 +639,8 @@ cudaError_t launchPartIteration(const MeshView& mv, const Controls& c, const Par
                                            const double*, const PartPtrs<T>&, cudaStream_t);     \
   template cudaError_t launchPartIteration<T>(const MeshView&, const Controls&, const PartView&, \
                                               const PartPtrs<T>&, const PcgPtrs<T>&, DevState*,  \
-                                              double*, cudaStream_t, LaunchTimer*, int);
+                                              double*, const LocalTuning&, cudaStream_t,         \
+                                              LaunchTimer*, int);
 S4G_INSTANTIATE(double)
 S4G_INSTANTIATE(float)
 #undef S4G_INSTANTIATE

@@ -370,13 +370,23 @@ kDiagPrecond(MeshView mv, PcgPtrs<T> p, DevState* st, double* partials) {
   if (!lastBlockDone(&st->counter[2], gridDim.x)) return;
   double sum[3];
   reducePartials<3>(partials, 4, gridDim.x, sum, smem);
-  if (threadIdx.x != 0) return;
-  st->counter[2] = 0;
-  for (int k = 0; k < 3; ++k)
-    if (st->active[k]) {
-      st->beta[k] = st->nIter[k] == 0 ? 0.0 : sum[k] / st->wArA[k];
-      st->wArA[k] = sum[k];
+  if (threadIdx.x >= 32) return;
+  const int l = threadIdx.x;  // a lane per component
+  double mine = 0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double v = __shfl_sync(0xffffffffu, sum[k], 0);
+    if (l == k) mine = v;
+  }
+  if (l == 0) st->counter[2] = 0;
+  if (l < 3) {
+    const int act = st->active[l], it = st->nIter[l];
+    const double wa = st->wArA[l];
+    if (act) {
+      st->beta[l] = it == 0 ? 0.0 : mine / wa;
+      st->wArA[l] = mine;
     }
+  }
 }
 
 // p = w (first iteration) or p = w + beta p
@@ -428,17 +438,27 @@ kSpmv(MeshView mv, PcgPtrs<T> p, DevState* st, double* partials) {
   if (!lastBlockDone(&st->counter[3], gridDim.x)) return;
   double sum[3];
   reducePartials<3>(partials, 4, gridDim.x, sum, smem);
-  if (threadIdx.x != 0) return;
-  st->counter[3] = 0;
+  if (threadIdx.x >= 32) return;
+  const int l = threadIdx.x;  // a lane per component
+  double mine = 0;
+#pragma unroll
   for (int k = 0; k < 3; ++k) {
-    if (!st->active[k]) continue;
-    st->wApA[k] = sum[k];
-    if (fabs(sum[k]) / st->normFactor[k] < 1e-300) {  // checkSingularity: stop this component
-      st->active[k] = 0;
-      continue;
+    const double v = __shfl_sync(0xffffffffu, sum[k], 0);
+    if (l == k) mine = v;
+  }
+  if (l == 0) st->counter[3] = 0;
+  if (l < 3) {
+    const int act = st->active[l];
+    const double nf = st->normFactor[l], wa = st->wArA[l];
+    if (act) {
+      st->wApA[l] = mine;
+      if (fabs(mine) < 1e-300 * nf) {  // checkSingularity: stop this component
+        st->active[l] = 0;
+      } else {
+        if (mine <= 0) atomicOr(&st->status, kErrIndefinite);
+        st->alpha[l] = wa / mine;
+      }
     }
-    if (sum[k] <= 0) atomicOr(&st->status, kErrIndefinite);
-    st->alpha[k] = st->wArA[k] / sum[k];
   }
 }
 
@@ -473,21 +493,34 @@ kUpdate(MeshView mv, Controls c, PcgPtrs<T> p, DevState* st, double* partials) {
   if (!lastBlockDone(&st->counter[4], gridDim.x)) return;
   double sum[3];
   reducePartials<3>(partials, 4, gridDim.x, sum, smem);
-  if (threadIdx.x != 0) return;
-  st->counter[4] = 0;
-  int any = 0;
+  if (threadIdx.x >= 32) return;
+  const int l = threadIdx.x;  // a lane per component
+  double mine = 0;
+#pragma unroll
   for (int k = 0; k < 3; ++k) {
-    if (!st->active[k]) continue;
-    const double fr = sum[k] / st->normFactor[k];
-    st->finalRes[k] = fr;
-    st->nIter[k] += 1;
-    const bool conv = fr < c.tol || (c.relTol > 1e-20 && fr < c.relTol * st->initRes[k]);
-    if (!isfinite(fr)) atomicOr(&st->status, kErrNaN);
-    st->active[k] = (!conv && st->nIter[k] < c.maxIter && isfinite(fr)) ? 1 : 0;
-    any |= st->active[k];
+    const double v = __shfl_sync(0xffffffffu, sum[k], 0);
+    if (l == k) mine = v;
   }
-  st->pcgIter += 1;
-  st->pcgContinue = any;
+  if (l == 0) st->counter[4] = 0;
+  int act1 = 0;
+  if (l < 3) {
+    const int act0 = st->active[l], it = st->nIter[l] + 1;
+    const double nf = st->normFactor[l], ir = st->initRes[l];
+    if (act0) {
+      const double fr = mine / nf;
+      st->finalRes[l] = fr;
+      st->nIter[l] = it;
+      const bool conv = fr < c.tol || (c.relTol > 1e-20 && fr < c.relTol * ir);
+      if (!isfinite(fr)) atomicOr(&st->status, kErrNaN);
+      act1 = (!conv && it < c.maxIter && isfinite(fr)) ? 1 : 0;
+      st->active[l] = act1;
+    }
+  }
+  const unsigned any = __ballot_sync(0xffffffffu, act1 != 0);
+  if (l == 0) {
+    st->pcgIter += 1;
+    st->pcgContinue = any != 0;
+  }
 }
 
 template <typename T>

@@ -25,7 +25,11 @@
 // compensated sums per thread, added up in FP64, in an order that depends on
 // the mesh and the value type only.  Rows have at most kResW neighbours
 // (hexahedra, prisms, tetrahedra); other meshes, and those whose shared row
-// vector does not fit, run the separate kernels.
+// vector does not fit, run the separate kernels.  So does FP64 with the
+// processor-local DIC or the diagonal preconditioner: over many correctors a
+// last bit of a sum can grow there (a processor-local 17 x 14 x 14 run: 1e-13
+// after 60 correctors, 2e-6 after 100; with the exact DIC it stays at 1e-16
+// over 200), so those runs keep the order of the sums that they have always had.
 
 #include <algorithm>
 
@@ -568,10 +572,12 @@ __global__ void kResTables(MeshView mv, ResView rv, const int* pos, const double
 template <typename T, int OCC>
 const void* resKernel(int mode) {
   constexpr int NT = kResThreads;
-  return mode == kResExact   ? (const void*)kResPcg<T, NT, kResExact, OCC>
-         : mode == kResLocal ? (const void*)kResPcg<T, NT, kResLocal, OCC>
-         : mode == kResDiag  ? (const void*)kResPcg<T, NT, kResDiag, OCC>
-                             : (const void*)kResPcg<T, NT, kResSingle, OCC>;
+  if constexpr (sizeof(T) == 4) {  // (FP64 has the exact DIC only)
+    if (mode == kResLocal) return (const void*)kResPcg<T, NT, kResLocal, OCC>;
+    if (mode == kResDiag) return (const void*)kResPcg<T, NT, kResDiag, OCC>;
+  }
+  return mode == kResExact ? (const void*)kResPcg<T, NT, kResExact, OCC>
+                           : (const void*)kResPcg<T, NT, kResSingle, OCC>;
 }
 template <typename T>
 const void* resKernelOf(int mode, int occ) {
@@ -626,7 +632,7 @@ template <typename T>
 cudaError_t resPrepare(const ResView& rv, int* clusters) {
   *clusters = 1 << 30;
   for (int occ = 1; occ <= 2; ++occ)
-    for (int diag = 0; diag < 2; ++diag) {
+    for (int diag = 0; diag < (sizeof(T) == 4 ? 2 : 1); ++diag) {
       const void* k = resKernelOf<T>(resMode(diag != 0, rv), occ);
       int dev = 0, optin = 0;
       cudaError_t e = cudaGetDevice(&dev);
