@@ -52,6 +52,7 @@ struct MeshView {
   // batched load cases: a launch's blockIdx.y is the case; per-case data
   // lies caseRec doubles (reduction records) or one field size apart
   long caseRec;
+  long ordOff;         // first record of the resident PCG's ordered sums (orderedSum)
   // within a case's records: the group records of the processor-local
   // preconditioner (8 doubles per group of 32 parts) start locGrpOff
   // doubles in, followed by the groups' arrival counters (unsigned)

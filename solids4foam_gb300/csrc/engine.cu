@@ -411,7 +411,8 @@ struct Engine {
     // records and group counters (zero between launches)
     mv.locGroups = (hp.nParts + 31) / 32;
     mv.locGrpOff = (long)std::max(8 * rowBlocks, 8 * (size_t)hp.nParts);
-    mv.caseRec = (mv.locGrpOff + 8 * (long)mv.locGroups + (mv.locGroups + 1) / 2 + 7) / 8 * 8;
+    mv.ordOff = (mv.locGrpOff + 8 * (long)mv.locGroups + (mv.locGroups + 1) / 2 + 7) / 8 * 8;
+    mv.caseRec = mv.ordOff + (mv.subdomains ? 0 : (long)ordRecords(hp.nParts, nC));
     S4G_TRY(alloc(&dPartials, (size_t)mv.caseRec));
     S4G_CUDA(cudaMemsetAsync(dPartials, 0, sizeof(double) * (size_t)mv.caseRec, s));
     S4G_TRY(alloc(&dOut, 9 * (size_t)nC));
@@ -706,6 +707,8 @@ struct Engine {
     rv.C = std::max(1, std::min({kResMaxCtas, (nC + rows - 1) / rows,
                                  rv.local ? hp.nParts : kResMaxCtas}));
     if (nC > kResMaxCtas * kResMaxRows(rv.local)) return S4G_OK;
+    // the order of the FP64 sums is that of a row per thread of the row kernels
+    if (sizeof(T) == 8 && (long)nC > (long)mv.rowGrid * kRowBlock) return S4G_OK;
     // rows by CTA and level
     std::vector<int> chunk(rv.C + 1, 0), lvl, pos(nC);
     if (rv.local) {
@@ -846,6 +849,23 @@ struct Engine {
       tb.q = a; tb.r = b;
     }
     S4G_CUDA(cudaStreamSynchronize(ctx->stream));  // the host arrays end here
+    rv.pos = q.pos;
+    if (sizeof(T) == 8) {
+      // kSweepSm's thread t sums rows t, t + kOrdLanes, ... of each level, last
+      // level first
+      std::vector<int> step{0}, row;
+      for (int p = 0; p < hp.nParts; ++p)
+        for (int h = 0; h < kOrdLanes; h += 32) {
+          for (int l = hp.lvlOff[p + 1] - 1; l >= hp.lvlOff[p]; --l)
+            for (int i = hp.lvlStart[l] + h; i < hp.lvlStart[l + 1]; i += kOrdLanes)
+              for (int t = 0; t < 32; ++t) row.push_back(i + t < hp.lvlStart[l + 1] ? pos[i + t] : -1);
+          step.push_back((int)(row.size() / 32));
+        }
+      int *dStep, *dRow;
+      S4G_TRY(upload(&dStep, step));
+      S4G_TRY(upload(&dRow, row));
+      rv.ordStep = dStep; rv.ordRow = dRow;
+    }
     rv.chunk = dChunk; rv.lvl = dLvl; rv.col = col; rv.cnt = cnt;
     q.ok = true;
     return S4G_OK;
@@ -965,7 +985,7 @@ struct Engine {
     ResView rv = q.rv;
     const bool many = nRun > 1 || batched;
     if (many) rv.place = q.placeMany;
-    return launchResPcg<T>(mv, c, rv, q.rp, p, dState, ctx->stream, nRun, many);
+    return launchResPcg<T>(mv, c, rv, q.rp, p, dState, dPartials, ctx->stream, nRun, many);
   }
   bool batched = false;  // capturing this mesh's loop into a batch's graph
 

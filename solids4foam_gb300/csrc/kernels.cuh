@@ -244,7 +244,16 @@ struct ResView {
   const int* lvl;      // [C][nLev + 1] first row (in the chunk) of each level; single: [nLev + 1]
   const uint32_t* col;   // [kResW][nC] product columns: CTA << 24 | row in its chunk
   const uint32_t* cnt;   // [nC] entries of the product
+  const int* pos;        // [nC] PCG row of each storage row
+  // (FP64) the order of w.r: per half of a part's kOrdLanes lanes the first of its
+  // steps, per step the PCG row of each of 32 lanes, -1: none
+  const int* ordStep;    // [2 nParts + 1]
+  const int* ordRow;     // [steps][32]
 };
+constexpr int kOrdLanes = 64;  // lanes of a part's w.r sum: the threads of kSweepSm
+// Records of the FP64 form's ordered sums: two of a part, two of 32 storage rows,
+// three values each.
+inline size_t ordRecords(int nParts, int nC) { return 6 * ((size_t)nParts + (nC + 31) / 32); }
 // One sweep's table, by row: three coefficients and a word of packed columns
 // (kernels_resident.cu).
 template <typename T> struct ResSweepTab;
@@ -293,8 +302,8 @@ void launchResTables(const MeshView& mv, const ResView& rv, const int* pos, cons
 // several meshes or cases run at once (two CTAs per SM).
 template <typename T>
 cudaError_t launchResPcg(const MeshView& mv, const Controls& c, const ResView& rv,
-                         const ResPtrs<T>& rp, const PcgPtrs<T>& p, DevState* st, cudaStream_t s,
-                         int nCases, bool many);
+                         const ResPtrs<T>& rp, const PcgPtrs<T>& p, DevState* st, double* partials,
+                         cudaStream_t s, int nCases, bool many);
 
 // ---- processor-local DIC PCG, a CTA per part (kernels_part.cu) ---------------
 // Plan of a mesh for a value type.

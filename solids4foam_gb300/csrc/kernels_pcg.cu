@@ -35,7 +35,7 @@
 namespace s4g {
 namespace {
 
-constexpr int kSweepSmBlock = 64;
+constexpr int kSweepSmBlock = kOrdLanes;
 
 // Poll with relaxed loads (an acquire load per poll would also invalidate the
 // SM's L1 each time), then one acquire fence once the flag is seen.

@@ -21,15 +21,13 @@
 // row's PCG position and the post pass reads x there (MeshView::pcgPos).
 //
 // Every vector entry is computed by the operations of the separate kernels
-// in the same order (in FP32 to the last bit); the global sums are the same
+// in the same order (to the last bit).  The global sums are, in FP32, the same
 // compensated sums per thread, added up in FP64, in an order that depends on
-// the mesh and the value type only.  Rows have at most kResW neighbours
+// the mesh and the value type only; in FP64 they are those of kernels_pcg.cu
+// bit for bit (orderedSum below).  Rows have at most kResW neighbours
 // (hexahedra, prisms, tetrahedra); other meshes, and those whose shared row
 // vector does not fit, run the separate kernels.  So does FP64 with the
-// processor-local DIC or the diagonal preconditioner: over many correctors a
-// last bit of a sum can grow there (a processor-local 17 x 14 x 14 run: 1e-13
-// after 60 correctors, 2e-6 after 100; with the exact DIC it stays at 1e-16
-// over 200), so those runs keep the order of the sums that they have always had.
+// processor-local DIC or the diagonal preconditioner.
 
 #include <algorithm>
 
@@ -118,10 +116,150 @@ __device__ __forceinline__ void clusterSum(typename Part<T>::V (&v)[M], typename
   }
 }
 
+// Barrier between phases: of the cluster, or of its only CTA.
+__device__ __forceinline__ void phaseBarrier(bool cluster) {
+  if (cluster) { clArrive(); clWait(); }
+  else __syncthreads();
+}
+
+// The FP64 form's sums.  The corrector loop can amplify a last bit of w.r or p.q
+// a thousandfold every ten correctors (a processor-local 17 x 14 x 14 run: 1e-13
+// after 60 correctors, 2e-6 after 100; exact DIC, 23 x 16 x 19: 2e-7 after 35), so
+// they are added up in the order of kernels_pcg.cu: w.r by part, 64 lanes that
+// take a row of each level, last level first, then by parts; sum|r| and p.q by
+// storage row, 256 rows a block, then by blocks.  The CTAs own rows in another
+// order, so rows go through global memory (L2), a warp takes 32 lanes of a part or
+// 32 rows, and every CTA adds up the records.  Two cluster barriers a sum instead
+// of one: cube of 8, exact DIC, 26 -> 30 us an iteration.
+__device__ __forceinline__ double warpTree(double v) {  // in lane 0
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  return v;
+}
+// w.r of component k over 32 lanes of a part (w and r by PCG row): the lanes' rows
+// in the order of their sums, a step at a time (ResView::ordRow), the rows of
+// kOrdAhead steps read while those before them are added.
+constexpr int kOrdAhead = 8;
+__device__ __forceinline__ double ordPart(const int* rowOf, int steps, const double* w, const double* r,
+                                          int k) {
+  constexpr int B = kOrdAhead;
+  const int* const at = rowOf + (threadIdx.x & 31);
+  double s = 0, wv[B], rv[B];
+  auto read = [&](int n0, double (&wn)[B], double (&rn)[B]) {
+    int q[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) q[u] = n0 + u < steps ? __ldg(at + 32 * (n0 + u)) : -1;
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      wn[u] = q[u] >= 0 ? __ldcg(w + 3 * (size_t)q[u] + k) : 0.0;
+      rn[u] = q[u] >= 0 ? __ldcg(r + 3 * (size_t)q[u] + k) : 0.0;
+    }
+  };
+  read(0, wv, rv);
+  for (int n = 0; n < steps; n += B) {
+    double wn[B], rn[B];
+    read(n + B, wn, rn);
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+      if (n + u < steps) s = fma(wv[u], rv[u], s);
+#pragma unroll
+    for (int u = 0; u < B; ++u) { wv[u] = wn[u]; rv[u] = rn[u]; }
+  }
+  return warpTree(s);
+}
+// The sums over 32 storage rows of three values a row: value k in lane 8 k
+template <bool ABS>
+__device__ __forceinline__ double ordRows(const int* pos, const double* a, int nC, int g) {
+  const int s = 32 * g + (int)(threadIdx.x & 31);
+  const size_t q = 3 * (size_t)(s < nC ? __ldg(pos + s) : 0);
+  double v[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double x = s < nC ? __ldcg(a + q + k) : 0.0;
+    v[k] = ABS ? fabs(x) : x;
+  }
+  return warpSpreadSum<double, 4>(v);
+}
+// The sum over the row records, of component k, blocks 32 h ... (and every 256th
+// after them)
+__device__ __forceinline__ double ordBlocks(const double* rec, int nC, int k, int h) {
+  const int nB = (nC + kRowBlock - 1) / kRowBlock, nG = (nC + 31) / 32;
+  double v = 0;
+  for (int b = 32 * h + (int)(threadIdx.x & 31); b < nB; b += kRowBlock) {
+    double x[kRowBlock / 32], t = 0;
+#pragma unroll
+    for (int j = 0; j < kRowBlock / 32; ++j) {
+      const int g = b * (kRowBlock / 32) + j;
+      x[j] = g < nG ? __ldcg(rec + 3 * (size_t)g + k) : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < kRowBlock / 32; ++j) t += x[j];
+    v += t;
+  }
+  return warpTree(v);
+}
+// The sum over the part records of component k
+__device__ __forceinline__ double ordParts(const double* rec, int nParts, int k) {
+  const int lane = (int)(threadIdx.x & 31);
+  double b = 0;
+  for (int j = 0; 32 * j < nParts && j < 8; ++j) {
+    double a = 0;
+    for (int p = lane + 32 * j; p < nParts; p += 256) {
+      const double x = __ldcg(rec + 6 * (size_t)p + k), y = __ldcg(rec + 6 * (size_t)p + 3 + k);
+      a += x + y;
+    }
+    b += a;
+  }
+  return warpTree(b);
+}
+// DOTS: w.r by part and sum|r| (w, r by PCG row) into out[0..5]; else the terms w by
+// storage row into out[0..2].  The rows' values are written; out is complete for the
+// lanes 0 .. 2 of warp 0.
+template <int NT, bool DOTS>
+__device__ __forceinline__ void orderedSum(const MeshView& mv, const ResView& rv, const double* w,
+                                           const double* r, double* rec, double* blk, double* out,
+                                           int C, unsigned rank, bool cluster) {
+  constexpr int W = NT / 32;
+  const int lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5;
+  const int nG = (mv.nC + 31) / 32, nP = DOTS ? 6 * mv.nParts : 0;
+  double* const rows = rec + 6 * (size_t)mv.nParts + (DOTS ? 0 : 3 * (size_t)nG);
+  phaseBarrier(cluster);
+  for (int q = (int)rank + C * wid; q < nP + nG; q += C * W) {
+    if (q < nP) {
+      const int task = q / 3, n0 = rv.ordStep[task];
+      const double s = ordPart(rv.ordRow + 32 * (size_t)n0, rv.ordStep[task + 1] - n0, w, r, q % 3);
+      if (lane == 0) rec[q] = s;
+    } else {
+      const double s = ordRows<DOTS>(rv.pos, DOTS ? r : w, mv.nC, q - nP);
+      if ((lane & 7) == 0 && lane < 24) rows[3 * (size_t)(q - nP) + (lane >> 3)] = s;
+    }
+  }
+  phaseBarrier(cluster);
+  const int nB = (mv.nC + kRowBlock - 1) / kRowBlock, nH = nB < kRowBlock ? (nB + 31) / 32 : W;
+  for (int q = wid; q < (DOTS ? 3 : 0) + 3 * nH; q += W) {
+    if (DOTS && q < 3) {
+      const double s = ordParts(rec, mv.nParts, q);
+      if (lane == 0) blk[24 + q] = s;
+    } else {
+      const int k = (q - (DOTS ? 3 : 0)) % 3, h = (q - (DOTS ? 3 : 0)) / 3;
+      const double s = ordBlocks(rows, mv.nC, k, h);
+      if (lane == 0) blk[3 * h + k] = s;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    double s = 0;
+    for (int h = 0; h < nH; ++h) s += blk[3 * h + lane];
+    out[(DOTS ? 3 : 0) + lane] = s;
+    if (DOTS) out[lane] = blk[24 + lane];
+  }
+}
+
 // Scalars of the iteration, in shared memory, decided by warp 0.
 template <typename T>
 struct ResScalars {
   double sum[8];
+  double blk[27];  // (ordered sums)
   double norm[3], lim[3], last[3], wArA[3], alpha[3], beta[3];
   T alphaT[3], betaT[3];  // in the value type (a conversion is an FP64 operation)
   int active[3], pend[3], nIter[3];
@@ -129,22 +267,19 @@ struct ResScalars {
   unsigned status;
 };
 
-// Barrier between phases: of the cluster, or of its only CTA.
-__device__ __forceinline__ void phaseBarrier(bool cluster) {
-  if (cluster) { clArrive(); clWait(); }
-  else __syncthreads();
-}
-
 // OCC: CTAs per SM the registers are limited to: 1 for a single solve, 2 where
 // several meshes or load cases run at once (a tenth slower alone, and twice the
 // clusters on the device).  Both compute the same bits.
 template <typename T, int NT, int MODE, int OCC>
 __global__ void __launch_bounds__(NT, OCC)
-kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevState* st) {
+kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevState* st,
+        double* partials) {
+  constexpr bool ORD = sizeof(T) == 8;
   using P = Part<T>;
   using V = typename P::V;
   p = casePcg(p, blockIdx.y, mv.nC);
   st += blockIdx.y;
+  double* const ordRec = partials + (size_t)blockIdx.y * mv.caseRec + mv.ordOff;
   if (!st->pcgContinue) return;  // the same in every CTA: rank 0 writes it at the end
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ ResScalars<T> sc;
@@ -174,6 +309,7 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
   T *rg = p.r + 3 * (size_t)base, *qg = p.q + 3 * (size_t)base, *pg = p.p + 3 * (size_t)base,
     *xg = p.x + 3 * (size_t)base;
   T* const rGlob = rg;
+  T* const wGlob = p.w + 3 * (size_t)base;
   T* const xGlob = xg;
   if (rv.place & 1) {
     const size_t b = sizeof(T) * 3 * (size_t)mr;
@@ -239,8 +375,7 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
   if (t < 3) {
     const double nf = st->normFactor[t], ir = st->initRes[t];
     sc.norm[t] = nf;
-    // sum|r| / norm < tolerance or relTol * initial
-    sc.lim[t] = fmax(c.tol, c.relTol > 1e-20 ? c.relTol * ir : 0.0) * nf;
+    sc.lim[t] = pcgLimit(c, ir);
     sc.last[t] = ir * nf;
     sc.wArA[t] = st->wArA[t]; sc.alpha[t] = 0; sc.beta[t] = 0; sc.alphaT[t] = T(0); sc.betaT[t] = T(0);
     sc.active[t] = st->active[t]; sc.pend[t] = 0; sc.nIter[t] = 0;
@@ -291,7 +426,7 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
               rr[h][k] = fmaT(-al[k], qv[h][k], rr[h][k]);
               rg[3 * i + k] = rr[h][k];
             }
-            ar[k].add(fabs(rr[h][k]));
+            if (!ORD) ar[k].add(fabs(rr[h][k]));
             w[k] = mulT(rd[h], rr[h][k]);
             if (MODE == kResDiag) wr[k].add(mulT(w[k], rr[h][k]));
           }
@@ -320,10 +455,20 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
         } else {
           URow<T>::load(uBase + kU * i, w);
         }
+        if (ORD) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) wr[k].add(mulT(w[k], rg[3 * i + k]));
+          for (int k = 0; k < 3; ++k) {
+            wGlob[3 * (size_t)i + k] = w[k];
+            if (rv.place & 1) rGlob[3 * (size_t)i + k] = rg[3 * i + k];
+          }
+        } else {
+#pragma unroll
+          for (int k = 0; k < 3; ++k) wr[k].add(mulT(w[k], rg[3 * i + k]));
+        }
       }
-    {
+    if constexpr (ORD) {
+      orderedSum<NT, true>(mv, rv, p.w, p.r, ordRec, sc.blk, sc.sum, C, rank, cluster);
+    } else {
       V v[8] = {P::of(wr[0]), P::of(wr[1]), P::of(wr[2]), P::of(ar[0]),
                 P::of(ar[1]), P::of(ar[2]), P::zero(), P::zero()};
       clusterSum<T, NT, 6>(v, wrec, rec0, sc.sum, C, rank, cluster);
@@ -342,7 +487,7 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
           sc.last[t] = s;
           sc.nIter[t] = ++it;
           if (!isfinite(s)) bad = kErrNaN;
-          act = (!(s < sc.lim[t]) && it < c.maxIter && isfinite(s)) ? 1 : 0;
+          act = (!pcgConverged(s, sc.norm[t], sc.lim[t]) && it < c.maxIter && isfinite(s)) ? 1 : 0;
           sc.active[t] = act;
         }
         if (act) {
@@ -440,12 +585,15 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
 #pragma unroll
           for (int k = 0; k < 3; ++k) {
             if (act[k]) qg[3 * i + k] = y[k];
-            pq[k].add(mulT(y[k], v[k]));
+            if (ORD) wGlob[3 * (size_t)i + k] = mulT(y[k], v[k]);
+            else pq[k].add(mulT(y[k], v[k]));
           }
         }
       }
     }
-    {
+    if constexpr (ORD) {
+      orderedSum<NT, false>(mv, rv, p.w, nullptr, ordRec, sc.blk, sc.sum, C, rank, cluster);
+    } else {
       V v[4] = {P::of(pq[0]), P::of(pq[1]), P::of(pq[2]), P::zero()};
       clusterSum<T, NT, 3>(v, wrec, rec1, sc.sum, C, rank, cluster);
     }
@@ -656,11 +804,12 @@ cudaError_t resPrepare(const ResView& rv, int* clusters) {
 
 template <typename T>
 cudaError_t launchResPcg(const MeshView& mv, const Controls& c, const ResView& rv,
-                         const ResPtrs<T>& rp, const PcgPtrs<T>& p, DevState* st, cudaStream_t s,
-                         int nCases, bool many) {
+                         const ResPtrs<T>& rp, const PcgPtrs<T>& p, DevState* st, double* partials,
+                         cudaStream_t s, int nCases, bool many) {
   cudaLaunchAttribute at[1];
   const cudaLaunchConfig_t cf = resConfig<T>(rv, nCases, s, at);
-  void* args[] = {(void*)&mv, (void*)&c, (void*)&rv, (void*)&rp, (void*)&p, (void*)&st};
+  void* args[] = {(void*)&mv, (void*)&c, (void*)&rv, (void*)&rp, (void*)&p, (void*)&st,
+                  (void*)&partials};
   return cudaLaunchKernelExC(&cf, resKernelOf<T>(resMode(c.precond != 0, rv), many ? 2 : 1), args);
 }
 
@@ -679,7 +828,7 @@ void launchResTables(const MeshView& mv, const ResView& rv, const int* pos, cons
   template cudaError_t resPrepare<T>(const ResView&, int*);                                    \
   template cudaError_t launchResPcg<T>(const MeshView&, const Controls&, const ResView&,       \
                                        const ResPtrs<T>&, const PcgPtrs<T>&, DevState*,        \
-                                       cudaStream_t, int, bool);                               \
+                                       double*, cudaStream_t, int, bool);                      \
   template void launchResTables<T>(const MeshView&, const ResView&, const int*, const double*, \
                                    const double*, const double*, const double*, bool,          \
                                    const ResPtrs<T>&, cudaStream_t);

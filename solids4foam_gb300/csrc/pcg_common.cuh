@@ -37,6 +37,21 @@ template <> struct Acc<float> {
   __device__ __forceinline__ double value() const { return (double)s + (double)c; }
 };
 
+// sum|r| / normFactor < the limit (tolerance, or relTol * the initial residual),
+// as that quotient compares, but divided only where rounding could decide (an FP64
+// division takes 564 cycles of the chain).
+__device__ __forceinline__ double pcgLimit(const Controls& c, double initRes) {
+  return fmax(c.tol, c.relTol > 1e-20 ? c.relTol * initRes : 0.0);
+}
+__device__ __forceinline__ bool pcgConverged(double s, double norm, double lim) {
+  const double b = lim * norm;
+  if (b > 1e-290) {
+    if (s < b * (1 - 4e-15)) return true;
+    if (s > b * (1 + 4e-15)) return false;
+  }
+  return s / norm < lim;
+}
+
 // End of a processor-local preconditioner launch, by warp 0 of its last CTA:
 // S = w.r of the components, then sum|r| (S[k] in lane k and k + 3 for lanes
 // 0 .. 5 of `mine`).  Per component the residual test of the pending iteration,
@@ -55,8 +70,7 @@ __device__ __forceinline__ void pcgDecideBeta(const Controls& c, DevState* st, d
     if (pend) {
       st->pending[l] = 0;
       st->nIter[l] = ++it;
-      // sum|r| / normFactor < tolerance, or relTol * the initial one
-      const bool conv = rs < c.tol * nf || (c.relTol > 1e-20 && rs < c.relTol * ir * nf);
+      const bool conv = pcgConverged(rs, nf, pcgLimit(c, ir));
       const bool fin = isfinite(rs);
       if (!fin) atomicOr(&st->status, kErrNaN);
       act = (!conv && it < c.maxIter && fin) ? 1 : 0;
