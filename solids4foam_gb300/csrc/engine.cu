@@ -111,6 +111,7 @@ struct EventTimer : LaunchTimer {
 // vector's memory holds.
 constexpr int kResMaxRows(bool local) { return !local ? 16000 : 2048; }
 constexpr int kResMaxDiagRows = 16384;
+constexpr int kLoopMinRows = 16384;  // (loopMesh)
 constexpr int kPcgUnroll = 8;  // PCG iterations of a pass of the device loop
 
 struct Engine {
@@ -168,11 +169,13 @@ struct Engine {
   template <typename T>
   struct Parts {
     bool tried = false, ok = false, valid = false;
+    bool loop = false;  // all parts resident at once: the loop in one launch
     PartView pv{};
     PartPtrs<T> pt{};
   };
   Parts<double> parts64;
   Parts<float> parts32;
+  LoopPtrs lp;
   int *dHaloCnt = nullptr, *dHalo = nullptr, haloCap = 0;
   unsigned short* dSlot = nullptr;
   template <typename T>
@@ -876,7 +879,8 @@ struct Engine {
   template <typename T>
   s4g_status ensureParts() {
     Parts<T>& q = parts<T>();
-    if (!mv.subdomains || lin.preconditioner != S4G_PRECOND_DIC || runsResident<T>()) return S4G_OK;
+    if (!mv.subdomains || lin.preconditioner != S4G_PRECOND_DIC || (runsResident<T>() && !loopMesh<T>()))
+      return S4G_OK;
     if (!q.tried) {
       q.tried = true;
       S4G_TRY(planParts<T>(q));
@@ -932,6 +936,17 @@ struct Engine {
       const int waves = (hp.nParts + most - 1) / most;
       pv.grid[k] = (hp.nParts + waves - 1) / waves;
     }
+    if constexpr (sizeof(T) == 4) {
+      int per = 0;
+      if (partLoopPrepare(mv, pv, &per) == cudaSuccess) q.loop = hp.nParts <= per * ctx->numSMs;
+      else cudaGetLastError();
+    }
+    if (q.loop && !lp.w) {
+      const size_t n = (size_t)nC + partLoopPackets(hp.nParts);
+      S4G_TRY(alloc(&lp.w, n));
+      S4G_CUDA(cudaMemsetAsync(lp.w, 0, sizeof(uint4) * n, s));
+      lp.rec = lp.w + nC;
+    }
     if (sizeof(T) == 4) {
       T* val;
       S4G_TRY(alloc(&val, (size_t)kResW * nC));
@@ -957,6 +972,17 @@ struct Engine {
     return mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC && !runsResident<T>() && parts<T>().ok;
   }
 
+  // ... and their loop as one launch: a single case on the device alone (several
+  // cases together have more parts than fit at once).
+  template <typename T>
+  bool runsPartLoop() { return runsParts<T>() && parts<T>().loop && nRun == 1 && !ctx->profile; }
+  template <typename T>
+  cudaError_t partLoop(const Controls& c, const PcgPtrs<T>& p) {
+    if constexpr (sizeof(T) == 4)
+      return launchPartLoop(mv, c, parts<T>().pv, parts<T>().pt, lp, p, dState, ctx->stream);
+    else return cudaErrorNotSupported;
+  }
+
   // The mesh as the field passes of a solve of type T see it: with the
   // resident PCG's row order, where that runs.
   template <typename T>
@@ -968,7 +994,18 @@ struct Engine {
   // The diagonal preconditioner's iteration has no levels to walk: past some
   // rows the whole device's row kernels are faster than one cluster.
   template <typename T>
-  bool runsResident() { return !ctx->profile && resident<T>().ok && residentForm<T>(); }
+  bool runsResident() {
+    return !ctx->profile && resident<T>().ok && residentForm<T>() && !(loopMesh<T>() && parts<T>().loop);
+  }
+  // Where kPartLoop takes over from the resident PCG: one solve at a time, and
+  // more rows than the cluster's 16 SMs are as fast for (30 correctors of 24^3
+  // cells 12.6 ms resident, 14.9 as a part per CTA; 28^3 18.6 and 16.8; 32^3 21.7
+  // and 18.8).
+  template <typename T>
+  bool loopMesh() const {
+    return sizeof(T) == 4 && mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC && nRun == 1 &&
+           !batched && hp.nC > kLoopMinRows;
+  }
   // The forms it has.  In FP64 the exact DIC only: the corrector loop of the
   // processor-local DIC (and, less, of the diagonal preconditioner) amplifies a
   // last bit of a sum over many correctors, and the separate kernels' sums are
@@ -1400,7 +1437,7 @@ struct Engine {
     cudaGraphConditionalHandle hOut, hPcg{};
     if (cudaGraphConditionalHandleCreate(&hOut, g, 0, cudaGraphCondAssignDefault) != cudaSuccess)
       return false;
-    if (!runsResident<T>() &&
+    if (!runsResident<T>() && !runsPartLoop<T>() &&
         cudaGraphConditionalHandleCreate(&hPcg, g, 0, cudaGraphCondAssignDefault) != cudaSuccess)
       return false;
     const unsigned outerLimit = (unsigned)c.nCorr + 4, pcgLimit = (unsigned)c.maxIter + 4;
@@ -1413,14 +1450,14 @@ struct Engine {
     if (!ok || cudaStreamBeginCaptureToGraph(s, outerBody, nullptr, nullptr, 0, mode) != cudaSuccess)
       return false;
     const MeshView fv = fieldView<T>();
-    const bool res = runsResident<T>();
+    const bool res = runsResident<T>() || runsPartLoop<T>();
     // of one case, the kernels that decide a loop set its condition
     const bool one = nRun == 1;
     LoopCond cOut{one ? 1 : 0, outerLimit, hOut}, cPcg{one && !res ? 1 : 0, pcgLimit, hPcg};
     launchRhs<T>(fv, c, f, p.x, p.r, dState, dPartials, s, nullptr, nRun, cPcg);
     if (res) {
       // the PCG loop of the corrector is one launch
-      ok = resPcg<T>(c, p) == cudaSuccess;
+      ok = (runsResident<T>() ? resPcg<T>(c, p) : partLoop<T>(c, p)) == cudaSuccess;
     } else {
       if (!one) launchSetLoopCond(hPcg, dState, nRun, 0, 1, pcgLimit, s);
       ok = addWhile(s, hPcg, &pcgBody);
@@ -1478,8 +1515,8 @@ struct Engine {
   s4g_status pcgLoop(const Controls& c, const PcgPtrs<T>& p, int grid) {
     // Iterations are launched in growing batches; the launches after the
     // device's stop decision return at once.
-    if (runsResident<T>()) {
-      S4G_CUDA(resPcg<T>(c, p));
+    if (runsResident<T>() || runsPartLoop<T>()) {
+      S4G_CUDA(runsResident<T>() ? resPcg<T>(c, p) : partLoop<T>(c, p));
       launches++;
       return readState();
     }
@@ -1527,7 +1564,7 @@ struct Engine {
   // Kernels that a device loop launched for `it` PCG iterations.
   template <typename T>
   long long pcgLaunches(const Controls& c, bool local, long long it) {
-    if (runsResident<T>()) return 0;  // (one per corrector)
+    if (runsResident<T>() || runsPartLoop<T>()) return 0;  // (one per corrector)
     const int perIt = local ? (tuning<T>().uIdx == 2 ? 3 : 2) : (c.precond == 0 ? 5 : 4);
     return it * perIt + (it + kPcgUnroll - 1) / kPcgUnroll;
   }
@@ -1547,7 +1584,7 @@ struct Engine {
         S4G_CUDA(cudaGetLastError());
         S4G_TRY(readState());
         const bool local = mv.subdomains && c.precond == 0;
-        launches += 1 + (long long)(hState->nCorrDone - corr0) * ((tl ? 7 : 6) + (runsResident<T>() ? 1 : 0)) +
+        launches += 1 + (long long)(hState->nCorrDone - corr0) * ((tl ? 7 : 6) + (runsResident<T>() || runsPartLoop<T>() ? 1 : 0)) +
                     pcgLaunches<T>(c, local, hState->pcgIter - it0);
         ranOnDevice = true;
         return S4G_OK;

@@ -337,6 +337,20 @@ cudaError_t launchPartTables(const MeshView& mv, const PartView& pv, const doubl
 // Sets the kernels' attributes; blocks[2]: resident CTAs per SM of each.
 template <typename T>
 cudaError_t partPrepare(const MeshView& mv, const PartView& pv, int* blocks);
+// 16-byte packets that the CTAs of kPartLoop exchange: w of a row; sums of the
+// CTAs, results and the count of sums (partLoopPackets of them).  Zero before
+// the first launch, used by that kernel alone.
+struct LoopPtrs {
+  uint4* w = nullptr;
+  uint4* rec = nullptr;
+};
+size_t partLoopPackets(int nParts);
+// The PCG loop of a corrector in one cooperative launch, a CTA per part, FP32
+// (blocks: resident CTAs per SM, 0 if the parts are too large for it).
+cudaError_t partLoopPrepare(const MeshView& mv, const PartView& pv, int* blocks);
+cudaError_t launchPartLoop(const MeshView& mv, const Controls& c, const PartView& pv,
+                           const PartPtrs<float>& pt, const LoopPtrs& lp, const PcgPtrs<float>& p,
+                           DevState* st, cudaStream_t s);
 // One PCG iteration (two kernels; in FP64 the product is kernels_local.cu's in the
 // form t names).
 template <typename T>

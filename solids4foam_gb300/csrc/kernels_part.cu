@@ -472,6 +472,386 @@ kPartSpmv(MeshView mv, PartView pv, PartPtrs<float> pt, PcgPtrs<float> p, DevSta
   pcgDecideAlpha(st, t < 3 ? sum[t] : 0.0, pb);
 }
 
+// ---- the whole loop of a corrector in one launch ---------------------------------
+// Meshes whose parts are all resident at once (a CTA per part; FP32): the
+// launches of kPartPrecond and kPartSpmv, their reading of the state and their
+// ends take longer than a part's work, so one cooperative launch runs the PCG
+// loop of a corrector.  r, x, p and q stay in registers, the tables in shared
+// memory; the part's halo keeps its p in shared memory and needs only w from
+// other parts once per iteration.
+//
+// What CTAs tell one another goes through 16-byte packets that carry their own
+// tag (the count of sums so far): a reader polls the packet itself, so neither a
+// counter nor a fence stands between a value and its use.  Rows publish w; a CTA
+// publishes its part of a sum, CTA 0 adds the parts up, decides and publishes the
+// result in kLoopCopies lines.  (With a counter, fences and the last CTA deciding
+// on the state in memory a sum took 7 us of a 27 us iteration of 512 parts.)  A
+// packet is written again only after its readers have taken part in a later sum.
+constexpr int kLoopThreads = 128, kLoopRows = 4, kLoopWalk = 64;
+constexpr int kLoopMaxRows = kLoopThreads * kLoopRows;
+constexpr int kLoopAhead = 2;  // CTAs whose packets a thread of CTA 0 has in flight
+constexpr int kLoopCopies = 32, kLoopLine = 8;  // result packets, 128 bytes apart
+
+__device__ __forceinline__ uint4 ldPacket(const uint4* p) {
+  unsigned long long a, b;
+  asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+               : "=l"(a), "=l"(b) : "l"(p) : "memory");
+  return make_uint4((unsigned)a, (unsigned)(a >> 32), (unsigned)b, (unsigned)(b >> 32));
+}
+__device__ __forceinline__ void stPacket(uint4* p, unsigned x, unsigned y, unsigned z, unsigned w) {
+  const unsigned long long a = x | (unsigned long long)y << 32, b = z | (unsigned long long)w << 32;
+  asm volatile("{ .reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t; }"
+               ::"l"(p), "l"(a), "l"(b) : "memory");
+}
+// The packet with this tag, after at most limit polls; false if it did not come.
+// shift: bits of the last word below the tag.
+__device__ __forceinline__ bool waitPacket(const uint4* p, unsigned tag, int shift, int limit, uint4& v) {
+  v = ldPacket(p);
+  for (int it = 0; (v.w ^ tag) >> shift; v = ldPacket(p))
+    if (++it > limit) return false;
+  return true;
+}
+
+// All CTAs' sums of N values.  A CTA's packets: the first parts of three values'
+// compensated sums, their second parts, the same of the next three.  CTA 0 leaves
+// the sums in its warp 0 (value k in lane k) and returns whether all came.
+template <int N, int M>
+__device__ __forceinline__ bool gridPut(float2 (&v)[M], uint4* rec, float2* wrec, unsigned tag, int limit,
+                                        double& mine) {
+  using P = Part<float>;
+  constexpr int NT = kLoopThreads, W = NT / 32, G = 32 / M, Q = 2 * N / 3;
+  const int t = (int)threadIdx.x, lane = t & 31, wid = t >> 5, k = lane / G, g = lane % G;
+  const int n = (int)gridDim.x;
+  const float2 s = warpSpreadSum<float, M>(v);
+  if (k < N && g == 0) wrec[wid * N + k] = s;
+  __syncthreads();
+  if (wid == 0) {
+    const float2 a = warpRecords<float, N, M>(wrec, W);
+    unsigned b[3];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      const int from = (3 * ((lane % Q) >> 1) + m) * G;
+      const float x = __shfl_sync(0xffffffffu, a.x, from), y = __shfl_sync(0xffffffffu, a.y, from);
+      b[m] = __float_as_uint((lane & 1) ? y : x);
+    }
+    if (lane < Q) stPacket(rec + (size_t)lane * n + blockIdx.x, b[0], b[1], b[2], tag);
+  }
+  if (blockIdx.x != 0) return true;
+  // thread t adds up the CTAs t, t + NT, ..., kLoopAhead at a time
+  bool ok = true;
+#pragma unroll
+  for (int m = 0; m < M; ++m) v[m] = P::zero();
+  for (int j0 = t; j0 < n; j0 += kLoopAhead * NT) {
+    uint4 x[kLoopAhead][Q];
+#pragma unroll
+    for (int u = 0; u < kLoopAhead; ++u)
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+        x[u][q] = j0 + u * NT < n ? ldPacket(rec + (size_t)q * n + j0 + u * NT) : make_uint4(0, 0, 0, tag);
+#pragma unroll
+    for (int u = 0; u < kLoopAhead; ++u)
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+        if (x[u][q].w != tag)
+          ok = waitPacket(rec + (size_t)q * n + j0 + u * NT, tag, 0, limit, x[u][q]) && ok;
+#pragma unroll
+    for (int u = 0; u < kLoopAhead; ++u)
+#pragma unroll
+      for (int q = 0; q < Q; q += 2) {
+        const uint4 h = x[u][q], l = x[u][q + 1];
+        const int m = 3 * (q / 2);
+        v[m] = P::add(v[m], make_float2(__uint_as_float(h.x), __uint_as_float(l.x)));
+        v[m + 1] = P::add(v[m + 1], make_float2(__uint_as_float(h.y), __uint_as_float(l.y)));
+        v[m + 2] = P::add(v[m + 2], make_float2(__uint_as_float(h.z), __uint_as_float(l.z)));
+      }
+  }
+  const float2 a = warpSpreadSum<float, M>(v);
+  __syncthreads();  // (warp 0 has read the records of its CTA)
+  if (k < N && g == 0) wrec[wid * N + k] = a;
+  ok = __syncthreads_and(ok) != 0;
+  if (wid == 0) {
+    const float2 b = warpRecords<float, N, M>(wrec, W);
+    mine = __shfl_sync(0xffffffffu, P::value(b), lane < N ? lane * G : 0);
+  }
+  return ok;
+}
+// The result of a sum: three values and flag bits beside the tag.  CTA 0 (the
+// values in lanes 0 .. 2 of warp 0) writes the copies, the others poll theirs.
+__device__ __forceinline__ void resultPut(uint4* out, unsigned tag, float v, unsigned flags) {
+  const int lane = threadIdx.x & 31;
+  const unsigned x = __float_as_uint(__shfl_sync(0xffffffffu, v, 0));
+  const unsigned y = __float_as_uint(__shfl_sync(0xffffffffu, v, 1));
+  const unsigned z = __float_as_uint(__shfl_sync(0xffffffffu, v, 2));
+  stPacket(out + kLoopLine * lane, x, y, z, tag << 8 | flags);
+}
+
+template <bool MORE, bool WIDE>
+__global__ void __launch_bounds__(kLoopThreads, 4)
+kPartLoop(MeshView mv, Controls c, PartView pv, PartPtrs<float> pt, LoopPtrs lp, PcgPtrs<float> p,
+          DevState* st) {
+  using T = float;
+  using E = PartEnt;
+  using P = Part<T>;
+  constexpr int NT = kLoopThreads, KR = kLoopRows, KH = 4;
+  constexpr unsigned kU = URow<T>::kBytes;
+  if (!st->pcgContinue) return;  // the same in every CTA: CTA 0 writes the state at its end
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ float2 wrec[6 * (NT / 32)];
+  __shared__ T sVal[3];
+  __shared__ unsigned sFlags;
+  __shared__ DevState sst;  // CTA 0: the state while the loop runs
+  const int t = (int)threadIdx.x, cap = pv.capRows, part = (int)blockIdx.x, nP = (int)gridDim.x;
+  const int pLo = mv.partStart[part], nR = mv.partStart[part + 1] - pLo, nH = pv.haloCnt[part];
+  const int l0 = mv.lvlOff[part], nL = mv.lvlOff[part + 1] - l0;
+  const bool lead = part == 0;
+  // (a shorter limit is for the waits between parts of the exact DIC's sweeps)
+  const int limit = mv.spinLimit > kSpinLimit ? mv.spinLimit : kSpinLimit;
+  uint4* const rec2 = lp.rec + 4 * (size_t)nP;
+  uint4* const out = rec2 + 2 * (size_t)nP;
+  unsigned* const count = reinterpret_cast<unsigned*>(out + kLoopLine * kLoopCopies);
+  unsigned tag = ldRelaxed(count);  // of the last sum; CTA 0 writes it at its end
+  const uint4* const mine = out + kLoopLine * (part % kLoopCopies);
+  // ---- shared memory: w or p of the rows, the zero row, p of the halo | sweep
+  //      tables | level bounds | product coefficients | product columns
+  const unsigned uBase = (unsigned)__cvta_generic_to_shared(smraw);
+  const int halo0 = cap + 4;
+  ResAddr ad[2];
+  unsigned at = uBase + kU * (unsigned)(halo0 + pv.haloCap);
+#pragma unroll
+  for (int d = 0; d < 2; ++d) {
+    ad[d].q = at; at += 16u * cap;
+    ad[d].r = at;
+    if (MORE) { ad[d].mq = at; at += 16u * cap; ad[d].mr = at; }
+  }
+  const unsigned lva = at + 16;
+  T* const sval = (T*)(smraw + (at - uBase) + 8 * (mv.maxLevels + 5));
+  unsigned short* const sslot = (unsigned short*)(sval + kResW * cap);
+  for (int i = t; i < nR; i += NT) {
+#pragma unroll
+    for (int d = 0; d < 2; ++d) {
+      E::fetch(ad[d].q + 16u * i, 0u, pt.sweep[d], pLo + i);
+      if (MORE) E::fetch(ad[d].mq + 16u * i, 0u, pt.more[d], pLo + i);
+    }
+#pragma unroll
+    for (int e = 0; e < kResW; ++e) {
+      sval[e * cap + i] = pt.val[(size_t)e * mv.nC + pLo + i];
+      const int w = pv.slot[(size_t)e * mv.nC + pLo + i];
+      sslot[e * cap + i] = (unsigned short)(w < nR ? w : w - nR + halo0);
+    }
+  }
+  for (int l = t; l < nL + 4; l += NT) {
+    int2 b = make_int2(0, 0);
+    if (l >= 2 && l < nL + 2)
+      b = make_int2(mv.lvlStart[l0 + l - 2] - pLo, mv.lvlStart[l0 + l - 1] - pLo);
+    asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(lva - 16 + 8u * l), "r"(b.x), "r"(b.y) : "memory");
+  }
+  if (t == 0) {
+    const T z[3] = {0, 0, 0};
+    URow<T>::store(uBase + kU * (unsigned)pv.zeroRow, z);
+    if (lead) sst = *st;
+  }
+  int hx[KH];
+  const int* __restrict__ hi = pv.halo + (size_t)part * pv.haloCap;
+#pragma unroll
+  for (int j = 0; j < KH; ++j) hx[j] = t + j * NT < nH ? hi[t + j * NT] : -1;
+  T r[KR][3], x[KR][3], pp[KR][3], q[KR][3], rd[KR], dg[KR];
+#pragma unroll
+  for (int j = 0; j < KR; ++j) {
+    const int i = t + j * NT;
+    rd[j] = i < nR ? p.rD[pLo + i] : T(0);
+    dg[j] = i < nR ? p.diag[pLo + i] : T(0);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      r[j][k] = i < nR ? p.r[3 * (size_t)(pLo + i) + k] : T(0);
+      x[j][k] = 0; pp[j][k] = 0; q[j][k] = 0;
+    }
+  }
+  cpAsyncWaitAll();
+  __syncthreads();
+  bool ok = true;
+  unsigned pend = 0;  // components with a pending update (bits)
+  T al[3] = {0, 0, 0};
+  // result of a sum: in sVal and sFlags after the next barrier
+  auto result = [&]() {
+    if (t == 0 && !lead) {
+      uint4 v;
+      ok = waitPacket(mine, tag << 8, 8, limit, v) && ok;
+      sVal[0] = __uint_as_float(v.x); sVal[1] = __uint_as_float(v.y); sVal[2] = __uint_as_float(v.z);
+      sFlags = v.w & 0xffu;
+    }
+    ok = __syncthreads_and(ok) != 0;
+  };
+  for (;;) {
+    ++tag;
+    // pending r -= alpha q, sum|r|, w = rD r
+    Acc<T> ar[3], wr[3];
+#pragma unroll
+    for (int j = 0; j < KR; ++j) {
+      const int i = t + j * NT;
+      if (i < nR) {
+        T w[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          if (pend >> k & 1) r[j][k] = fmaT(-al[k], q[j][k], r[j][k]);
+          ar[k].add(fabs(r[j][k]));
+          w[k] = mulT(rd[j], r[j][k]);
+        }
+        URow<T>::store(uBase + kU * (unsigned)i, w);
+      }
+    }
+    __syncthreads();
+    if (nL > 1 && t < kLoopWalk) {
+      resSweepBody<0, false, false, false, MORE, WIDE, E>(pt.sweep[0], pt.more[0], ad[0], uBase, 0u, lva,
+                                                          nL, kLoopWalk, 0);
+      resSweepBody<1, false, false, false, MORE, WIDE, E>(pt.sweep[1], pt.more[1], ad[1], uBase, 0u, lva,
+                                                          nL, kLoopWalk, 0);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < KR; ++j) {
+      const int i = t + j * NT;
+      if (i < nR) {
+        T w[3];
+        URow<T>::load(uBase + kU * (unsigned)i, w);
+        stPacket(lp.w + pLo + i, __float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2]), tag);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) wr[k].add(mulT(w[k], r[j][k]));
+      }
+    }
+    {
+      float2 v[8] = {P::of(wr[0]), P::of(wr[1]), P::of(wr[2]), P::of(ar[0]),
+                     P::of(ar[1]), P::of(ar[2]), P::zero(), P::zero()};
+      double sum = 0;
+      ok = gridPut<6>(v, lp.rec, wrec, tag, limit, sum) && ok;
+      if (lead && t < 32) {
+        pcgDecideBeta(c, &sst, sum, pend != 0);
+        __syncwarp();
+        const bool act = t < 3 && sst.active[t < 3 ? t : 0], first = t < 3 && sst.nIter[t < 3 ? t : 0] == 0;
+        const unsigned f = __ballot_sync(0xffffffffu, act) | __ballot_sync(0xffffffffu, first) << 3 |
+                           (sst.pcgContinue ? 64u : 0u);
+        const T b = t < 3 ? (T)sst.beta[t] : T(0);
+        resultPut(out, tag, b, f);
+        if (t < 3) sVal[t] = b;
+        if (t == 0) sFlags = f;
+      }
+    }
+    // (the halo's w while CTA 0 decides)
+    uint4 wh[KH];
+#pragma unroll
+    for (int j = 0; j < KH; ++j)
+      if (hx[j] >= 0) wh[j] = ldPacket(lp.w + hx[j]);
+#pragma unroll
+    for (int j = 0; j < KH; ++j)
+      if (hx[j] >= 0 && wh[j].w != tag) ok = waitPacket(lp.w + hx[j], tag, 0, limit, wh[j]) && ok;
+    result();
+    if (!ok) break;
+    const unsigned fl = sFlags;
+    const bool go = (fl & 64u) != 0;
+    // pending x += alpha p_old; p = w + beta p_old
+    T b[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) b[k] = sVal[k];
+#pragma unroll
+    for (int j = 0; j < KR; ++j) {
+      const int i = t + j * NT;
+      if (i < nR) {
+        T u[3];
+        URow<T>::load(uBase + kU * (unsigned)i, u);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          if (pend >> k & 1) x[j][k] = fmaT(al[k], pp[j][k], x[j][k]);
+          if (!(fl >> (3 + k) & 1)) u[k] = fmaT(b[k], pp[j][k], u[k]);
+          if (fl >> k & 1) pp[j][k] = u[k];
+        }
+        URow<T>::store(uBase + kU * (unsigned)i, u);
+      }
+    }
+    if (!go) break;
+#pragma unroll
+    for (int j = 0; j < KH; ++j)
+      if (hx[j] >= 0) {
+        const unsigned a = uBase + kU * (unsigned)(halo0 + t + j * NT);
+        T o[3], w[3] = {__uint_as_float(wh[j].x), __uint_as_float(wh[j].y), __uint_as_float(wh[j].z)};
+        URow<T>::load(a, o);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          if (!(fl >> (3 + k) & 1)) w[k] = fmaT(b[k], o[k], w[k]);
+        URow<T>::store(a, w);
+      }
+    __syncthreads();
+    ++tag;
+    // q = A p, p.q
+    Acc<T> pq[3];
+#pragma unroll
+    for (int j = 0; j < KR; ++j) {
+      const int i = t + j * NT;
+      if (i < nR) {
+        T v[3], y[3], xv[kResW][3];
+        URow<T>::load(uBase + kU * (unsigned)i, v);
+#pragma unroll
+        for (int e = 0; e < kResW; ++e) URow<T>::load(uBase + kU * (unsigned)sslot[e * cap + i], xv[e]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) y[k] = mulT(dg[j], v[k]);
+#pragma unroll
+        for (int e = 0; e < kResW; ++e) {
+          const T a = sval[e * cap + i];
+#pragma unroll
+          for (int k = 0; k < 3; ++k) y[k] = fmaT(a, xv[e][k], y[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          if (fl >> k & 1) q[j][k] = y[k];
+          pq[k].add(mulT(y[k], v[k]));
+        }
+      }
+    }
+    {
+      float2 v[4] = {P::of(pq[0]), P::of(pq[1]), P::of(pq[2]), P::zero()};
+      double sum = 0;
+      ok = gridPut<3>(v, rec2, wrec, tag, limit, sum) && ok;
+      if (lead && t < 32) {
+        pcgDecideAlpha(&sst, sum, 0);
+        __syncwarp();
+        const bool on = t < 3 && sst.pending[t < 3 ? t : 0];
+        const unsigned f = __ballot_sync(0xffffffffu, on) | (sst.pcgContinue ? 64u : 0u);
+        const T b = t < 3 ? (T)sst.alpha[t] : T(0);
+        resultPut(out, tag, b, f);
+        if (t < 3) sVal[t] = b;
+        if (t == 0) sFlags = f;
+      }
+    }
+    result();
+    if (!ok) break;
+    pend = sFlags & 7u;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) al[k] = sVal[k];
+    if (!(sFlags & 64u)) break;
+  }
+#pragma unroll
+  for (int j = 0; j < KR; ++j) {
+    const int i = t + j * NT;
+    if (i < nR) stRow(p.x, (size_t)(pLo + i), x[j]);
+  }
+  if (t == 0 && !ok) atomicOr(&st->status, kErrTimeout);
+  if (lead) {
+    // the state back; x is complete.  (No tag of a wait that gave up comes again.)
+    __syncthreads();
+    if (t < 3) {
+      st->active[t] = sst.active[t]; st->nIter[t] = sst.nIter[t]; st->finalRes[t] = sst.finalRes[t];
+      st->wArA[t] = sst.wArA[t]; st->wApA[t] = sst.wApA[t];
+      st->alpha[t] = sst.alpha[t]; st->beta[t] = sst.beta[t];
+      st->pending[t] = sst.pending[t];
+      st->xPend[t] = 0;
+    }
+    if (t == 0) {
+      st->pcgIter = sst.pcgIter;
+      st->pcgContinue = sst.pcgContinue;
+      if (sst.status) atomicOr(&st->status, sst.status);
+      *count = tag + 4;
+    }
+  }
+}
+
 // ---- tables --------------------------------------------------------------------
 // Entries of a part's rows that lead out of it (the largest count in *most).
 __global__ void kPartCount(MeshView mv, int* cnt, int* most) {
@@ -593,6 +973,45 @@ cudaError_t partPrepare(const MeshView& mv, const PartView& pv, int* blocks) {
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+
+namespace {
+const void* loopKernel(const PartView& pv) {
+  if (pv.wide) return (const void*)kPartLoop<true, true>;
+  return pv.more ? (const void*)kPartLoop<true, false> : (const void*)kPartLoop<false, false>;
+}
+size_t loopSmem(const MeshView& mv, const PartView& pv) {
+  const size_t cap = pv.capRows;
+  return URow<float>::kBytes * (cap + 4 + pv.haloCap) + 16 * (pv.more ? 4 : 2) * cap +
+         8 * (size_t)(mv.maxLevels + 5) + kResW * 6 * cap;
+}
+}  // namespace
+
+size_t partLoopPackets(int nParts) { return 6 * (size_t)nParts + kLoopLine * kLoopCopies + 1; }
+
+cudaError_t partLoopPrepare(const MeshView& mv, const PartView& pv, int* blocks) {
+  *blocks = 0;
+  if (pv.capRows > kLoopMaxRows || pv.haloCap > 4 * kLoopThreads) return cudaSuccess;
+  const void* k = loopKernel(pv);
+  const cudaError_t e = setMaxDynamicSmem(k);
+  if (e != cudaSuccess) return e;
+  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, k, kLoopThreads, loopSmem(mv, pv));
+}
+cudaError_t launchPartLoop(const MeshView& mv, const Controls& c, const PartView& pv,
+                           const PartPtrs<float>& pt, const LoopPtrs& lp, const PcgPtrs<float>& p,
+                           DevState* st, cudaStream_t s) {
+  cudaLaunchConfig_t cf{};
+  cf.gridDim = dim3(mv.nParts);
+  cf.blockDim = dim3(kLoopThreads);
+  cf.dynamicSmemBytes = loopSmem(mv, pv);
+  cf.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeCooperative;
+  at[0].val.cooperative = 1;
+  cf.attrs = at;
+  cf.numAttrs = 1;
+  void* args[] = {(void*)&mv, (void*)&c, (void*)&pv, (void*)&pt, (void*)&lp, (void*)&p, (void*)&st};
+  return cudaLaunchKernelExC(&cf, loopKernel(pv), args);
 }
 
 cudaError_t launchPartCount(const MeshView& mv, int* cnt, int* most, cudaStream_t s) {
