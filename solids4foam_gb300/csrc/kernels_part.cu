@@ -45,7 +45,7 @@ template <> struct PartCfg<float> {
 };
 template <> struct PartCfg<double> {
   using Ent = ResEnt<double>;
-  static constexpr int kNT = 192, kKeep = 3, kOcc = 3;
+  static constexpr int kNT = 192, kKeep = 3, kOcc = 4;
   static constexpr bool kSplit = true, kOrdered = true;
 };
 constexpr int kPartSpmvThreads = 128;
@@ -140,8 +140,8 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
     }
   }
   const unsigned lva = at + 16;  // two empty levels before the first
-  // (ordered sums) the part's residual
-  T* const sr = (T*)(smraw + (at - uBase) + 8 * (mv.maxLevels + 5));
+  // (ordered sums) the part's residual, in the tables' place after the sweeps
+  T* const sr = (T*)(smraw + (ad[0].q - uBase));
   double* grec = partials + mv.locGrpOff;
   unsigned* gcnt = reinterpret_cast<unsigned*>(grec + 8 * (size_t)mv.locGroups);
   int prev = -1;
@@ -221,7 +221,6 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
               rg[g + k] = rK[j][k];
             }
             w[k] = mulT(rd[j], rK[j][k]);
-            if (C::kOrdered) sr[3 * i + k] = rK[j][k];
           }
           URow<T>::store(uBase + kU * (unsigned)i, w);
         }
@@ -239,7 +238,6 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
           rg[g + k] = rv;
         }
         w[k] = mulT(rd, rv);
-        if (C::kOrdered) sr[3 * i + k] = rv;
       }
       URow<T>::store(uBase + kU * (unsigned)i, w);
     }
@@ -260,7 +258,11 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
         URow<T>::load(uBase + kU * (unsigned)i, w);
         stRow(p.w, (size_t)(pLo + i), w);
 #pragma unroll
-        for (int k = 0; k < 3 && !C::kOrdered; ++k) {
+        for (int k = 0; k < 3; ++k) {
+          if (C::kOrdered) {
+            sr[3 * i + k] = rK[j][k];
+            continue;
+          }
           wr[k].add(mulT(w[k], rK[j][k]));
           ar[k].add(fabs(rK[j][k]));
         }
@@ -271,33 +273,40 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
       URow<T>::load(uBase + kU * (unsigned)i, w);
       stRow(p.w, (size_t)(pLo + i), w);
 #pragma unroll
-      for (int k = 0; k < 3 && !C::kOrdered; ++k) {
+      for (int k = 0; k < 3; ++k) {
         const T r = rg[3 * (size_t)(pLo + i) + k];  // written by this thread
+        if (C::kOrdered) {
+          sr[3 * i + k] = r;
+          continue;
+        }
         wr[k].add(mulT(w[k], r));
         ar[k].add(fabs(r));
       }
     }
     if (C::kOrdered) {
-      // lane l of 64 sums rows l, l + 64, ..., then a fixed tree
-      double d6[6] = {0, 0, 0, 0, 0, 0};
-      if (t < 64)
+      // lane l of 64 sums rows l, l + 64, ..., then a fixed tree: sum64's, by the
+      // spread sum (9 additions a warp for 30)
+      __syncthreads();
+      const int k = (t & 31) / 4;
+      double s6 = 0;
+      if (t < 64) {
+        double d[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         for (int i = t; i < nR; i += 64) {
           T w[3];
           URow<T>::load(uBase + kU * (unsigned)i, w);
 #pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            const T r = sr[3 * i + k];
-            d6[k] = fma((double)w[k], (double)r, d6[k]);
-            d6[3 + k] += fabs((double)r);
+          for (int m = 0; m < 3; ++m) {
+            const T r = sr[3 * i + m];
+            d[m] = fma((double)w[m], (double)r, d[m]);
+            d[3 + m] += fabs((double)r);
           }
         }
-      if (t == 0) sGroup = done ? prev / kLocGroup : -1;
-      sum64<6>(d6, sum);
-      if (t == 0) {
-        double* q = partials + 8 * (size_t)part;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) q[k] = d6[k];
+        s6 = warpSpreadSum<double, 8>(d);
+        if (t >= 32 && t % 4 == 0 && k < 6) sum[k] = s6;
       }
+      if (t == 0) sGroup = done ? prev / kLocGroup : -1;
+      __syncthreads();
+      if (t < 32 && t % 4 == 0 && k < 6) partials[8 * (size_t)part + k] = s6 + sum[k];
       if (sGroup >= 0 && t < 32) locGroupSum(partials, grec, gcnt, sGroup, nParts);
       prev = part;
     }
@@ -945,7 +954,7 @@ template <typename T>
 size_t precondSmem(const MeshView& mv, const PartView& pv) {
   const size_t ent = 16 + PartCfg<T>::Ent::kB;
   return URow<T>::kBytes * (size_t)(pv.capRows + 4) + 2 * (pv.more ? 2 : 1) * ent * pv.capRows +
-         8 * (size_t)(mv.maxLevels + 5) + (PartCfg<T>::kOrdered ? 3 * sizeof(T) * pv.capRows : 0);
+         8 * (size_t)(mv.maxLevels + 5);
 }
 size_t spmvSmem(const PartView& pv) {
   return URow<float>::kBytes * (size_t)(pv.capRows + pv.haloCap);
