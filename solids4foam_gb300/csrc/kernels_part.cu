@@ -375,6 +375,20 @@ kPartSpmv(MeshView mv, PartView pv, PartPtrs<float> pt, PcgPtrs<float> p, DevSta
     int hx[KH];  // the rows of the thread's first halo places
 #pragma unroll
     for (int j = 0; j < KH; ++j) hx[j] = t + j * NT < nH ? hi[t + j * NT] : -1;
+    // a row's coefficients are read a row ahead, the first one's while p_new is
+    // formed
+    T aN[kResW], dgN = T(0);
+    unsigned short clN[kResW];
+    auto coefs = [&](int i) {
+      if (i >= nR) return;
+      dgN = p.diag[pLo + i];
+#pragma unroll
+      for (int e = 0; e < kResW; ++e) {
+        clN[e] = pv.slot[(size_t)e * mv.nC + pLo + i];
+        aN[e] = pt.val[(size_t)e * mv.nC + pLo + i];
+      }
+    };
+    coefs(t);
     // p_new of the part's rows and of the rows around it
     for (int i0 = t; i0 < nR; i0 += RP * NT) {
       T w[RP][3], o[RP][3], x[RP][3];
@@ -435,42 +449,27 @@ kPartSpmv(MeshView mv, PartView pv, PartPtrs<float> pt, PcgPtrs<float> p, DevSta
       URow<T>::store(uBase + kU * (unsigned)(nR + h), v);
     }
     __syncthreads();
-    for (int i0 = t; i0 < nR; i0 += RP * NT) {
-      T a[RP][kResW], dg[RP];
-      unsigned short cl[RP][kResW];
+    for (int i = t; i < nR; i += NT) {
+      T a[kResW], v[3], y[3], x[kResW][3];
+      const T dg = dgN;
+      unsigned short cl[kResW];
 #pragma unroll
-      for (int h = 0; h < RP; ++h) {
-        const int i = i0 + h * NT;
-        if (i < nR) {
-          dg[h] = p.diag[pLo + i];
+      for (int e = 0; e < kResW; ++e) { a[e] = aN[e]; cl[e] = clN[e]; }
+      coefs(i + NT);
+      URow<T>::load(uBase + kU * (unsigned)i, v);
 #pragma unroll
-          for (int e = 0; e < kResW; ++e) {
-            cl[h][e] = pv.slot[(size_t)e * mv.nC + pLo + i];
-            a[h][e] = pt.val[(size_t)e * mv.nC + pLo + i];
-          }
-        }
-      }
+      for (int e = 0; e < kResW; ++e) URow<T>::load(uBase + kU * (unsigned)cl[e], x[e]);
 #pragma unroll
-      for (int h = 0; h < RP; ++h) {
-        const int i = i0 + h * NT;
-        if (i < nR) {
-          T v[3], y[3], x[kResW][3];
-          URow<T>::load(uBase + kU * (unsigned)i, v);
+      for (int k = 0; k < 3; ++k) y[k] = mulT(dg, v[k]);
 #pragma unroll
-          for (int e = 0; e < kResW; ++e) URow<T>::load(uBase + kU * (unsigned)cl[h][e], x[e]);
+      for (int e = 0; e < kResW; ++e)  // (padded: the row itself times zero)
 #pragma unroll
-          for (int k = 0; k < 3; ++k) y[k] = mulT(dg[h], v[k]);
+        for (int k = 0; k < 3; ++k) y[k] = fmaT(a[e], x[e][k], y[k]);
+      const size_t g = 3 * (size_t)(pLo + i);
 #pragma unroll
-          for (int e = 0; e < kResW; ++e)  // (padded: the row itself times zero)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) y[k] = fmaT(a[h][e], x[e][k], y[k]);
-          const size_t g = 3 * (size_t)(pLo + i);
-#pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            if (act[k]) qo[g + k] = y[k];
-            pq[k].add(mulT(y[k], v[k]));
-          }
-        }
+      for (int k = 0; k < 3; ++k) {
+        if (act[k]) qo[g + k] = y[k];
+        pq[k].add(mulT(y[k], v[k]));
       }
     }
     __syncthreads();
