@@ -1006,10 +1006,11 @@ struct Engine {
     return sizeof(T) == 4 && mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC && nRun == 1 &&
            !batched && hp.nC > kLoopMinRows;
   }
-  // The forms it has.  In FP64 the exact DIC only: the corrector loop of the
-  // processor-local DIC (and, less, of the diagonal preconditioner) amplifies a
-  // last bit of a sum over many correctors, and the separate kernels' sums are
-  // the ones results are compared with.
+  // The forms it has.  In FP64 the exact DIC only, whose sums it adds in the
+  // separate kernels' order: the corrector loop can amplify a last bit of a sum
+  // over many correctors.  (FP64 processor-local and diagonal runs of small meshes
+  // keep the separate kernels: their ordered sums in the cluster would take most
+  // of what its one launch saves.)
   template <typename T>
   bool residentForm() const {
     const bool dic = lin.preconditioner == S4G_PRECOND_DIC;
