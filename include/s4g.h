@@ -138,7 +138,10 @@ typedef struct s4g_mesh_opts {
                              part (processor-local DIC of a decomposed run) */
   int no_autotune;        /* 1: skip the kernel-variant autotuner of the
                              processor-local PCG (results are identical
-                             either way; only the speed differs) */
+                             either way; only the speed differs).  2: as 1,
+                             and the PCG runs its general kernels, one
+                             launch per step, on any mesh (the same results;
+                             the form the others are tested against) */
   int empty_direction;    /* 2-D cases: 1, 2 or 3 for an x, y or z empty
                              direction, whose empty patches' faces the caller
                              leaves out of the mesh description (they have no
@@ -409,6 +412,11 @@ s4g_status s4g_get_pointD(s4g_mesh* mesh, double* pointD_out);
 /* Cell gradient of D from the last solve, [n_cells][9] row-major,
  * grad(D)_ij = dD_j/dx_i (the reference's gradD field). */
 s4g_status s4g_get_gradD(s4g_mesh* mesh, double* gradD_out);
+
+/* Scalars of the PCG in the last solve's last corrector (its first load case),
+ * per component: out [4][3] = w.r, p.Ap, alpha, beta.  For diagnosis and tests:
+ * every form of the PCG that a mesh may run gives the same bits. */
+s4g_status s4g_get_pcg_scalars(s4g_mesh* mesh, double* out);
 
 /* -------------------------------------------- operator-level entry points
  * For kernel-by-kernel parity checks.  Vectors are in the caller's cell

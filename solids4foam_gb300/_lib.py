@@ -146,6 +146,7 @@ _SIGS = {
                                   ct.POINTER(Perf)]),
     "s4g_state_reset": (ct.c_int, [ct.c_void_p]),
     "s4g_get_gradD": (ct.c_int, [ct.c_void_p, ct.c_void_p]),
+    "s4g_get_pcg_scalars": (ct.c_int, [ct.c_void_p, ct.c_void_p]),
     "s4g_solve_batch": (ct.c_int, [ct.c_void_p, ct.c_int, ct.c_void_p, ct.c_void_p, ct.c_void_p]),
     "s4g_mesh_set_points": (ct.c_int, [ct.c_void_p, ct.c_int, ct.c_void_p, ct.c_void_p,
                                        ct.c_void_p]),

@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <chrono>
 #include <cmath>
 #include <cstdio>
@@ -110,8 +111,13 @@ struct EventTimer : LaunchTimer {
 // by where the separate kernels are as fast.  Exact DIC: as many as the row
 // vector's memory holds.
 constexpr int kResMaxRows(bool local) { return !local ? 16000 : 2048; }
+// Rows beyond which the part loop, and for several load cases or meshes at once the part
+// kernels, take over from it (processor-local DIC, FP32; 30 correctors of n^3 cells in
+// blocks of 8, resident and other; one solve: n = 24 17.4 and 19.2 ms, 26 28.1 and 22.0;
+// eight load cases: 24 25.7 and 31.8, 26 42.1 and 41.1, 28 52.5 and 44.5; a batch of
+// eight meshes: 24 23.4 and 22.4, 26 40.2 and 27.8).
+constexpr int kResAheadRows = 16384;
 constexpr int kResMaxDiagRows = 16384;
-constexpr int kLoopMinRows = 16384;  // (loopMesh)
 constexpr int kPcgUnroll = 8;  // PCG iterations of a pass of the device loop
 
 struct Engine {
@@ -151,6 +157,7 @@ struct Engine {
   LocalTuning tune64, tune32;   // fused-iteration variants (FP64 / FP32 inner solve)
   bool tuned64 = false, tuned32 = false;
   bool autotune = true;
+  bool generalPcg = false;  // the separate kernels on any mesh
   double tuneUs[2][kLocNumNT + kLocNumU] = {};  // last timings (us), for perf
   // cluster-resident PCG (kernels_resident.cu), per value type: the plan, made
   // at the first solve of that type, and its tables
@@ -170,12 +177,14 @@ struct Engine {
   struct Parts {
     bool tried = false, ok = false, valid = false;
     bool loop = false;  // all parts resident at once: the loop in one launch
+    int loopMost = 0;   // the CTAs of such a launch that the device holds
     PartView pv{};
     PartPtrs<T> pt{};
   };
   Parts<double> parts64;
   Parts<float> parts32;
   LoopPtrs lp;
+  size_t lpCount = 0;  // packets of lp
   int *dHaloCnt = nullptr, *dHalo = nullptr, haloCap = 0;
   unsigned short* dSlot = nullptr;
   template <typename T>
@@ -328,6 +337,7 @@ struct Engine {
     mv.nC = nC; mv.nI = nI; mv.nB = nB; mv.nParts = hp.nParts;
     mv.subdomains = (o && o->dic_subdomains) ? 1 : 0;
     mv.emptyDir = o ? o->empty_direction : 0;
+    generalPcg = o && o->no_autotune == 2;
     mv.rowGrid = std::max(1, std::min((nC + kRowBlock - 1) / kRowBlock,
                                       ctx->numSMs * kRowBlocksPerSM));
     // 64-thread blocks until they fill the SMs four times over (measured on a
@@ -415,7 +425,7 @@ struct Engine {
     mv.locGroups = (hp.nParts + 31) / 32;
     mv.locGrpOff = (long)std::max(8 * rowBlocks, 8 * (size_t)hp.nParts);
     mv.ordOff = (mv.locGrpOff + 8 * (long)mv.locGroups + (mv.locGroups + 1) / 2 + 7) / 8 * 8;
-    mv.caseRec = mv.ordOff + (mv.subdomains ? 0 : (long)ordRecords(hp.nParts, nC));
+    mv.caseRec = mv.ordOff + ((long)ordRecords(hp.nParts, nC) + 7) / 8 * 8;
     S4G_TRY(alloc(&dPartials, (size_t)mv.caseRec));
     S4G_CUDA(cudaMemsetAsync(dPartials, 0, sizeof(double) * (size_t)mv.caseRec, s));
     S4G_TRY(alloc(&dOut, 9 * (size_t)nC));
@@ -671,7 +681,7 @@ struct Engine {
   template <typename T>
   s4g_status ensureResident() {
     Resident<T>& q = resident<T>();
-    if (ctx->profile || !residentForm<T>()) return S4G_OK;
+    if (ctx->profile || generalPcg || !residentForm<T>()) return S4G_OK;
     cudaStream_t s = ctx->stream;
     if (!q.tried) {
       q.tried = true;
@@ -704,9 +714,10 @@ struct Engine {
     rv.ring = kResThreads;
     // Exact DIC: the substitutions inside one CTA where all rows fit its memory
     // (a level costs the CTA's barrier, not the cluster's).  Rows per CTA: a
-    // level's cost hardly depends on them, the other phases' time does.
+    // level's cost hardly depends on them, the other phases' time does, the sums'
+    // above all (13 x 11 x 10 cells in blocks of 8: 91 ms with 1024 rows, 82 with 256).
     rv.single = !rv.local && resSmemBytes<T>(rv, 0) <= limit;
-    const int rows = rv.local ? 1024 : 256;
+    const int rows = 256;
     rv.C = std::max(1, std::min({kResMaxCtas, (nC + rows - 1) / rows,
                                  rv.local ? hp.nParts : kResMaxCtas}));
     if (nC > kResMaxCtas * kResMaxRows(rv.local)) return S4G_OK;
@@ -714,9 +725,9 @@ struct Engine {
     if (sizeof(T) == 8 && (long)nC > (long)mv.rowGrid * kRowBlock) return S4G_OK;
     // rows by CTA and level
     std::vector<int> chunk(rv.C + 1, 0), lvl, pos(nC);
+    std::vector<int> first(rv.C + 1, hp.nParts);  // (local) first part of each CTA
     if (rv.local) {
       rv.nLev = hp.maxLocalLevels;
-      std::vector<int> first(rv.C + 1, hp.nParts);  // first part of each CTA
       first[0] = 0;
       for (int c = 1, p = 0; c < rv.C; ++c) {
         // the part boundary nearest an even share, one part at least each
@@ -834,12 +845,13 @@ struct Engine {
       cudaGetLastError();
       return S4G_OK;
     }
-    int *dChunk, *dLvl;
+    int *dChunk, *dLvl, *dFirst;
     uint32_t *col, *cnt;
     T *val, *dg, *rd;
     const size_t nE = (size_t)kResW * nC;
     S4G_TRY(upload(&dChunk, chunk));
     S4G_TRY(upload(&dLvl, lvl));
+    S4G_TRY(upload(&dFirst, first));
     S4G_TRY(upload(&q.pos, pos));
     S4G_TRY(alloc(&col, nE)); S4G_TRY(alloc(&cnt, (size_t)nC)); S4G_TRY(alloc(&val, nE));
     S4G_TRY(alloc(&dg, (size_t)nC)); S4G_TRY(alloc(&rd, (size_t)nC));
@@ -853,7 +865,8 @@ struct Engine {
     }
     S4G_CUDA(cudaStreamSynchronize(ctx->stream));  // the host arrays end here
     rv.pos = q.pos;
-    if (sizeof(T) == 8) {
+    rv.part0 = dFirst;
+    if (!rv.local) {
       // kSweepSm's thread t sums rows t, t + kOrdLanes, ... of each level, last
       // level first
       std::vector<int> step{0}, row;
@@ -879,12 +892,16 @@ struct Engine {
   template <typename T>
   s4g_status ensureParts() {
     Parts<T>& q = parts<T>();
-    if (!mv.subdomains || lin.preconditioner != S4G_PRECOND_DIC || (runsResident<T>() && !loopMesh<T>()))
+    if (generalPcg || !mv.subdomains || lin.preconditioner != S4G_PRECOND_DIC ||
+        (runsResident<T>() && hp.nC <= kResAheadRows))
       return S4G_OK;
     if (!q.tried) {
       q.tried = true;
       S4G_TRY(planParts<T>(q));
     }
+    // packets of a launch whose waits gave up may carry the tags of the next one
+    if (q.loop && (hState->status & kErrTimeout))
+      S4G_CUDA(cudaMemsetAsync(lp.w, 0, sizeof(uint4) * lpCount, ctx->stream));
     if (!q.ok || q.valid) return S4G_OK;
     S4G_CUDA(launchPartTables<T>(mv, q.pv, dVal, dRDa, q.pt, ctx->stream));
     launches++;
@@ -938,14 +955,19 @@ struct Engine {
     }
     if constexpr (sizeof(T) == 4) {
       int per = 0;
-      if (partLoopPrepare(mv, pv, &per) == cudaSuccess) q.loop = hp.nParts <= per * ctx->numSMs;
-      else cudaGetLastError();
+      if (partLoopPrepare(mv, pv, &per) != cudaSuccess) {
+        cudaGetLastError();
+        per = 0;
+      }
+      q.loopMost = per * ctx->numSMs;
+      q.loop = hp.nParts <= q.loopMost;
     }
     if (q.loop && !lp.w) {
-      const size_t n = (size_t)nC + partLoopPackets(hp.nParts);
-      S4G_TRY(alloc(&lp.w, n));
-      S4G_CUDA(cudaMemsetAsync(lp.w, 0, sizeof(uint4) * n, s));
-      lp.rec = lp.w + nC;
+      lpCount = 2 * (size_t)nC + partLoopPackets(mv);
+      S4G_TRY(alloc(&lp.w, lpCount));
+      S4G_CUDA(cudaMemsetAsync(lp.w, 0, sizeof(uint4) * lpCount, s));
+      lp.t = lp.w + nC;
+      lp.rec = lp.t + nC;
     }
     if (sizeof(T) == 4) {
       T* val;
@@ -972,10 +994,20 @@ struct Engine {
     return mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC && !runsResident<T>() && parts<T>().ok;
   }
 
-  // ... and their loop as one launch: a single case on the device alone (several
-  // cases together have more parts than fit at once).
+  // (launches of one of their iterations)
   template <typename T>
-  bool runsPartLoop() { return runsParts<T>() && parts<T>().loop && nRun == 1 && !ctx->profile; }
+  int partLaunches() { return sizeof(T) == 4 || tuning<T>().uIdx == 2 ? 3 : 2; }
+
+  // ... and their loop as one launch: one load case (several together have more parts
+  // than fit at once).  Solves of other contexts may run beside it: a cooperative launch
+  // waits until all of its CTAs find room.  In a batch, whose meshes run side by side,
+  // only where the loops of all its meshes fit at once; else they would run one after
+  // the other (eight meshes of n^3 cells in blocks of 8, 30 correctors, loops and part
+  // kernels: n = 32, 512 parts together, 36.0 and 49.2 ms; 34, 1000 parts, 74.5 and 61.0).
+  template <typename T>
+  bool runsPartLoop() {
+    return runsParts<T>() && parts<T>().loop && nRun == 1 && !ctx->profile && (!batched || batchLoop);
+  }
   template <typename T>
   cudaError_t partLoop(const Controls& c, const PcgPtrs<T>& p) {
     if constexpr (sizeof(T) == 4)
@@ -995,16 +1027,12 @@ struct Engine {
   // rows the whole device's row kernels are faster than one cluster.
   template <typename T>
   bool runsResident() {
-    return !ctx->profile && resident<T>().ok && residentForm<T>() && !(loopMesh<T>() && parts<T>().loop);
+    return !ctx->profile && resident<T>().ok && residentForm<T>() && !overtaken<T>();
   }
-  // Where kPartLoop takes over from the resident PCG: one solve at a time, and
-  // more rows than the cluster's 16 SMs are as fast for (30 correctors of 24^3
-  // cells 12.6 ms resident, 14.9 as a part per CTA; 28^3 18.6 and 16.8; 32^3 21.7
-  // and 18.8).
   template <typename T>
-  bool loopMesh() const {
-    return sizeof(T) == 4 && mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC && nRun == 1 &&
-           !batched && hp.nC > kLoopMinRows;
+  bool overtaken() const {
+    if (sizeof(T) == 8 || !mv.subdomains || lin.preconditioner != S4G_PRECOND_DIC) return false;
+    return hp.nC > kResAheadRows && (nRun > 1 || batched ? parts32.ok : parts32.loop);
   }
   // The forms it has.  In FP64 the exact DIC only, whose sums it adds in the
   // separate kernels' order: the corrector loop can amplify a last bit of a sum
@@ -1025,7 +1053,8 @@ struct Engine {
     if (many) rv.place = q.placeMany;
     return launchResPcg<T>(mv, c, rv, q.rp, p, dState, dPartials, ctx->stream, nRun, many);
   }
-  bool batched = false;  // capturing this mesh's loop into a batch's graph
+  bool batched = false;    // capturing this mesh's loop into a batch's graph
+  bool batchLoop = false;  // (runsPartLoop)
 
   // FP32 copies of the matrix, factor and work vectors (mixed precision).
   s4g_status ensureFp32() {
@@ -1530,7 +1559,7 @@ struct Engine {
         if (runsParts<T>()) {
           launchPartIteration<T>(mv, c, parts<T>().pv, parts<T>().pt, p, dState, dPartials, tuning<T>(),
                                  ctx->stream, tm(), nRun);
-          *count += sizeof(T) == 8 && tuning<T>().uIdx == 2 ? 3 : 2;
+          *count += partLaunches<T>();
         } else if (mv.subdomains && c.precond == 0)
           launchLocalIteration<T>(mv, c, p, dState, dPartials, tuning<T>(), ctx->stream,
                                   count, tm(), nRun);
@@ -1546,8 +1575,9 @@ struct Engine {
         S4G_CUDA(cudaGraphLaunch(exec, ctx->stream));
         long long perBatch = 0;  // count what the batch launches
         const int ut = tuning<T>().uIdx;
-        perBatch = (mv.subdomains && c.precond == 0) ? (long long)chunk * (ut == 2 ? 3 : 2)
-                                                     : (long long)chunk * (c.precond == 0 ? 5 : 4);
+        perBatch = runsParts<T>() ? (long long)chunk * partLaunches<T>()
+                   : (mv.subdomains && c.precond == 0) ? (long long)chunk * (ut == 2 ? 3 : 2)
+                                                       : (long long)chunk * (c.precond == 0 ? 5 : 4);
         launches += perBatch;
       } else {
         launchBatch(chunk, &launches);
@@ -1566,7 +1596,8 @@ struct Engine {
   template <typename T>
   long long pcgLaunches(const Controls& c, bool local, long long it) {
     if (runsResident<T>() || runsPartLoop<T>()) return 0;  // (one per corrector)
-    const int perIt = local ? (tuning<T>().uIdx == 2 ? 3 : 2) : (c.precond == 0 ? 5 : 4);
+    const int perIt = runsParts<T>() ? partLaunches<T>()
+                      : local ? (tuning<T>().uIdx == 2 ? 3 : 2) : (c.precond == 0 ? 5 : 4);
     return it * perIt + (it + kPcgUnroll - 1) / kPcgUnroll;
   }
 
@@ -1789,9 +1820,20 @@ struct Engine {
     S4G_CUDA(cudaGetLastError());
     return S4G_OK;
   }
-  bool batchCapture(cudaGraph_t g) {
+  // The CTAs of this mesh's part loop (0: it runs another form), and how many the device
+  // holds.
+  int batchLoopParts(int* most) {
+    batched = true;
+    const bool loops = precision == S4G_FP32_REFINE && runsParts<float>() && parts32.loop;
+    batched = false;
+    if (!loops) return 0;
+    *most = std::min(*most, parts32.loopMost);
+    return hp.nParts;
+  }
+  bool batchCapture(cudaGraph_t g, bool loops) {
     const Controls c = controls(0);
     batched = true;
+    batchLoop = loops;
     const bool ok = precision == S4G_FP32_REFINE ? buildLoopGraph<float>(g, c, 0, pc32, sweepGrid32)
                                                  : buildLoopGraph<double>(g, c, 0, pc, sweepGrid);
     batched = false;
@@ -1803,9 +1845,11 @@ struct Engine {
     ranOnDevice = true;
     const bool local = mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC;
     const Controls c = controls(0);
+    batched = true;
     launches += 1 + (long long)hState->nCorrDone * 6 +
                 (precision == S4G_FP32_REFINE ? pcgLaunches<float>(c, local, hState->pcgIter)
                                               : pcgLaunches<double>(c, local, hState->pcgIter));
+    batched = false;
     if (Dout) {
       launchGather(hp.nC, 3, dC2s, f.D[hState->dcur], dOut, s);
       S4G_CUDA(cudaMemcpyAsync(Dout, dOut, sizeof(double) * 3 * hp.nC, cudaMemcpyDeviceToHost, s));
@@ -1974,6 +2018,16 @@ struct Engine {
     S4G_CUDA(cudaMemcpyAsync(out, dPointD, sizeof(double) * 3 * (size_t)nPoints,
                              cudaMemcpyDeviceToHost, ctx->stream));
     S4G_CUDA(cudaStreamSynchronize(ctx->stream));
+    return S4G_OK;
+  }
+
+  s4g_status getPcgScalars(double* out) {
+    if (lastModel < 0) return setErr(S4G_BAD_ARG, "no solve has run");
+    if (!out) return setErr(S4G_BAD_ARG, "null output");
+    for (int k = 0; k < 3; ++k) {
+      out[k] = hState->wArA[k]; out[3 + k] = hState->wApA[k];
+      out[6 + k] = hState->alpha[k]; out[9 + k] = hState->beta[k];
+    }
     return S4G_OK;
   }
 
@@ -2233,6 +2287,11 @@ s4g_status s4g_get_gradD(s4g_mesh* mesh, double* gradD_out) {
   return mesh->e.getGradD(gradD_out);
 }
 
+s4g_status s4g_get_pcg_scalars(s4g_mesh* mesh, double* out) {
+  if (!mesh || !out) return setErr(S4G_BAD_ARG, "null argument");
+  return mesh->e.getPcgScalars(out);
+}
+
 s4g_status s4g_mesh_set_points(s4g_mesh* mesh, int n_points, const double* points,
                                const int* point_cell_start, const int* point_cells) {
   if (!mesh) return setErr(S4G_BAD_ARG, "null mesh");
@@ -2294,8 +2353,11 @@ s4g_status s4g_solve_batch(s4g_mesh* const* meshes, int n_meshes, double* const*
   }
   cudaGraph_t g = nullptr;
   if (cudaGraphCreate(&g, 0) != cudaSuccess) return setErr(S4G_CUDA_ERROR, "cudaGraphCreate failed");
+  long loopParts = 0;
+  int loopMost = INT_MAX;
+  for (int i = 0; i < n_meshes; ++i) loopParts += meshes[i]->e.batchLoopParts(&loopMost);
   for (int i = 0; i < n_meshes; ++i)
-    if (!meshes[i]->e.batchCapture(g)) {
+    if (!meshes[i]->e.batchCapture(g, loopParts <= loopMost)) {
       cudaGraphDestroy(g);
       cudaGetLastError();
       return setErr(S4G_CUDA_ERROR, "capturing a mesh's corrector loop into the batch graph failed");

@@ -245,15 +245,15 @@ struct ResView {
   const uint32_t* col;   // [kResW][nC] product columns: CTA << 24 | row in its chunk
   const uint32_t* cnt;   // [nC] entries of the product
   const int* pos;        // [nC] PCG row of each storage row
-  // (FP64) the order of w.r: per half of a part's kOrdLanes lanes the first of its
+  const int* part0;      // processor-local DIC: [C + 1] first part of each CTA
+  // exact DIC, the order of w.r: per half of a part's kOrdLanes lanes the first of its
   // steps, per step the PCG row of each of 32 lanes, -1: none
   const int* ordStep;    // [2 nParts + 1]
   const int* ordRow;     // [steps][32]
 };
 constexpr int kOrdLanes = 64;  // lanes of a part's w.r sum: the threads of kSweepSm
-// Records of the FP64 form's ordered sums: two of a part, two of 32 storage rows,
-// three values each.
-inline size_t ordRecords(int nParts, int nC) { return 6 * ((size_t)nParts + (nC + 31) / 32); }
+// Values of the sums' records (kernels_resident.cu): 12 of a part, 9 of 32 storage rows.
+inline size_t ordRecords(int nParts, int nC) { return 12 * (size_t)nParts + 9 * (size_t)((nC + 31) / 32); }
 // One sweep's table, by row: three coefficients and a word of packed columns
 // (kernels_resident.cu).
 template <typename T> struct ResSweepTab;
@@ -337,14 +337,16 @@ cudaError_t launchPartTables(const MeshView& mv, const PartView& pv, const doubl
 // Sets the kernels' attributes; blocks[2]: resident CTAs per SM of each.
 template <typename T>
 cudaError_t partPrepare(const MeshView& mv, const PartView& pv, int* blocks);
-// 16-byte packets that the CTAs of kPartLoop exchange: w of a row; sums of the
-// CTAs, results and the count of sums (partLoopPackets of them).  Zero before
-// the first launch, used by that kernel alone.
+// 16-byte packets that the CTAs of kPartLoop exchange: w of a row, its term of p.q;
+// records of the sums, results and the count of sums (partLoopPackets of them).  Zero
+// before the first launch and after a launch whose waits gave up; used by that kernel
+// alone.
 struct LoopPtrs {
   uint4* w = nullptr;
+  uint4* t = nullptr;
   uint4* rec = nullptr;
 };
-size_t partLoopPackets(int nParts);
+size_t partLoopPackets(const MeshView& mv);
 // The PCG loop of a corrector in one cooperative launch, a CTA per part, FP32
 // (blocks: resident CTAs per SM, 0 if the parts are too large for it).
 cudaError_t partLoopPrepare(const MeshView& mv, const PartView& pv, int* blocks);

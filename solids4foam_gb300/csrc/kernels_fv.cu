@@ -355,7 +355,7 @@ template <int NM>
 __device__ __forceinline__ double blockSumsMaxima(double (&sums)[4], double (&mx)[NM], int nm, double* smem) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
   constexpr int R = 4 + NM;
-  double v = warpSpreadSum<double, 4>(sums);
+  double v = warpSpreadSum<4>(sums);
 #pragma unroll
   for (int k = 0; k < NM; ++k)
     if (k < nm)
@@ -754,7 +754,7 @@ kRhs(MeshView mv, Controls c, FieldPtrs f, T* __restrict__ x, T* __restrict__ r,
   constexpr int NV = 6;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
   auto blockTotal = [&](double (&v)[8]) {  // value k in the lanes 4 k .. of warp 0
-    double a = warpSpreadSum<double, 8>(v);
+    double a = warpSpreadSum<8>(v);
     if (lane % 4 == 0 && lane / 4 < NV) smem[wid * NV + lane / 4] = a;
     __syncthreads();
     if (wid == 0) {

@@ -1,31 +1,31 @@
-// PCG with the processor-local DIC on the whole device, a CTA per part: two
-// kernels per iteration, for meshes beyond the cluster-resident PCG.
+// PCG with the processor-local DIC on the whole device, a CTA per part, for meshes
+// beyond the cluster-resident PCG; in FP32 three kernels per iteration:
 //
 //   kPartPrecond  r -= alpha q of the pending iteration, sum|r|, w = M^-1 r of
 //                 each part and w.r; the last CTA runs the residual test and
 //                 decides beta.
-//   kPartSpmv     the pending x += alpha p, p_new = w + beta p_old, q = A p_new
-//                 and p.q; the last CTA decides alpha.
+//   kPartSpmv     the pending x += alpha p, p_new = w + beta p_old, q = A p_new.
+//   kPartDot      p.q; the last CTA decides alpha.
 //
-// Both hold a part's rows in shared memory while they work on it: w during the
-// substitutions, p_new -- of the part's rows and of the rows around it that
+// The first two hold a part's rows in shared memory while they work on it: w during
+// the substitutions, p_new -- of the part's rows and of the rows around it that
 // they touch -- during the product, so that a row's six neighbours are shared-
-// memory reads instead of gathers of w and p_old through L1.  The arithmetic of
-// every vector entry is that of the separate kernels (kernels_local.cu), to the
-// bit in FP32; a CTA takes parts b, b + G, ... and adds up its threads' sums
-// once, at the end, and the last CTA adds the CTAs' records in order: the order
-// of the sums depends on the mesh, the value type and the device only.
+// memory reads instead of gathers of w and p_old through L1.  In FP64 the product
+// stays with kernels_local.cu.
 //
-// In FP64 the corrector loop of some processor-local runs amplifies a last bit of
-// a sum a thousandfold every ten correctors (measured: 1e-13 after 60, 2e-6
-// after 100).  There the preconditioner keeps the sums of kernels_local.cu in
-// their order -- 64 lanes over a part's rows, parts in groups of 32
-// (part_sums.cuh) -- and the product and its sums stay with kernels_local.cu.
+// The arithmetic of every vector entry is that of the separate kernels
+// (kernels_local.cu), and so is that of the global sums, to the bit: w.r and sum|r| by
+// 64 lanes over a part's rows, parts in groups of 32 (part_sums.cuh); p.q by storage
+// row, the rows of a thread of the row kernels' grid together, blocks of 256 threads.
+// The corrector loop of some runs amplifies a last bit of a sum a thousandfold every
+// ten correctors (FP64: 1e-13 after 60, 2e-6 after 100), and in FP32 a last bit of the
+// FP64 sum can turn the rounding of alpha or beta.
 //
 // Parts of rows with at most six neighbours that fit shared memory (in FP32
-// at most 1022 rows: 10-bit columns); others run kernels_local.cu.
+// at most 1016 rows: 10-bit columns); others run kernels_local.cu.
 
 #include <algorithm>
+#include <type_traits>
 
 #include "kernels.cuh"
 #include "pcg_common.cuh"
@@ -43,12 +43,12 @@ template <> struct PartCfg<float> {
   // (8 resident CTAs at 123 registers; 6 at 139 before: 128^3 61.4 -> 60.1 us a
   // launch, 16 cases of 40^3 39.4 -> 35.5; fewer rows a thread keeps: 65 and 70 us)
   static constexpr int kNT = 64, kKeep = 8, kOcc = 7;
-  static constexpr bool kSplit = false, kOrdered = false;
+  static constexpr bool kSplit = false;
 };
 template <> struct PartCfg<double> {
   using Ent = ResEnt<double>;
   static constexpr int kNT = 192, kKeep = 3, kOcc = 4;
-  static constexpr bool kSplit = true, kOrdered = true;
+  static constexpr bool kSplit = true;
 };
 constexpr int kPartSpmvThreads = 128;
 
@@ -61,62 +61,16 @@ __device__ __forceinline__ void stRow(T* v, size_t i, const T (&o)[3]) {
   v[3 * i] = o[0]; v[3 * i + 1] = o[1]; v[3 * i + 2] = o[2];
 }
 
-// Sums of N values of every thread of the CTA into its record (rec[value][CTA]),
-// and by the last CTA of the launch over all records: thread t sums CTAs t,
-// t + NT, ..., four records' loads in flight, then a fixed tree.  True in every
-// thread of the last CTA; its threads 0 .. 31 find the sums in out[0..N).
-template <typename T, int NT, int N, int M>
-__device__ __forceinline__ bool gridSum(typename Part<T>::V (&v)[M], typename Part<T>::V* rec,
-                                        typename Part<T>::V* wrec, double* out, unsigned* counter) {
-  using P = Part<T>;
-  using V = typename P::V;
-  constexpr int W = NT / 32, G = 32 / M;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, k = lane / G, g = lane % G;
-  const V s = warpSpreadSum<T, M>(v);
-  if (k < N && g == 0) wrec[wid * N + k] = s;
-  __syncthreads();
-  if (wid == 0) {
-    const V a = warpRecords<T, N, M>(wrec, W);
-    if (k < N && g == 0) rec[(size_t)k * gridDim.x + blockIdx.x] = a;
-    __syncwarp();
-    if (lane < N) __threadfence();
-  }
-  if (!lastBlockDone(counter, gridDim.x)) return false;
-  const int n = (int)gridDim.x;
-#pragma unroll
-  for (int m = 0; m < M; ++m) v[m] = P::zero();
-  for (int j0 = (int)threadIdx.x; j0 < n; j0 += 4 * NT) {
-    V x[4][N];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int m = 0; m < N; ++m)
-        x[u][m] = j0 + u * NT < n ? P::ldcg(rec + (size_t)m * n + j0 + u * NT) : P::zero();
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-      for (int m = 0; m < N; ++m) v[m] = P::add(v[m], x[u][m]);
-  }
-  const V a = warpSpreadSum<T, M>(v);
-  if (k < N && g == 0) wrec[wid * N + k] = a;
-  __syncthreads();
-  if (wid == 0) {
-    const V b = warpRecords<T, N, M>(wrec, W);
-    if (k < N && g == 0) out[k] = P::value(b);
-    __syncwarp();
-  }
-  return true;
-}
-
 template <typename T, bool MORE, bool WIDE>
 __global__ void __launch_bounds__(PartCfg<T>::kNT, PartCfg<T>::kOcc)
 kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p, DevState* st,
              double* partials) {
   using C = PartCfg<T>;
   using E = typename C::Ent;
-  using P = Part<T>;
-  using V = typename P::V;
   constexpr int NT = C::kNT, KR = C::kKeep;
+  // the sums' 64 lanes: lane l the rows l, l + 64, ... of a part.  With 64 threads they
+  // are the thread's own rows.
+  constexpr bool OWN = NT == 64;
   constexpr unsigned kU = URow<T>::kBytes, kB = E::kB;
   p = casePcg(p, blockIdx.y, mv.nC);
   st += blockIdx.y;
@@ -124,7 +78,6 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
   if (!st->pcgContinue) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ __align__(16) int4 sDesc[2][2];
-  __shared__ V wrec[6 * (NT / 32)];
   __shared__ double sum[12];
   __shared__ int sGroup;
   const int t = (int)threadIdx.x, cap = pv.capRows;
@@ -142,11 +95,10 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
     }
   }
   const unsigned lva = at + 16;  // two empty levels before the first
-  // (ordered sums) the part's residual, in the tables' place after the sweeps
+  // (not OWN) the part's residual, in the tables' place after the sweeps
   T* const sr = (T*)(smraw + (ad[0].q - uBase));
   double* grec = partials + mv.locGrpOff;
   unsigned* gcnt = reinterpret_cast<unsigned*>(grec + 8 * (size_t)mv.locGroups);
-  int prev = -1;
   const T* __restrict__ qg = p.q;
   const T* __restrict__ rDg = p.rD;
   T* __restrict__ rg = p.r;
@@ -167,7 +119,6 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
   }
   cpAsyncWaitAll();
   __syncthreads();
-  Acc<T> wr[3], ar[3];
   for (int buf = 0; part < nParts; part += (int)gridDim.x, buf ^= 1) {
     const int4 dA = sDesc[buf][0], dB = sDesc[buf][1];
     const int pLo = dA.x, nR = dA.y, l0 = dB.z, nL = dB.w;
@@ -176,9 +127,6 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
       cpAsync16(&sDesc[buf ^ 1][0], mv.locDesc + 2 * next);
       cpAsync16(&sDesc[buf ^ 1][1], mv.locDesc + 2 * next + 1);
     }
-    // the previous part's record is reported on its group's counter
-    bool done = false;
-    if (C::kOrdered && t == 0 && prev >= 0) done = locArrive(gcnt, prev, nParts);
     // the part's tables in flight while the vectors stream
     for (int i = t; i < nR; i += NT)
 #pragma unroll
@@ -251,7 +199,8 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
       resSweepBody<1, false, false, C::kSplit, MORE, WIDE, E>(pt.sweep[1], pt.more[1], ad[1], uBase, 0u,
                                                               lva, nL, NT, 0);
     }
-    // w out, w.r and sum|r| over the thread's rows in row order
+    // w out, w.r and sum|r| of the lane's rows in row order
+    Acc<T> wr[3], ar[3];
 #pragma unroll
     for (int j = 0; j < KR; ++j) {
       const int i = t + j * NT;
@@ -261,12 +210,12 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
         stRow(p.w, (size_t)(pLo + i), w);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-          if (C::kOrdered) {
+          if (OWN) {
+            wr[k].add(mulT(w[k], rK[j][k]));
+            ar[k].add(fabs(rK[j][k]));
+          } else {
             sr[3 * i + k] = rK[j][k];
-            continue;
           }
-          wr[k].add(mulT(w[k], rK[j][k]));
-          ar[k].add(fabs(rK[j][k]));
         }
       }
     }
@@ -277,69 +226,70 @@ kPartPrecond(MeshView mv, Controls c, PartView pv, PartPtrs<T> pt, PcgPtrs<T> p,
 #pragma unroll
       for (int k = 0; k < 3; ++k) {
         const T r = rg[3 * (size_t)(pLo + i) + k];  // written by this thread
-        if (C::kOrdered) {
+        if (OWN) {
+          wr[k].add(mulT(w[k], r));
+          ar[k].add(fabs(r));
+        } else {
           sr[3 * i + k] = r;
-          continue;
         }
-        wr[k].add(mulT(w[k], r));
-        ar[k].add(fabs(r));
       }
     }
-    if (C::kOrdered) {
-      // lane l of 64 sums rows l, l + 64, ..., then a fixed tree: sum64's, by the
-      // spread sum (9 additions a warp for 30)
-      __syncthreads();
-      const int k = (t & 31) / 4;
-      double s6 = 0;
-      if (t < 64) {
-        double d[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (!OWN) __syncthreads();
+    // then a fixed tree: sum64's
+    // w.r of component k in lane 8 k, sum|r| in lane 8 k + 1
+    const int l8 = t & 7, k3 = (t & 31) >> 3;
+    double s6 = 0;
+    if (t < 64) {
+      double d[2];
+      if constexpr (OWN) {
+        const T x[2][3] = {{wr[0].s, wr[1].s, wr[2].s}, {ar[0].s, ar[1].s, ar[2].s}};
+        const T e[2][3] = {{wr[0].c, wr[1].c, wr[2].c}, {ar[0].c, ar[1].c, ar[2].c}};
+        warpFloatSums<2, true>(x, e, d);
+      } else {
+        double v[2][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}};
         for (int i = t; i < nR; i += 64) {
           T w[3];
           URow<T>::load(uBase + kU * (unsigned)i, w);
 #pragma unroll
           for (int m = 0; m < 3; ++m) {
             const T r = sr[3 * i + m];
-            d[m] = fma((double)w[m], (double)r, d[m]);
-            d[3 + m] += fabs((double)r);
+            v[0][m] = fma((double)w[m], (double)r, v[0][m]);
+            v[1][m] += fabs((double)r);
           }
         }
-        s6 = warpSpreadSum<double, 8>(d);
-        if (t >= 32 && t % 4 == 0 && k < 6) sum[k] = s6;
+        warpSpreadSums<4, 2>(v, d);
       }
-      if (t == 0) sGroup = done ? prev / kLocGroup : -1;
-      __syncthreads();
-      if (t < 32 && t % 4 == 0 && k < 6) partials[8 * (size_t)part + k] = s6 + sum[k];
-      if (sGroup >= 0 && t < 32) locGroupSum(partials, grec, gcnt, sGroup, nParts);
-      prev = part;
+      s6 = l8 == 0 ? d[0] : d[1];
+      if (t >= 32 && l8 < 2 && k3 < 3) sum[3 * l8 + k3] = s6;
     }
-    __syncthreads();  // the next part reuses the shared memory
+    __syncthreads();  // the next part reuses the vector and the tables
+    if (t < 32 && l8 < 2 && k3 < 3) partials[8 * (size_t)part + 3 * l8 + k3] = s6 + sum[3 * l8 + k3];
   }
-  if (C::kOrdered) {
-    locFinish(mv, c, st, partials, prev, anyPend, sum, &sGroup);
-    return;
+  // the records are reported on their groups' counters at the end (a fence for every part
+  // would wait for the part's w to drain, some 1.5 us each)
+  if (t < 32) {
+    __syncwarp();
+    const int step = (int)gridDim.x;
+    for (int p0 = (int)blockIdx.x; p0 < nParts; p0 += 32 * step) {
+      const long mine = p0 + (long)t * step;
+      unsigned full = __ballot_sync(0xffffffffu, mine < nParts && locArrive(gcnt, (int)mine, nParts));
+      for (; full; full &= full - 1)
+        locGroupSum(partials, grec, gcnt, (p0 + (__ffs((int)full) - 1) * step) / kLocGroup, nParts);
+    }
   }
-  V v[8] = {P::of(wr[0]), P::of(wr[1]), P::of(wr[2]), P::of(ar[0]),
-            P::of(ar[1]), P::of(ar[2]), P::zero(), P::zero()};
-  if (!gridSum<T, NT, 6>(v, (V*)partials, wrec, sum, &st->counter[5])) return;
-  if (t >= 32) return;
-  if (t == 0) st->counter[5] = 0;
-  pcgDecideBeta(c, st, t < 6 ? sum[t] : 0.0, anyPend);
+  __syncthreads();
+  locFinish(mv, c, st, partials, -1, anyPend, sum, &sGroup);
 }
 
 __global__ void __launch_bounds__(kPartSpmvThreads, 8)
-kPartSpmv(MeshView mv, PartView pv, PartPtrs<float> pt, PcgPtrs<float> p, DevState* st, double* partials) {
+kPartSpmv(MeshView mv, PartView pv, PartPtrs<float> pt, PcgPtrs<float> p, const DevState* st) {
   using T = float;
-  using P = Part<T>;
-  using V = typename P::V;
   constexpr int NT = kPartSpmvThreads, RP = 1, KH = 4;
   constexpr unsigned kU = URow<T>::kBytes;
   p = casePcg(p, blockIdx.y, mv.nC);
   st += blockIdx.y;
-  partials += (size_t)blockIdx.y * mv.caseRec;
   if (!st->pcgContinue) return;
   extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ V wrec[3 * (NT / 32)];
-  __shared__ double sum[4];
   const unsigned uBase = (unsigned)__cvta_generic_to_shared(smraw);
   const int t = (int)threadIdx.x;
   const int pb = st->pbuf;
@@ -355,7 +305,6 @@ kPartSpmv(MeshView mv, PartView pv, PartPtrs<float> pt, PcgPtrs<float> p, DevSta
     act[k] = st->active[k] != 0; first[k] = st->nIter[k] == 0; b[k] = (T)st->beta[k];
     xp[k] = st->xPend[k] != 0; al[k] = (T)st->alpha[k];
   }
-  Acc<T> pq[3];
   // the part's first row, rows and halo, read a part ahead
   int part = (int)blockIdx.x, pLo = 0, nR = 0, nH = 0;
   if (part < mv.nParts) {
@@ -467,39 +416,104 @@ kPartSpmv(MeshView mv, PartView pv, PartPtrs<float> pt, PcgPtrs<float> p, DevSta
         for (int k = 0; k < 3; ++k) y[k] = fmaT(a[e], x[e][k], y[k]);
       const size_t g = 3 * (size_t)(pLo + i);
 #pragma unroll
-      for (int k = 0; k < 3; ++k) {
+      for (int k = 0; k < 3; ++k)
         if (act[k]) qo[g + k] = y[k];
-        pq[k].add(mulT(y[k], v[k]));
-      }
     }
     __syncthreads();
     part = next; pLo = pLo1; nR = nR1 - pLo1; nH = nH1;
   }
-  V v[4] = {P::of(pq[0]), P::of(pq[1]), P::of(pq[2]), P::zero()};
-  if (!gridSum<T, NT, 3>(v, (V*)partials, wrec, sum, &st->counter[6])) return;
+}
+
+// p.q of the product, in the order of kLocSpmv: a thread the storage rows of the row
+// kernels' grid, blocks of 256 threads, then the blocks.  (In the product itself the
+// rows are by part.)  Reads q and p_new, in good part from L2 right after the product.
+__global__ void __launch_bounds__(kRowBlock)
+kPartDot(MeshView mv, PcgPtrs<float> p, DevState* st, double* partials) {
+  p = casePcg(p, blockIdx.y, mv.nC);
+  st += blockIdx.y;
+  partials += (size_t)blockIdx.y * mv.caseRec;
+  if (!st->pcgContinue) return;
+  constexpr int W = kRowBlock / 32, B = 7;
+  __shared__ double red[3 * W];
+  const int t = (int)threadIdx.x, lane = t & 31, wid = t >> 5;
+  const int pb = st->pbuf;
+  const float* __restrict__ pn = pb ? p.p : p.p2;
+  const float* __restrict__ q = p.q;
+  const int step = (int)(gridDim.x * kRowBlock);
+  Acc<float> a[3];
+  for (int s0 = (int)blockIdx.x * kRowBlock + t; s0 < mv.nC; s0 += B * step) {
+    float y[B][3], v[B][3];
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+      if (s0 + u * step < mv.nC) {
+        ldRow(q, (size_t)(s0 + u * step), y[u]);
+        ldRow(pn, (size_t)(s0 + u * step), v[u]);
+      }
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+      if (s0 + u * step < mv.nC)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) a[k].add(mulT(y[u][k], v[u][k]));
+  }
+  // blockSum's order, by the spread sum
+  auto blockTotal = [&](double s) {  // value k in thread k, from the warps' sums in lanes 8 k
+    if ((lane & 7) == 0 && lane < 24) red[3 * wid + (lane >> 3)] = s;
+    __syncthreads();
+    double o = 0;
+    if (t < 3) {
+      o = red[t];
+#pragma unroll
+      for (int w = 1; w < W; ++w) o += red[3 * w + t];
+    }
+    return o;
+  };
+  const float x[1][3] = {{a[0].s, a[1].s, a[2].s}}, cmp[1][3] = {{a[0].c, a[1].c, a[2].c}};
+  double own[1];
+  warpFloatSums<1, true>(x, cmp, own);
+  const double mine = blockTotal(own[0]);
+  if (t < 3) {
+    partials[8 * (size_t)blockIdx.x + t] = mine;
+    __threadfence();
+  }
+  if (!lastBlockDone(&st->counter[6], gridDim.x)) return;
+  double v[4] = {0, 0, 0, 0};
+  for (int j = t; j < (int)gridDim.x; j += kRowBlock)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const double x = __ldcg(partials + 8 * (size_t)j + k);
+      v[k] = j == t ? x : v[k] + x;
+    }
+  const double total = blockTotal(warpSpreadSum<4>(v));
   if (t >= 32) return;
   if (t == 0) st->counter[6] = 0;
-  pcgDecideAlpha(st, t < 3 ? sum[t] : 0.0, pb);
+  pcgDecideAlpha(st, total, pb);
 }
 
 // ---- the whole loop of a corrector in one launch ---------------------------------
 // Meshes whose parts are all resident at once (a CTA per part; FP32): the
-// launches of kPartPrecond and kPartSpmv, their reading of the state and their
-// ends take longer than a part's work, so one cooperative launch runs the PCG
-// loop of a corrector.  r, x, p and q stay in registers, the tables in shared
-// memory; the part's halo keeps its p in shared memory and needs only w from
-// other parts once per iteration.
+// launches of the part kernels, their reading of the state and their ends take longer
+// than a part's work, so one cooperative launch runs the PCG loop of a corrector.
+// r, x, p and q stay in registers, the tables in shared memory; the part's halo keeps
+// its p in shared memory and needs only w from other parts once per iteration.
 //
 // What CTAs tell one another goes through 16-byte packets that carry their own
 // tag (the count of sums so far): a reader polls the packet itself, so neither a
 // counter nor a fence stands between a value and its use.  Rows publish w; a CTA
-// publishes its part of a sum, CTA 0 adds the parts up, decides and publishes the
-// result in kLoopCopies lines.  (With a counter, fences and the last CTA deciding
-// on the state in memory a sum took 7 us of a 27 us iteration of 512 parts.)  A
-// packet is written again only after its readers have taken part in a later sum.
+// publishes its records of a sum, CTA 0 adds the records up, decides and publishes the
+// result in kLoopCopies lines.  A packet is written again only after its readers have
+// taken part in a later sum.
+//
+// The sums have the order of kernels_local.cu (the comment at the top):
+//   w.r, sum|r|  64 lanes over the part's rows, lane l the rows l, l + 64, ...: the
+//                first half of them in thread l, the rest in thread l + 64, which goes
+//                on with that thread's sum (sum|r|'s second half runs beside the walk).
+//                A record of six values per part; CTA 0 adds up groups of 32 parts.
+//   p.q          blocks of 256 storage rows, in each lane the rows a row kernels' grid
+//                apart.  A block is added up by the CTA that owns its first row; the rows
+//                of it that other CTAs own come as packets.
 constexpr int kLoopThreads = 128, kLoopRows = 4, kLoopWalk = 64;
 constexpr int kLoopMaxRows = kLoopThreads * kLoopRows;
-constexpr int kLoopAhead = 2;  // CTAs whose packets a thread of CTA 0 has in flight
+constexpr int kLoopAhead = 2;  // part groups whose packets a warp of CTA 0 has in flight
 constexpr int kLoopCopies = 32, kLoopLine = 8;  // result packets, 128 bytes apart
 
 __device__ __forceinline__ uint4 ldPacket(const uint4* p) {
@@ -521,67 +535,101 @@ __device__ __forceinline__ bool waitPacket(const uint4* p, unsigned tag, int shi
     if (++it > limit) return false;
   return true;
 }
-
-// All CTAs' sums of N values.  A CTA's packets: the first parts of three values'
-// compensated sums, their second parts, the same of the next three.  CTA 0 leaves
-// the sums in its warp 0 (value k in lane k) and returns whether all came.
-template <int N, int M>
-__device__ __forceinline__ bool gridPut(float2 (&v)[M], uint4* rec, float2* wrec, unsigned tag, int limit,
-                                        double& mine) {
-  using P = Part<float>;
-  constexpr int NT = kLoopThreads, W = NT / 32, G = 32 / M, Q = 2 * N / 3;
-  const int t = (int)threadIdx.x, lane = t & 31, wid = t >> 5, k = lane / G, g = lane % G;
-  const int n = (int)gridDim.x;
-  const float2 s = warpSpreadSum<float, M>(v);
-  if (k < N && g == 0) wrec[wid * N + k] = s;
-  __syncthreads();
-  if (wid == 0) {
-    const float2 a = warpRecords<float, N, M>(wrec, W);
-    unsigned b[3];
+// N packets with this tag (addr(n) null: none), polled together: one after the other,
+// each would cost a round trip to L2 of its own once its first load came too early.
+template <int N, typename F>
+__device__ __forceinline__ bool waitPackets(F addr, unsigned tag, int limit, uint4 (&v)[N]) {
 #pragma unroll
-    for (int m = 0; m < 3; ++m) {
-      const int from = (3 * ((lane % Q) >> 1) + m) * G;
-      const float x = __shfl_sync(0xffffffffu, a.x, from), y = __shfl_sync(0xffffffffu, a.y, from);
-      b[m] = __float_as_uint((lane & 1) ? y : x);
-    }
-    if (lane < Q) stPacket(rec + (size_t)lane * n + blockIdx.x, b[0], b[1], b[2], tag);
+  for (int n = 0; n < N; ++n) v[n] = addr(n) ? ldPacket(addr(n)) : make_uint4(0, 0, 0, tag);
+  for (int it = 0;;) {
+    bool all = true;
+#pragma unroll
+    for (int n = 0; n < N; ++n) all = all && v[n].w == tag;
+    if (all) return true;
+    if (++it > limit) return false;
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+      if (v[n].w != tag) v[n] = ldPacket(addr(n));
   }
-  if (blockIdx.x != 0) return true;
-  // thread t adds up the CTAs t, t + NT, ..., kLoopAhead at a time
+}
+// FP64 values in packets: value k in the words 2 k, 2 k + 1; three words a packet.
+__device__ __forceinline__ unsigned valueWord(double v, int w) {
+  return (unsigned)((w & 1) ? __double2hiint(v) : __double2loint(v));
+}
+__device__ __forceinline__ double wordsValue(unsigned lo, unsigned hi) {
+  return __hiloint2double((int)hi, (int)lo);
+}
+// CTA 0: the sum over the parts' records (value k in lane k of warp 0); false if some did
+// not come.  grp: 6 values of each of 64 lanes over the groups; out: 6 values.
+__device__ __forceinline__ bool loopPartTotal(const uint4* rec, int n, double* grp, double* out, unsigned tag,
+                                              int limit, double& mine) {
+  constexpr int W = kLoopThreads / 32, A = kLoopAhead;
+  const int lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5, nGrp = (n + 31) / 32;
   bool ok = true;
+  for (int g0 = wid; g0 < nGrp; g0 += A * W) {
+    uint4 x[4 * A];
+    ok = waitPackets(
+             [&](int i) {
+               const int part = 32 * (g0 + i / 4 * W) + lane;
+               return part < n ? rec + (size_t)(i % 4) * n + part : (const uint4*)nullptr;
+             },
+             tag, limit, x) && ok;
 #pragma unroll
-  for (int m = 0; m < M; ++m) v[m] = P::zero();
-  for (int j0 = t; j0 < n; j0 += kLoopAhead * NT) {
-    uint4 x[kLoopAhead][Q];
-#pragma unroll
-    for (int u = 0; u < kLoopAhead; ++u)
-#pragma unroll
-      for (int q = 0; q < Q; ++q)
-        x[u][q] = j0 + u * NT < n ? ldPacket(rec + (size_t)q * n + j0 + u * NT) : make_uint4(0, 0, 0, tag);
-#pragma unroll
-    for (int u = 0; u < kLoopAhead; ++u)
-#pragma unroll
-      for (int q = 0; q < Q; ++q)
-        if (x[u][q].w != tag)
-          ok = waitPacket(rec + (size_t)q * n + j0 + u * NT, tag, 0, limit, x[u][q]) && ok;
-#pragma unroll
-    for (int u = 0; u < kLoopAhead; ++u)
-#pragma unroll
-      for (int q = 0; q < Q; q += 2) {
-        const uint4 h = x[u][q], l = x[u][q + 1];
-        const int m = 3 * (q / 2);
-        v[m] = P::add(v[m], make_float2(__uint_as_float(h.x), __uint_as_float(l.x)));
-        v[m + 1] = P::add(v[m + 1], make_float2(__uint_as_float(h.y), __uint_as_float(l.y)));
-        v[m + 2] = P::add(v[m + 2], make_float2(__uint_as_float(h.z), __uint_as_float(l.z)));
+    for (int u = 0; u < A; ++u) {
+      const int g = g0 + u * W;
+      if (g >= nGrp) break;
+      const uint4 *const y = x + 4 * u;
+      double v[8] = {wordsValue(y[0].x, y[0].y), wordsValue(y[0].z, y[1].x), wordsValue(y[1].y, y[1].z),
+                     wordsValue(y[2].x, y[2].y), wordsValue(y[2].z, y[3].x), wordsValue(y[3].y, y[3].z), 0, 0};
+      const double s = warpSpreadSum<8>(v);
+      if ((lane & 3) == 0 && lane < 24) {
+        double* const o = grp + 6 * (g & 63) + (lane >> 2);
+        *o = g < 64 ? s : *o + s;
       }
+    }
   }
-  const float2 a = warpSpreadSum<float, M>(v);
-  __syncthreads();  // (warp 0 has read the records of its CTA)
-  if (k < N && g == 0) wrec[wid * N + k] = a;
   ok = __syncthreads_and(ok) != 0;
-  if (wid == 0) {
-    const float2 b = warpRecords<float, N, M>(wrec, W);
-    mine = __shfl_sync(0xffffffffu, P::value(b), lane < N ? lane * G : 0);
+  groupTotal<W>(grp, nGrp, out);
+  __syncthreads();
+  if (lane < 6) mine = out[lane];
+  return ok;
+}
+// CTA 0: the sum over the n row blocks' records (reducePartials with 256 threads), value k
+// in lane k of warp 0.  red: 24 values.
+__device__ __forceinline__ bool loopBlockTotal(const uint4* rec, int n, double* red, unsigned tag, int limit,
+                                               double& mine) {
+  constexpr int NT = kLoopThreads;
+  const int t = (int)threadIdx.x, lane = t & 31, wid = t >> 5;
+  bool ok = true;
+  double v[2][4], s[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) v[h][0] = v[h][1] = v[h][2] = v[h][3] = 0;
+  for (int j0 = t; j0 < n; j0 += kRowBlock) {
+    uint4 x[4];
+    ok = waitPackets(
+             [&](int i) {
+               const int j = j0 + NT * (i / 2);
+               return j < n ? rec + (size_t)(i % 2) * n + j : (const uint4*)nullptr;
+             },
+             tag, limit, x) && ok;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint4 &y0 = x[2 * h], &y1 = x[2 * h + 1];
+      const double d[3] = {wordsValue(y0.x, y0.y), wordsValue(y0.z, y1.x), wordsValue(y1.y, y1.z)};
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[h][k] = j0 == t ? d[k] : v[h][k] + d[k];
+    }
+  }
+  warpSpreadSums<4, 2>(v, s);
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    if ((lane & 7) == 0 && lane < 24) red[3 * (wid + 4 * h) + (lane >> 3)] = s[h];
+  ok = __syncthreads_and(ok) != 0;
+  if (t < 3) {
+    double a = red[t];
+#pragma unroll
+    for (int w = 1; w < kRowBlock / 32; ++w) a += red[3 * w + t];
+    mine = a;
   }
   return ok;
 }
@@ -601,28 +649,36 @@ kPartLoop(MeshView mv, Controls c, PartView pv, PartPtrs<float> pt, LoopPtrs lp,
           DevState* st) {
   using T = float;
   using E = PartEnt;
-  using P = Part<T>;
   constexpr int NT = kLoopThreads, KR = kLoopRows, KH = 4;
   constexpr unsigned kU = URow<T>::kBytes;
   if (!st->pcgContinue) return;  // the same in every CTA: CTA 0 writes the state at its end
   extern __shared__ __align__(16) unsigned char smraw[];
-  __shared__ float2 wrec[6 * (NT / 32)];
+  __shared__ double grp[64 * 6];  // (CTA 0: sums over part groups); before that, in sums of
+  float2* const hand = reinterpret_cast<float2*>(grp);  // lanes: the first halves' sums [3][64]
+  __shared__ double red[6], blk[2][24];
   __shared__ T sVal[3];
   __shared__ unsigned sFlags;
   __shared__ DevState sst;  // CTA 0: the state while the loop runs
   const int t = (int)threadIdx.x, cap = pv.capRows, part = (int)blockIdx.x, nP = (int)gridDim.x;
+  const int lane = t & 31, wid = t >> 5;
   const int pLo = mv.partStart[part], nR = mv.partStart[part + 1] - pLo, nH = pv.haloCnt[part];
   const int l0 = mv.lvlOff[part], nL = mv.lvlOff[part + 1] - l0;
   const bool lead = part == 0;
   // (a shorter limit is for the waits between parts of the exact DIC's sweeps)
   const int limit = mv.spinLimit > kSpinLimit ? mv.spinLimit : kSpinLimit;
+  // the thread's rows: i0, i0 + 64, ..., nMine of them
+  const int half = (nR + 127) / 128, i0 = (t & 63) + (t >> 6) * 64 * half;
+  const int nMine = i0 < nR ? min(half, (nR - i0 + 63) / 64) : 0;
+  // the row blocks that the CTA adds up, the distance of a lane's rows
+  const int nB = mv.rowGrid, stride = nB * kRowBlock, b0 = (pLo + kRowBlock - 1) / kRowBlock;
+  const int nMyB = min((pLo + nR + kRowBlock - 1) / kRowBlock, nB) - b0;  // at most 2
   uint4* const rec2 = lp.rec + 4 * (size_t)nP;
-  uint4* const out = rec2 + 2 * (size_t)nP;
+  uint4* const out = rec2 + 2 * (size_t)nB;
   unsigned* const count = reinterpret_cast<unsigned*>(out + kLoopLine * kLoopCopies);
   unsigned tag = ldRelaxed(count);  // of the last sum; CTA 0 writes it at its end
   const uint4* const mine = out + kLoopLine * (part % kLoopCopies);
-  // ---- shared memory: w or p of the rows, the zero row, p of the halo | sweep
-  //      tables | level bounds | product coefficients | product columns
+  // ---- shared memory: w, p or p.q's terms of the rows, the zero row, p of the halo |
+  //      sweep tables | level bounds | product coefficients | product columns
   const unsigned uBase = (unsigned)__cvta_generic_to_shared(smraw);
   const int halo0 = cap + 4;
   ResAddr ad[2];
@@ -667,12 +723,12 @@ kPartLoop(MeshView mv, Controls c, PartView pv, PartPtrs<float> pt, LoopPtrs lp,
   T r[KR][3], x[KR][3], pp[KR][3], q[KR][3], rd[KR], dg[KR];
 #pragma unroll
   for (int j = 0; j < KR; ++j) {
-    const int i = t + j * NT;
-    rd[j] = i < nR ? p.rD[pLo + i] : T(0);
-    dg[j] = i < nR ? p.diag[pLo + i] : T(0);
+    const int i = i0 + 64 * j;
+    rd[j] = j < nMine ? p.rD[pLo + i] : T(0);
+    dg[j] = j < nMine ? p.diag[pLo + i] : T(0);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-      r[j][k] = i < nR ? p.r[3 * (size_t)(pLo + i) + k] : T(0);
+      r[j][k] = j < nMine ? p.r[3 * (size_t)(pLo + i) + k] : T(0);
       x[j][k] = 0; pp[j][k] = 0; q[j][k] = 0;
     }
   }
@@ -691,49 +747,162 @@ kPartLoop(MeshView mv, Controls c, PartView pv, PartPtrs<float> pt, LoopPtrs lp,
     }
     ok = __syncthreads_and(ok) != 0;
   };
+  // a lane's sums between its two threads
+  auto handOver = [&](const Acc<T> (&a)[3]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) hand[64 * k + t] = make_float2(a[k].s, a[k].c);
+  };
+  auto takeOver = [&](Acc<T> (&a)[3]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float2 h = hand[64 * k + t - 64];
+      a[k].s = h.x; a[k].c = h.y;
+    }
+  };
+  auto laneSums = [](const Acc<T> (&a)[3]) {  // component k in lane 8 k
+    const T x[1][3] = {{a[0].s, a[1].s, a[2].s}}, e[1][3] = {{a[0].c, a[1].c, a[2].c}};
+    double s[1];
+    warpFloatSums<1, true>(x, e, s);
+    return s[0];
+  };
+  // p.q of the CTA's NB row blocks: the warps' sums in blk.  The terms of the CTA's own rows
+  // are in the shared vector.
+  auto blockSums = [&](auto nb) {
+    constexpr int NB = decltype(nb)::value;
+    bool came = true;
+    Acc<T> a[2 * NB][3];
+    const bool two = mv.nC > stride;
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      if (e == 1 && !two) break;
+      auto rowOf = [&](int n) { return b0 * kRowBlock + NT * n + t + stride * e; };
+      uint4 pk[2 * NB];
+      came = waitPackets(
+                 [&](int n) {
+                   const int row = rowOf(n);
+                   return row < mv.nC && (row < pLo || row >= pLo + nR) ? lp.t + row : (const uint4*)nullptr;
+                 },
+                 tag, limit, pk) && came;
+#pragma unroll
+      for (int n = 0; n < 2 * NB; ++n) {
+        const int row = rowOf(n);
+        if (row >= mv.nC) continue;
+        T u[3];
+        if (row < pLo || row >= pLo + nR) {
+          u[0] = __uint_as_float(pk[n].x); u[1] = __uint_as_float(pk[n].y); u[2] = __uint_as_float(pk[n].z);
+        } else {
+          URow<T>::load(uBase + kU * (unsigned)(row - pLo), u);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          if (e == 0) a[n][k].s = u[k];
+          else a[n][k].add(u[k]);
+      }
+    }
+    T x[2 * NB][3], cmp[2 * NB][3];
+    double s[2 * NB];
+#pragma unroll
+    for (int n = 0; n < 2 * NB; ++n)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) { x[n][k] = a[n][k].s; cmp[n][k] = a[n][k].c; }
+    if (two) warpFloatSums<2 * NB, true>(x, cmp, s);
+    else warpFloatSums<2 * NB>(x, s);
+#pragma unroll
+    for (int n = 0; n < 2 * NB; ++n)
+      if ((lane & 7) == 0 && lane < 24) blk[n >> 1][3 * (wid + 4 * (n & 1)) + (lane >> 3)] = s[n];
+    return came;
+  };
   for (;;) {
     ++tag;
-    // pending r -= alpha q, sum|r|, w = rD r
-    Acc<T> ar[3], wr[3];
+    // pending r -= alpha q, w = rD r; sum|r| of the lanes' first halves
 #pragma unroll
-    for (int j = 0; j < KR; ++j) {
-      const int i = t + j * NT;
-      if (i < nR) {
+    for (int j = 0; j < KR; ++j)
+      if (j < nMine) {
         T w[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
           if (pend >> k & 1) r[j][k] = fmaT(-al[k], q[j][k], r[j][k]);
-          ar[k].add(fabs(r[j][k]));
           w[k] = mulT(rd[j], r[j][k]);
         }
-        URow<T>::store(uBase + kU * (unsigned)i, w);
+        URow<T>::store(uBase + kU * (unsigned)(i0 + 64 * j), w);
       }
-    }
-    __syncthreads();
-    if (nL > 1 && t < kLoopWalk) {
-      resSweepBody<0, false, false, false, MORE, WIDE, E>(pt.sweep[0], pt.more[0], ad[0], uBase, 0u, lva,
-                                                          nL, kLoopWalk, 0);
-      resSweepBody<1, false, false, false, MORE, WIDE, E>(pt.sweep[1], pt.more[1], ad[1], uBase, 0u, lva,
-                                                          nL, kLoopWalk, 0);
-    }
-    __syncthreads();
+    Acc<T> ar[3], wr[3];
+    auto addAbs = [&]() {
 #pragma unroll
-    for (int j = 0; j < KR; ++j) {
-      const int i = t + j * NT;
-      if (i < nR) {
+      for (int j = 0; j < KR; ++j)
+        if (j < nMine)
+#pragma unroll
+          for (int k = 0; k < 3; ++k) ar[k].add(fabs(r[j][k]));
+    };
+    if (t < 64) {
+      addAbs();
+      handOver(ar);
+    }
+    __syncthreads();
+    double absHalf = 0;  // (warps 2, 3) sum|r| over half of the lanes: value k in lane 8 k
+    if (t < kLoopWalk) {
+      if (nL > 1) {
+        resSweepBody<0, false, false, false, MORE, WIDE, E>(pt.sweep[0], pt.more[0], ad[0], uBase, 0u, lva,
+                                                            nL, kLoopWalk, 0);
+        resSweepBody<1, false, false, false, MORE, WIDE, E>(pt.sweep[1], pt.more[1], ad[1], uBase, 0u, lva,
+                                                            nL, kLoopWalk, 0);
+      }
+    } else {
+      takeOver(ar);
+      addAbs();
+      absHalf = laneSums(ar);
+    }
+    __syncthreads();
+    auto addDots = [&]() {
+#pragma unroll
+      for (int j = 0; j < KR; ++j)
+        if (j < nMine) {
+          T w[3];
+          URow<T>::load(uBase + kU * (unsigned)(i0 + 64 * j), w);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) wr[k].add(mulT(w[k], r[j][k]));
+        }
+    };
+#pragma unroll
+    for (int j = 0; j < KR; ++j)
+      if (j < nMine) {
+        const int i = i0 + 64 * j;
         T w[3];
         URow<T>::load(uBase + kU * (unsigned)i, w);
         stPacket(lp.w + pLo + i, __float_as_uint(w[0]), __float_as_uint(w[1]), __float_as_uint(w[2]), tag);
-#pragma unroll
-        for (int k = 0; k < 3; ++k) wr[k].add(mulT(w[k], r[j][k]));
+      }
+    if (t < 64) {
+      addDots();
+      handOver(wr);
+    }
+    __syncthreads();
+    double dotHalf = 0;
+    if (t >= 64) {
+      takeOver(wr);
+      addDots();
+      dotHalf = laneSums(wr);
+      if (wid == 3 && (lane & 7) == 0 && lane < 24) {
+        red[lane >> 3] = dotHalf;
+        red[3 + (lane >> 3)] = absHalf;
       }
     }
-    {
-      float2 v[8] = {P::of(wr[0]), P::of(wr[1]), P::of(wr[2]), P::of(ar[0]),
-                     P::of(ar[1]), P::of(ar[2]), P::zero(), P::zero()};
+    __syncthreads();
+    if (wid == 2) {
+      const int k = (lane >> 3) % 3;
+      const double d = dotHalf + red[k], a = absHalf + red[3 + k];
+      unsigned b[3];
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const int m = 3 * (lane & 3) + e, from = 8 * ((m >> 1) % 3);
+        const double vd = __shfl_sync(0xffffffffu, d, from), va = __shfl_sync(0xffffffffu, a, from);
+        b[e] = valueWord(m < 6 ? vd : va, m);
+      }
+      if (lane < 4) stPacket(lp.rec + (size_t)lane * nP + part, b[0], b[1], b[2], tag);
+    }
+    if (lead) {
       double sum = 0;
-      ok = gridPut<6>(v, lp.rec, wrec, tag, limit, sum) && ok;
-      if (lead && t < 32) {
+      ok = loopPartTotal(lp.rec, nP, grp, blk[0], tag, limit, sum) && ok;
+      if (t < 32) {
         pcgDecideBeta(c, &sst, sum, pend != 0);
         __syncwarp();
         const bool act = t < 3 && sst.active[t < 3 ? t : 0], first = t < 3 && sst.nIter[t < 3 ? t : 0] == 0;
@@ -747,12 +916,7 @@ kPartLoop(MeshView mv, Controls c, PartView pv, PartPtrs<float> pt, LoopPtrs lp,
     }
     // (the halo's w while CTA 0 decides)
     uint4 wh[KH];
-#pragma unroll
-    for (int j = 0; j < KH; ++j)
-      if (hx[j] >= 0) wh[j] = ldPacket(lp.w + hx[j]);
-#pragma unroll
-    for (int j = 0; j < KH; ++j)
-      if (hx[j] >= 0 && wh[j].w != tag) ok = waitPacket(lp.w + hx[j], tag, 0, limit, wh[j]) && ok;
+    ok = waitPackets([&](int j) { return hx[j] >= 0 ? lp.w + hx[j] : (const uint4*)nullptr; }, tag, limit, wh) && ok;
     result();
     if (!ok) break;
     const unsigned fl = sFlags;
@@ -762,9 +926,9 @@ kPartLoop(MeshView mv, Controls c, PartView pv, PartPtrs<float> pt, LoopPtrs lp,
 #pragma unroll
     for (int k = 0; k < 3; ++k) b[k] = sVal[k];
 #pragma unroll
-    for (int j = 0; j < KR; ++j) {
-      const int i = t + j * NT;
-      if (i < nR) {
+    for (int j = 0; j < KR; ++j)
+      if (j < nMine) {
+        const int i = i0 + 64 * j;
         T u[3];
         URow<T>::load(uBase + kU * (unsigned)i, u);
 #pragma unroll
@@ -775,7 +939,6 @@ kPartLoop(MeshView mv, Controls c, PartView pv, PartPtrs<float> pt, LoopPtrs lp,
         }
         URow<T>::store(uBase + kU * (unsigned)i, u);
       }
-    }
     if (!go) break;
 #pragma unroll
     for (int j = 0; j < KH; ++j)
@@ -790,12 +953,11 @@ kPartLoop(MeshView mv, Controls c, PartView pv, PartPtrs<float> pt, LoopPtrs lp,
       }
     __syncthreads();
     ++tag;
-    // q = A p, p.q
-    Acc<T> pq[3];
+    // q = A p
 #pragma unroll
-    for (int j = 0; j < KR; ++j) {
-      const int i = t + j * NT;
-      if (i < nR) {
+    for (int j = 0; j < KR; ++j)
+      if (j < nMine) {
+        const int i = i0 + 64 * j;
         T v[3], y[3], xv[kResW][3];
         URow<T>::load(uBase + kU * (unsigned)i, v);
 #pragma unroll
@@ -809,24 +971,56 @@ kPartLoop(MeshView mv, Controls c, PartView pv, PartPtrs<float> pt, LoopPtrs lp,
           for (int k = 0; k < 3; ++k) y[k] = fmaT(a, xv[e][k], y[k]);
         }
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
+        for (int k = 0; k < 3; ++k)
           if (fl >> k & 1) q[j][k] = y[k];
-          pq[k].add(mulT(y[k], v[k]));
-        }
       }
+    __syncthreads();  // (p of the rows has been read)
+    // the terms of p.q in its place; those that another CTA adds up as packets (a stopped
+    // component's are not used)
+#pragma unroll
+    for (int j = 0; j < KR; ++j)
+      if (j < nMine) {
+        const int i = i0 + 64 * j, row = pLo + i;
+        const int first = (row < stride ? row : row - stride) / kRowBlock * kRowBlock;
+        T u[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) u[k] = mulT(q[j][k], pp[j][k]);
+        if (first < pLo || first >= pLo + nR)
+          stPacket(lp.t + row, __float_as_uint(u[0]), __float_as_uint(u[1]), __float_as_uint(u[2]), tag);
+        URow<T>::store(uBase + kU * (unsigned)i, u);
+      }
+    __syncthreads();
+    if (nMyB == 2) ok = blockSums(std::integral_constant<int, 2>()) && ok;
+    else if (nMyB == 1) ok = blockSums(std::integral_constant<int, 1>()) && ok;
+    __syncthreads();
+    if (wid == 0 && nMyB > 0) {  // the blocks' sums in lanes 0 .. 3 nMyB - 1, then two packets each
+      double s = 0;
+      if (lane < 3 * nMyB) {
+        s = blk[lane / 3][lane % 3];
+#pragma unroll
+        for (int w = 1; w < kRowBlock / 32; ++w) s += blk[lane / 3][3 * w + lane % 3];
+      }
+      unsigned b3[3];
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const int m = 3 * (lane & 1) + e;
+        const double v = __shfl_sync(0xffffffffu, s, 3 * (lane >> 1 & 1) + (m >> 1));
+        b3[e] = valueWord(v, m);
+      }
+      if (lane < 2 * nMyB) stPacket(rec2 + (size_t)(lane & 1) * nB + b0 + (lane >> 1), b3[0], b3[1], b3[2], tag);
     }
-    {
-      float2 v[4] = {P::of(pq[0]), P::of(pq[1]), P::of(pq[2]), P::zero()};
+    if (lead) {
+      __syncthreads();  // (the blocks' records have been read)
       double sum = 0;
-      ok = gridPut<3>(v, rec2, wrec, tag, limit, sum) && ok;
-      if (lead && t < 32) {
+      ok = loopBlockTotal(rec2, nB, blk[0], tag, limit, sum) && ok;
+      if (t < 32) {
         pcgDecideAlpha(&sst, sum, 0);
         __syncwarp();
         const bool on = t < 3 && sst.pending[t < 3 ? t : 0];
         const unsigned f = __ballot_sync(0xffffffffu, on) | (sst.pcgContinue ? 64u : 0u);
-        const T b = t < 3 ? (T)sst.alpha[t] : T(0);
-        resultPut(out, tag, b, f);
-        if (t < 3) sVal[t] = b;
+        const T a = t < 3 ? (T)sst.alpha[t] : T(0);
+        resultPut(out, tag, a, f);
+        if (t < 3) sVal[t] = a;
         if (t == 0) sFlags = f;
       }
     }
@@ -838,13 +1032,11 @@ kPartLoop(MeshView mv, Controls c, PartView pv, PartPtrs<float> pt, LoopPtrs lp,
     if (!(sFlags & 64u)) break;
   }
 #pragma unroll
-  for (int j = 0; j < KR; ++j) {
-    const int i = t + j * NT;
-    if (i < nR) stRow(p.x, (size_t)(pLo + i), x[j]);
-  }
+  for (int j = 0; j < KR; ++j)
+    if (j < nMine) stRow(p.x, (size_t)(pLo + i0 + 64 * j), x[j]);
   if (t == 0 && !ok) atomicOr(&st->status, kErrTimeout);
   if (lead) {
-    // the state back; x is complete.  (No tag of a wait that gave up comes again.)
+    // the state back; x is complete
     __syncthreads();
     if (t < 3) {
       st->active[t] = sst.active[t]; st->nIter[t] = sst.nIter[t]; st->finalRes[t] = sst.finalRes[t];
@@ -857,7 +1049,7 @@ kPartLoop(MeshView mv, Controls c, PartView pv, PartPtrs<float> pt, LoopPtrs lp,
       st->pcgIter = sst.pcgIter;
       st->pcgContinue = sst.pcgContinue;
       if (sst.status) atomicOr(&st->status, sst.status);
-      *count = tag + 4;
+      *count = tag;
     }
   }
 }
@@ -976,7 +1168,7 @@ cudaError_t partPrepare(const MeshView& mv, const PartView& pv, int* blocks) {
   const size_t sm[2] = {precondSmem<T>(mv, pv), spmvSmem(pv)};
   const int nt[2] = {PartCfg<T>::kNT, kPartSpmvThreads};
   blocks[1] = 1;
-  for (int j = 0; j < (PartCfg<T>::kOrdered ? 1 : 2); ++j) {
+  for (int j = 0; j < (sizeof(T) == 8 ? 1 : 2); ++j) {
     cudaError_t e = setMaxDynamicSmem(k[j]);
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks[j], k[j], nt[j], sm[j]);
@@ -997,11 +1189,14 @@ size_t loopSmem(const MeshView& mv, const PartView& pv) {
 }
 }  // namespace
 
-size_t partLoopPackets(int nParts) { return 6 * (size_t)nParts + kLoopLine * kLoopCopies + 1; }
+size_t partLoopPackets(const MeshView& mv) {
+  return 4 * (size_t)mv.nParts + 2 * (size_t)mv.rowGrid + kLoopLine * kLoopCopies + 1;
+}
 
 cudaError_t partLoopPrepare(const MeshView& mv, const PartView& pv, int* blocks) {
   *blocks = 0;
   if (pv.capRows > kLoopMaxRows || pv.haloCap > 4 * kLoopThreads) return cudaSuccess;
+  if (mv.nC > 2 * mv.rowGrid * kRowBlock) return cudaSuccess;  // (two rows a lane of p.q)
   const void* k = loopKernel(pv);
   const cudaError_t e = setMaxDynamicSmem(k);
   if (e != cudaSuccess) return e;
@@ -1053,9 +1248,12 @@ cudaError_t launchPartIteration(const MeshView& mv, const Controls& c, const Par
   }
   {
     TimeScope ts(tm, S4G_K_LOC_SPMV, s);
-    if constexpr (PartCfg<T>::kOrdered) launchLocalSpmv<T>(mv, p, st, partials, t, s, nCases);
-    else
-      kPartSpmv<<<dim3(pv.grid[1], nCases), kPartSpmvThreads, spmvSmem(pv), s>>>(mv, pv, pt, p, st, partials);
+    if constexpr (sizeof(T) == 8) {
+      launchLocalSpmv<T>(mv, p, st, partials, t, s, nCases);
+    } else {
+      kPartSpmv<<<dim3(pv.grid[1], nCases), kPartSpmvThreads, spmvSmem(pv), s>>>(mv, pv, pt, p, st);
+      kPartDot<<<dim3(mv.rowGrid, nCases), kRowBlock, 0, s>>>(mv, p, st, partials);
+    }
   }
   return cudaGetLastError();
 }

@@ -20,14 +20,12 @@
 // levels need a CTA barrier only.  The right-hand-side pass writes r at a
 // row's PCG position and the post pass reads x there (MeshView::pcgPos).
 //
-// Every vector entry is computed by the operations of the separate kernels
-// in the same order (to the last bit).  The global sums are, in FP32, the same
-// compensated sums per thread, added up in FP64, in an order that depends on
-// the mesh and the value type only; in FP64 they are those of kernels_pcg.cu
-// bit for bit (orderedSum below).  Rows have at most kResW neighbours
-// (hexahedra, prisms, tetrahedra); other meshes, and those whose shared row
-// vector does not fit, run the separate kernels.  So does FP64 with the
-// processor-local DIC or the diagonal preconditioner.
+// Every vector entry is computed by the operations of the separate kernels in
+// the same order, and so are the global sums (to the last bit): see "Sums" below.
+// Rows have at most kResW neighbours (hexahedra, prisms, tetrahedra); other
+// meshes, and those whose shared row vector does not fit, run the separate
+// kernels.  So does FP64 with the processor-local DIC or the diagonal
+// preconditioner.
 
 #include <algorithm>
 
@@ -41,6 +39,9 @@ namespace {
 // Forms: exact DIC with a cluster barrier per level, processor-local DIC,
 // diagonal, exact DIC with the substitutions inside one CTA.
 enum { kResExact = 0, kResLocal = 1, kResDiag = 2, kResSingle = 3 };
+// (processor-local, FP32) six values of each of 64 lanes over the part groups, and 15
+// words of up to 32 rows
+constexpr size_t kResGroupBytes = 64 * 6 * sizeof(double) + 15 * 32 * 4;
 
 template <typename T>
 struct ResSweeps {
@@ -80,125 +81,186 @@ __device__ __forceinline__ void sweeps(const ResSweeps<T>& sw, const ResView& rv
   if (!CROSS) __syncthreads();
 }
 
-// Cluster-wide sum of N <= M values of every thread: warp sums, the CTA's sum
-// by warp 0, which stores it in a slot of every CTA's `rec` (rank order), and
-// after the cluster barrier warp 0 of each CTA adds the slots in that order:
-// all CTAs get the same bits.  The sums are left in out[0..N) for warp 0; the
-// caller synchronises the CTA before other warps read what it derives.
-template <typename T, int NT, int N, int M>
-__device__ __forceinline__ void clusterSum(typename Part<T>::V (&v)[M], typename Part<T>::V* wrec,
-                                           typename Part<T>::V* rec, double* out, int C,
-                                           unsigned rank, bool cluster) {
-  constexpr int W = NT / 32, G = 32 / M;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int k = lane / G, g = lane % G;  // the value a lane holds, its copy
-  const typename Part<T>::V s = warpSpreadSum<T, M>(v);
-  if (k < N && g == 0) wrec[wid * N + k] = s;
-  __syncthreads();
-  if (wid == 0) {
-    const typename Part<T>::V a = warpRecords<T, N, M>(wrec, W);
-    if (!cluster) {
-      if (k < N && g == 0) out[k] = Part<T>::value(a);
-    } else if (k < N) {
-      const unsigned at = (unsigned)__cvta_generic_to_shared(rec + (int)rank * N + k);
-      for (int j = g; j < C; j += G) stRemote(mapa(at, (unsigned)j), a);
-    }
-    __syncwarp();
-  }
-  if (cluster) {
-    clArrive();
-    clWait();
-    if (wid == 0) {
-      const typename Part<T>::V a = warpRecords<T, N, M>(rec, C);
-      if (k < N && g == 0) out[k] = Part<T>::value(a);
-      __syncwarp();
-    }
-  }
-}
-
 // Barrier between phases: of the cluster, or of its only CTA.
 __device__ __forceinline__ void phaseBarrier(bool cluster) {
   if (cluster) { clArrive(); clWait(); }
   else __syncthreads();
 }
 
-// The FP64 form's sums.  The corrector loop can amplify a last bit of w.r or p.q
-// a thousandfold every ten correctors (a processor-local 17 x 14 x 14 run: 1e-13
-// after 60 correctors, 2e-6 after 100; exact DIC, 23 x 16 x 19: 2e-7 after 35), so
-// they are added up in the order of kernels_pcg.cu: w.r by part, 64 lanes that
-// take a row of each level, last level first, then by parts; sum|r| and p.q by
-// storage row, 256 rows a block, then by blocks.  The CTAs own rows in another
-// order, so rows go through global memory (L2), a warp takes 32 lanes of a part or
-// 32 rows, and every CTA adds up the records.  Two cluster barriers a sum instead
-// of one: cube of 8, exact DIC, 26 -> 30 us an iteration.
-__device__ __forceinline__ double warpTree(double v) {  // in lane 0
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  return v;
+// ---- Sums -------------------------------------------------------------------------
+// The corrector loop can amplify a last bit of w.r or p.q a thousandfold every ten
+// correctors (FP64, processor-local, 17 x 14 x 14: 1e-13 after 60 correctors, 2e-6
+// after 100; exact DIC, 23 x 16 x 19: 2e-7 after 35), and in FP32 a last bit of the
+// FP64 sum can turn the rounding of alpha or beta.  So the sums are added up in the
+// order of the separate kernels, whatever form a mesh runs:
+//   exact DIC   w.r by part (kernels_pcg.cu): 64 lanes that take a row of each
+//               level, last level first, then by parts; sum|r| and p.q by storage
+//               row, 256 rows a block, then by blocks.
+//   diagonal    all three by storage row.
+//   processor-  w.r and sum|r| by part (kernels_local.cu): 64 lanes over the part's
+//   local DIC   rows in storage order, parts in groups of 32; p.q by storage row.
+// A lane adds up its rows as Acc<T> does there, from there on in FP64.
+//
+// With the exact DIC and the diagonal the CTAs own rows in another order, so the
+// rows' values go through global memory (L2), a warp takes 32 lanes of a part or 32
+// rows, and every CTA adds up the records: two cluster barriers a sum (FP64, cube of
+// 8, exact DIC: 30 us an iteration, 26 with the CTAs' own sums).  A CTA of the
+// processor-local form owns whole parts and a contiguous range of storage rows, so
+// only the records cross CTAs: one cluster barrier a sum.
+// The row kernels' grid: blocks of 256 storage rows, and rows this far apart are one
+// thread's.
+__device__ __forceinline__ int ordStride(const MeshView& mv) { return mv.rowGrid * kRowBlock; }
+// records of 32 virtual rows
+__device__ __forceinline__ int ordGroups(const MeshView& mv) {
+  return (min(mv.nC, ordStride(mv)) + 31) / 32;
 }
-// w.r of component k over 32 lanes of a part (w and r by PCG row): the lanes' rows
-// in the order of their sums, a step at a time (ResView::ordRow), the rows of
-// kOrdAhead steps read while those before them are added.
-constexpr int kOrdAhead = 8;
-__device__ __forceinline__ double ordPart(const int* rowOf, int steps, const double* w, const double* r,
-                                          int k) {
-  constexpr int B = kOrdAhead;
+// w.r of the components K0 .. K0 + NK - 1 over 32 lanes of a part (w and r by PCG row):
+// the lanes' rows in the order of their sums, a step at a time (ResView::ordRow), the
+// rows of the next steps read while those before them are added.  FP64 contracts the
+// product with the addition, as the sweep does.
+__device__ __forceinline__ void ordAdd(Acc<double>& a, double w, double r) { a.s = fma(w, r, a.s); }
+__device__ __forceinline__ void ordAdd(Acc<float>& a, float w, float r) { a.add(__fmul_rn(w, r)); }
+template <int NK, typename T>
+__device__ __forceinline__ void ordPart(const int* rowOf, int steps, const T* w, const T* r, int k0,
+                                        Acc<T> (&s)[NK]) {
+  constexpr int B = NK == 1 ? 8 : 4;
   const int* const at = rowOf + (threadIdx.x & 31);
-  double s = 0, wv[B], rv[B];
-  auto read = [&](int n0, double (&wn)[B], double (&rn)[B]) {
+  T wv[B][NK], rv[B][NK];
+  auto read = [&](int n0, T (&wn)[B][NK], T (&rn)[B][NK]) {
     int q[B];
 #pragma unroll
     for (int u = 0; u < B; ++u) q[u] = n0 + u < steps ? __ldg(at + 32 * (n0 + u)) : -1;
 #pragma unroll
-    for (int u = 0; u < B; ++u) {
-      wn[u] = q[u] >= 0 ? __ldcg(w + 3 * (size_t)q[u] + k) : 0.0;
-      rn[u] = q[u] >= 0 ? __ldcg(r + 3 * (size_t)q[u] + k) : 0.0;
-    }
+    for (int u = 0; u < B; ++u)
+#pragma unroll
+      for (int k = 0; k < NK; ++k) {
+        wn[u][k] = q[u] >= 0 ? __ldcg(w + 3 * (size_t)q[u] + k0 + k) : T(0);
+        rn[u][k] = q[u] >= 0 ? __ldcg(r + 3 * (size_t)q[u] + k0 + k) : T(0);
+      }
   };
   read(0, wv, rv);
   for (int n = 0; n < steps; n += B) {
-    double wn[B], rn[B];
+    T wn[B][NK], rn[B][NK];
     read(n + B, wn, rn);
 #pragma unroll
     for (int u = 0; u < B; ++u)
-      if (n + u < steps) s = fma(wv[u], rv[u], s);
+      if (n + u < steps)  // (a lane without a row: plus zero)
 #pragma unroll
-    for (int u = 0; u < B; ++u) { wv[u] = wn[u]; rv[u] = rn[u]; }
-  }
-  return warpTree(s);
-}
-// The sums over 32 storage rows of three values a row: value k in lane 8 k
-template <bool ABS>
-__device__ __forceinline__ double ordRows(const int* pos, const double* a, int nC, int g) {
-  const int s = 32 * g + (int)(threadIdx.x & 31);
-  const size_t q = 3 * (size_t)(s < nC ? __ldg(pos + s) : 0);
-  double v[4] = {0, 0, 0, 0};
+        for (int k = 0; k < NK; ++k) ordAdd(s[k], wv[u][k], rv[u][k]);
 #pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    const double x = s < nC ? __ldcg(a + q + k) : 0.0;
-    v[k] = ABS ? fabs(x) : x;
+    for (int u = 0; u < B; ++u)
+#pragma unroll
+      for (int k = 0; k < NK; ++k) { wv[u][k] = wn[u][k]; rv[u][k] = rn[u][k]; }
   }
-  return warpSpreadSum<double, 4>(v);
 }
-// The sum over the row records, of component k, blocks 32 h ... (and every 256th
-// after them)
-__device__ __forceinline__ double ordBlocks(const double* rec, int nC, int k, int h) {
-  const int nB = (nC + kRowBlock - 1) / kRowBlock, nG = (nC + 31) / 32;
+// N x 32 virtual rows of the row kernels, from row0 on, `apart` rows between the groups:
+// per group and component the sums of |r| (ABS) or the terms a, three values a row by
+// PCG row; component k of group n in lane 8 k of s[n].
+template <bool ABS, int N, typename T>
+__device__ __forceinline__ void ordRows(const MeshView& mv, const int* pos, const T* a, int row0, int apart,
+                                        double (&s)[N]) {
+  const bool one = mv.nC <= ordStride(mv);  // a row a lane (an addition to zero is one too)
+  double v[N][4];
+  T x[N][3];
+  const int lane = (int)threadIdx.x & 31;
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const int row = row0 + n * apart + lane;
+    const bool on = row < mv.nC && row < ordStride(mv);
+    const size_t q = on ? 3 * (size_t)__ldg(pos + row) : 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) x[n][k] = on ? __ldcg(a + q + k) : T(0);
+  }
+  if constexpr (sizeof(T) == 4)
+    if (one) {
+#pragma unroll
+      for (int n = 0; n < N; ++n)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) x[n][k] = ABS ? fabsf(x[n][k]) : x[n][k];
+      warpFloatSums<N>(x, s);
+      return;
+    }
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    v[n][3] = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) v[n][k] = toF64(ABS ? fabs(x[n][k]) : x[n][k]);
+    if (!one) {
+      Acc<T> c[3];
+#pragma unroll
+      for (int k = 0; k < 3; ++k) c[k].s = ABS ? fabs(x[n][k]) : x[n][k];
+      const int r0 = row0 + n * apart + lane;
+      for (int row = r0 + ordStride(mv); r0 < ordStride(mv) && row < mv.nC; row += ordStride(mv)) {
+        const size_t q = 3 * (size_t)__ldg(pos + row);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const T y = __ldcg(a + q + k);
+          c[k].add(ABS ? fabs(y) : y);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 3; ++k) v[n][k] = accValue(c[k]);
+    }
+  }
+  warpSpreadSums<4, N>(v, s);
+}
+// w.r and |r| of the diagonal form (FP32) over 32 virtual rows (a row a lane: the form has
+// at most kResMaxDiagRows rows): w.r of component k in lane 8 k, sum|r| in lane 8 k + 1
+__device__ __forceinline__ double ordRowsDiag(const MeshView& mv, const int* pos, const float* w, const float* r,
+                                              int g) {
+  const int lane = (int)threadIdx.x & 31, row = 32 * g + lane;
+  float x[2][3] = {{0, 0, 0}, {0, 0, 0}};
+  if (row < mv.nC) {
+    const size_t q = 3 * (size_t)__ldg(pos + row);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const float v = __ldcg(r + q + k);
+      x[0][k] = mulT(__ldcg(w + q + k), v);
+      x[1][k] = fabsf(v);
+    }
+  }
+  double s[2];
+  warpFloatSums<2>(x, s);
+  return (lane & 1) ? s[1] : s[0];
+}
+// The sum over the row records (stride values each), of value k, blocks 32 h ... (and
+// every 256th after them)
+__device__ __forceinline__ double ordBlocks(const MeshView& mv, const double* rec, int stride, int k, int h) {
+  const int nB = mv.rowGrid, nG = ordGroups(mv), b0 = 32 * h + (int)(threadIdx.x & 31);
   double v = 0;
-  for (int b = 32 * h + (int)(threadIdx.x & 31); b < nB; b += kRowBlock) {
-    double x[kRowBlock / 32], t = 0;
+  for (int b = b0; b < nB; b += kRowBlock) {
+    double x[kRowBlock / 32];
 #pragma unroll
     for (int j = 0; j < kRowBlock / 32; ++j) {
       const int g = b * (kRowBlock / 32) + j;
-      x[j] = g < nG ? __ldcg(rec + 3 * (size_t)g + k) : 0.0;
+      x[j] = g < nG ? __ldcg(rec + stride * (size_t)g + k) : 0.0;
     }
+    double t = x[0];
 #pragma unroll
-    for (int j = 0; j < kRowBlock / 32; ++j) t += x[j];
-    v += t;
+    for (int j = 1; j < kRowBlock / 32; ++j) t += x[j];
+    v = b == b0 ? t : v + t;
   }
-  return warpTree(v);
+  return warpTree(v, nB - 32 * h);
 }
-// The sum over the part records of component k
+// Row sums of NV values from their records into out[0..NV): the end of a sum, by the
+// whole CTA; complete for the threads 0 .. NV - 1.
+template <int NT, int NV>
+__device__ __forceinline__ void ordRowTotal(const MeshView& mv, const double* rec, double* blk, double* out) {
+  constexpr int W = NT / 32;
+  const int lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5;
+  const int nH = mv.rowGrid < kRowBlock ? (mv.rowGrid + 31) / 32 : W;
+  for (int q = wid; q < NV * nH; q += W) {
+    const double s = ordBlocks(mv, rec, NV, q % NV, q / NV);
+    if (lane == 0) blk[q] = s;
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < NV) {
+    double s = blk[threadIdx.x];
+    for (int h = 1; h < nH; ++h) s += blk[NV * h + (int)threadIdx.x];
+    out[threadIdx.x] = s;
+  }
+}
+// The sum over the part records of component k (reduceRecords)
 __device__ __forceinline__ double ordParts(const double* rec, int nParts, int k) {
   const int lane = (int)(threadIdx.x & 31);
   double b = 0;
@@ -206,61 +268,175 @@ __device__ __forceinline__ double ordParts(const double* rec, int nParts, int k)
     double a = 0;
     for (int p = lane + 32 * j; p < nParts; p += 256) {
       const double x = __ldcg(rec + 6 * (size_t)p + k), y = __ldcg(rec + 6 * (size_t)p + 3 + k);
-      a += x + y;
+      a = p < 256 ? x + y : a + (x + y);
     }
-    b += a;
+    b = j == 0 ? a : b + a;
   }
-  return warpTree(b);
+  return warpTree(b, nParts);
 }
-// DOTS: w.r by part and sum|r| (w, r by PCG row) into out[0..5]; else the terms w by
-// storage row into out[0..2].  The rows' values are written; out is complete for the
-// lanes 0 .. 2 of warp 0.
-template <int NT, bool DOTS>
-__device__ __forceinline__ void orderedSum(const MeshView& mv, const ResView& rv, const double* w,
-                                           const double* r, double* rec, double* blk, double* out,
-                                           int C, unsigned rank, bool cluster) {
-  constexpr int W = NT / 32;
+// Exact DIC and diagonal.  DOTS: w.r and sum|r| (w, r by PCG row) into out[0..5];
+// else the terms w into out[0..2].  The rows' values are written; out is complete for
+// the lanes 0 .. 2 of warp 0.  (blk: 3 + 48 values.)
+template <int NT, bool DOTS, bool DIAG, typename T>
+__device__ __forceinline__ void orderedSum(const MeshView& mv, const ResView& rv, const T* w, const T* r,
+                                           double* rec, double* blk, double* out, int C, unsigned rank,
+                                           bool cluster) {
+  // FP64: a component of a half part a warp (a multiply-add of a warp takes 64 cycles);
+  // FP32: the three together (9 FP64 additions for 18)
+  constexpr int W = NT / 32, NK = sizeof(T) == 8 ? 1 : 3, N = 4;
   const int lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5;
-  const int nG = (mv.nC + 31) / 32, nP = DOTS ? 6 * mv.nParts : 0;
-  double* const rows = rec + 6 * (size_t)mv.nParts + (DOTS ? 0 : 3 * (size_t)nG);
+  const int nG = ordGroups(mv), nP = DOTS && !DIAG ? 6 / NK * mv.nParts : 0;
+  double* const rows = rec + 6 * (size_t)mv.nParts + (DOTS ? 0 : 6 * (size_t)nG);
   phaseBarrier(cluster);
-  for (int q = (int)rank + C * wid; q < nP + nG; q += C * W) {
-    if (q < nP) {
-      const int task = q / 3, n0 = rv.ordStep[task];
-      const double s = ordPart(rv.ordRow + 32 * (size_t)n0, rv.ordStep[task + 1] - n0, w, r, q % 3);
+  int q = (int)rank + C * wid;
+  for (; q < nP; q += C * W) {
+    const int task = q / (3 / NK), n0 = rv.ordStep[task];
+    Acc<T> a[NK];
+    ordPart(rv.ordRow + 32 * (size_t)n0, rv.ordStep[task + 1] - n0, w, r, q % (3 / NK), a);
+    if (NK == 1) {
+      const double s = warpTree(accValue(a[0]));
       if (lane == 0) rec[q] = s;
-    } else {
-      const double s = ordRows<DOTS>(rv.pos, DOTS ? r : w, mv.nC, q - nP);
-      if ((lane & 7) == 0 && lane < 24) rows[3 * (size_t)(q - nP) + (lane >> 3)] = s;
+    }
+    if constexpr (NK == 3) {
+      const float x[1][3] = {{a[0].s, a[1].s, a[2].s}}, c[1][3] = {{a[0].c, a[1].c, a[2].c}};
+      double s[1];
+      warpFloatSums<1, true>(x, c, s);
+      if ((lane & 7) == 0 && lane < 24) rec[3 * (size_t)q + (lane >> 3)] = s[0];
+    }
+  }
+  q -= nP;
+  if constexpr (DOTS && DIAG) {
+    for (; q < nG; q += C * W) {
+      const double s = ordRowsDiag(mv, rv.pos, w, r, q);
+      if ((lane & 7) < 2 && lane < 24) rows[6 * (size_t)q + 3 * (lane & 1) + (lane >> 3)] = s;
+    }
+  } else {
+    auto put = [&](int g, double s) {
+      if ((lane & 7) == 0 && lane < 24 && g < nG) rows[3 * (size_t)g + (lane >> 3)] = s;
+    };
+    for (; q + (N - 1) * C * W < nG; q += N * C * W) {
+      double s[N];
+      ordRows<DOTS, N>(mv, rv.pos, DOTS ? r : w, 32 * q, 32 * C * W, s);
+#pragma unroll
+      for (int n = 0; n < N; ++n) put(q + n * C * W, s[n]);
+    }
+    for (; q < nG; q += 2 * C * W) {
+      double s[2];
+      ordRows<DOTS, 2>(mv, rv.pos, DOTS ? r : w, 32 * q, 32 * C * W, s);
+      put(q, s[0]);
+      put(q + C * W, s[1]);
     }
   }
   phaseBarrier(cluster);
-  const int nB = (mv.nC + kRowBlock - 1) / kRowBlock, nH = nB < kRowBlock ? (nB + 31) / 32 : W;
-  for (int q = wid; q < (DOTS ? 3 : 0) + 3 * nH; q += W) {
-    if (DOTS && q < 3) {
-      const double s = ordParts(rec, mv.nParts, q);
-      if (lane == 0) blk[24 + q] = s;
-    } else {
-      const int k = (q - (DOTS ? 3 : 0)) % 3, h = (q - (DOTS ? 3 : 0)) / 3;
-      const double s = ordBlocks(rows, mv.nC, k, h);
-      if (lane == 0) blk[3 * h + k] = s;
+  if (DOTS && DIAG) {
+    ordRowTotal<NT, 6>(mv, rows, blk, out);
+    __syncwarp();  // (threads 0 .. 5 to threads 0 .. 2)
+    return;
+  }
+  if (DOTS && wid >= W - 3) {
+    const double s = ordParts(rec, mv.nParts, wid - (W - 3));
+    if (lane == 0) blk[48 + wid - (W - 3)] = s;
+  }
+  ordRowTotal<NT, 3>(mv, rows, blk, out + (DOTS ? 3 : 0));
+  if (DOTS && threadIdx.x < 3) out[lane] = blk[48 + lane];
+}
+// Processor-local: w.r and sum|r| by part into out[0..5], from w of the CTA's rows in
+// the shared vector and r by row of the CTA.  A warp takes half of a part's lanes and one
+// of the two sums.  rec: 12 values a part ([half][w.r, sum|r|][component]); grp: 6 values
+// of each of 64 lanes over the groups.
+template <int NT, typename T>
+__device__ __forceinline__ void localDots(const MeshView& mv, const ResView& rv, unsigned uBase, const T* r,
+                                          int base, const unsigned short* pos, double* rec, double* grp, double* out, unsigned rank,
+                                          bool cluster) {
+  constexpr int W = NT / 32, B = 8;
+  const int lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5;
+  const int p0 = rv.part0[rank], p1 = rv.part0[rank + 1];
+  for (int q = 4 * p0 + wid; q < 4 * p1; q += W) {
+    const int part = q >> 2, lo = mv.partStart[part], hi = mv.partStart[part + 1];
+    const bool dots = (q & 1) == 0;
+    Acc<T> a[3];
+    for (int s0 = lo + 16 * (q & 2) + lane; s0 < hi; s0 += 64 * B) {
+      int at[B];
+#pragma unroll
+      for (int u = 0; u < B; ++u) at[u] = s0 + 64 * u < hi ? pos[s0 + 64 * u - base] : -1;
+#pragma unroll
+      for (int u = 0; u < B; ++u)
+        if (at[u] >= 0) {
+          T w[3];
+          if (dots) URow<T>::load(uBase + URow<T>::kBytes * (unsigned)at[u], w);
+#pragma unroll
+          for (int k = 0; k < 3; ++k) {
+            const T x = r[3 * (size_t)at[u] + k];
+            a[k].add(dots ? mulT(w[k], x) : fabs(x));
+          }
+        }
     }
+    const float x[1][3] = {{a[0].s, a[1].s, a[2].s}}, c[1][3] = {{a[0].c, a[1].c, a[2].c}};
+    double s[1];
+    warpFloatSums<1, true>(x, c, s);
+    if ((lane & 7) == 0 && lane < 24) rec[3 * (size_t)q + (lane >> 3)] = s[0];
+  }
+  phaseBarrier(cluster);
+  // groups of 32 parts; lane v of 64 adds up the groups v, v + 64, ... in that order
+  const int nGrp = (mv.nParts + 31) / 32;
+  for (int j = wid; j < 6 * min(nGrp, 64); j += W) {
+    const int k = j % 6;
+    double s = 0;
+    for (int g = j / 6; g < nGrp; g += 64) {
+      const int part = 32 * g + lane;
+      const double* const x = rec + 12 * (size_t)part + k;
+      const double v = warpTree(part < mv.nParts ? __ldcg(x) + __ldcg(x + 6) : 0.0, mv.nParts - 32 * g);
+      s = g < 64 ? v : s + v;
+    }
+    if (lane == 0) grp[6 * (j / 6) + k] = s;
   }
   __syncthreads();
-  if (threadIdx.x < 3) {
-    double s = 0;
-    for (int h = 0; h < nH; ++h) s += blk[3 * h + lane];
-    out[(DOTS ? 3 : 0) + lane] = s;
-    if (DOTS) out[lane] = blk[24 + lane];
+  groupTotal<W>(grp, nGrp, out);
+  __syncthreads();
+}
+// Processor-local: the terms y v by storage row into out[0..2], from y by row of the
+// CTA and v in the shared vector.  A 32-row record is the CTA's that owns its first row;
+// other(s, t): the terms t of a row s of another CTA.
+template <int NT, typename T, typename F>
+__device__ __forceinline__ void localRowSum(const MeshView& mv, unsigned uBase, const T* y, int base, int R,
+                                            const unsigned short* pos, double* rec, double* blk, double* out,
+                                            bool cluster, F other) {
+  constexpr int W = NT / 32, N = 2;
+  const int lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5;
+  const int gEnd = (base + R + 31) / 32;
+  __syncthreads();
+  for (int g0 = (base + 31) / 32 + wid; g0 < gEnd; g0 += N * W) {
+    T t[N][3];
+    double s[N];
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      const int row = 32 * (g0 + n * W) + lane;
+      t[n][0] = t[n][1] = t[n][2] = T(0);
+      if (row < base + R) {
+        const int i = pos[row - base];
+        T u[3];
+        URow<T>::load(uBase + URow<T>::kBytes * (unsigned)i, u);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) t[n][k] = mulT(y[3 * (size_t)i + k], u[k]);
+      } else if (g0 + n * W < gEnd && row < mv.nC) {
+        other(row, t[n]);
+      }
+    }
+    warpFloatSums<N>(t, s);
+#pragma unroll
+    for (int n = 0; n < N; ++n)
+      if ((lane & 7) == 0 && lane < 24 && g0 + n * W < gEnd) rec[3 * (size_t)(g0 + n * W) + (lane >> 3)] = s[n];
   }
+  phaseBarrier(cluster);
+  ordRowTotal<NT, 3>(mv, rec, blk, out);
 }
 
 // Scalars of the iteration, in shared memory, decided by warp 0.
 template <typename T>
 struct ResScalars {
   double sum[8];
-  double blk[27];  // (ordered sums)
-  double norm[3], lim[3], last[3], wArA[3], alpha[3], beta[3];
+  double blk[51];  // (the sums' records over blocks)
+  double norm[3], lim[3], last[3], wArA[3], wApA[3], alpha[3], beta[3];
   T alphaT[3], betaT[3];  // in the value type (a conversion is an FP64 operation)
   int active[3], pend[3], nIter[3];
   int any, iters;
@@ -274,16 +450,13 @@ template <typename T, int NT, int MODE, int OCC>
 __global__ void __launch_bounds__(NT, OCC)
 kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevState* st,
         double* partials) {
-  constexpr bool ORD = sizeof(T) == 8;
-  using P = Part<T>;
-  using V = typename P::V;
+  constexpr bool LOCAL = MODE == kResLocal, DIAG = MODE == kResDiag;
   p = casePcg(p, blockIdx.y, mv.nC);
   st += blockIdx.y;
   double* const ordRec = partials + (size_t)blockIdx.y * mv.caseRec + mv.ordOff;
   if (!st->pcgContinue) return;  // the same in every CTA: rank 0 writes it at the end
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ ResScalars<T> sc;
-  constexpr int W = NT / 32;
   constexpr int kRows = 2;  // rows of a thread in flight
   constexpr unsigned kU = URow<T>::kBytes;
   const int C = (int)gridDim.x, t = (int)threadIdx.x;
@@ -291,17 +464,19 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
   const unsigned rank = cluster ? clRank() : 0u;
   const int base = rv.chunk[rank], R = rv.chunk[rank + 1] - base;
   const int mr = rv.maxRows;
-  // ---- shared memory: u and its zero row | sum records | level starts |
-  //      vectors | tables
+  // ---- shared memory: u and its zero row | group sums | level starts | vectors |
+  //      tables
   unsigned char* sp = smraw;
   const unsigned uBase = (unsigned)__cvta_generic_to_shared(sp);
   sp += (size_t)kU * rv.uRows;
-  V* wrec = (V*)sp;  // warp records, then the CTAs' records of the two sums
-  sp += sizeof(V) * 6 * W;
-  V* rec0 = (V*)sp;
-  sp += sizeof(V) * 6 * kResMaxCtas;
-  V* rec1 = (V*)sp;
-  sp += sizeof(V) * 3 * kResMaxCtas;
+  // (processor-local) sums of part groups; columns, coefficients, position, diagonal and
+  // entry count of the up to 31 rows after the CTA's own that share a 32-row record with
+  // its last ones
+  double* const grp = (double*)sp;
+  uint32_t* const ext = (uint32_t*)(grp + 64 * 6);
+  float* const extT = (float*)ext;
+  unsigned short* const posS = (unsigned short*)(sp + kResGroupBytes);  // row of each storage row
+  if (rv.local) sp += kResGroupBytes + 2 * (size_t)((mr + 7) / 8 * 8);
   // (first, end) of the levels, with two empty levels before and after them
   int2* lv = (int2*)sp;
   const unsigned lva = (unsigned)__cvta_generic_to_shared(lv + 2);
@@ -377,12 +552,29 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
     sc.norm[t] = nf;
     sc.lim[t] = pcgLimit(c, ir);
     sc.last[t] = ir * nf;
-    sc.wArA[t] = st->wArA[t]; sc.alpha[t] = 0; sc.beta[t] = 0; sc.alphaT[t] = T(0); sc.betaT[t] = T(0);
+    sc.wArA[t] = st->wArA[t]; sc.wApA[t] = st->wApA[t]; sc.alpha[t] = 0; sc.beta[t] = 0; sc.alphaT[t] = T(0); sc.betaT[t] = T(0);
     sc.active[t] = st->active[t]; sc.pend[t] = 0; sc.nIter[t] = 0;
     const T z[3] = {T(0), T(0), T(0)};
     if (t == 0) URow<T>::store(uBase + kU * (rv.uRows - 1), z);
   }
   if (t == 0) { sc.any = 1; sc.iters = 0; sc.status = 0; }
+  if (LOCAL)
+    for (int i = t; i < R; i += NT) posS[i] = (unsigned short)(rv.pos[base + i] - base);
+  if (LOCAL && t < 32) {
+    const int row = (base + R) / 32 * 32 + t;  // (a storage row: the chunks are storage ranges)
+    if (row >= base + R && row < mv.nC) {
+      const int g = rv.pos[row];
+      unsigned owner = rank;
+      while (rv.chunk[owner + 1] <= g) ++owner;
+      ext[32 * 2 * kResW + t] = owner << 24 | (unsigned)(g - rv.chunk[owner]);
+      ext[32 * (2 * kResW + 2) + t] = rv.cnt[g];
+      extT[32 * (2 * kResW + 1) + t] = (float)rp.diag[g];
+      for (int e = 0; e < kResW; ++e) {
+        ext[32 * e + t] = rv.col[(size_t)e * mv.nC + g];
+        extT[32 * (kResW + e) + t] = (float)rp.val[(size_t)e * mv.nC + g];
+      }
+    }
+  }
   if (rv.place & 1)  // (in global memory the right-hand-side pass has set both)
     for (int i = t; i < R; i += NT)
 #pragma unroll
@@ -400,7 +592,6 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
     T al[3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) { pend[k] = sc.pend[k] != 0; al[k] = sc.alphaT[k]; }
-    Acc<T> ar[3], wr[3];
     for (int i0 = t; i0 < R; i0 += kRows * NT) {
       T rd[kRows], rr[kRows][3], qv[kRows][3];
 #pragma unroll
@@ -426,9 +617,11 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
               rr[h][k] = fmaT(-al[k], qv[h][k], rr[h][k]);
               rg[3 * i + k] = rr[h][k];
             }
-            if (!ORD) ar[k].add(fabs(rr[h][k]));
             w[k] = mulT(rd[h], rr[h][k]);
-            if (MODE == kResDiag) wr[k].add(mulT(w[k], rr[h][k]));
+            if (DIAG) {
+              wGlob[3 * (size_t)i + k] = w[k];
+              if (rv.place & 1) rGlob[3 * (size_t)i + k] = rr[h][k];
+            }
           }
           if (MODE == kResSingle && cluster) URow<T>::storeCluster(wBase + kU * i, w);
           else URow<T>::store(wBase + kU * i, w);
@@ -446,7 +639,7 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
       if (rank == 0) sweeps<NT, false>(sw, rv, uBase, rank, lva);
       if (cluster) phaseBarrier(true);
     }
-    if (MODE != kResDiag)
+    if (!DIAG && !LOCAL)
       for (int i = t; i < R; i += NT) {
         T w[3];
         if (MODE == kResSingle && cluster) {
@@ -455,24 +648,14 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
         } else {
           URow<T>::load(uBase + kU * i, w);
         }
-        if (ORD) {
 #pragma unroll
-          for (int k = 0; k < 3; ++k) {
-            wGlob[3 * (size_t)i + k] = w[k];
-            if (rv.place & 1) rGlob[3 * (size_t)i + k] = rg[3 * i + k];
-          }
-        } else {
-#pragma unroll
-          for (int k = 0; k < 3; ++k) wr[k].add(mulT(w[k], rg[3 * i + k]));
+        for (int k = 0; k < 3; ++k) {
+          wGlob[3 * (size_t)i + k] = w[k];
+          if (rv.place & 1) rGlob[3 * (size_t)i + k] = rg[3 * i + k];
         }
       }
-    if constexpr (ORD) {
-      orderedSum<NT, true>(mv, rv, p.w, p.r, ordRec, sc.blk, sc.sum, C, rank, cluster);
-    } else {
-      V v[8] = {P::of(wr[0]), P::of(wr[1]), P::of(wr[2]), P::of(ar[0]),
-                P::of(ar[1]), P::of(ar[2]), P::zero(), P::zero()};
-      clusterSum<T, NT, 6>(v, wrec, rec0, sc.sum, C, rank, cluster);
-    }
+    if constexpr (LOCAL) localDots<NT>(mv, rv, uBase, rg, base, posS, ordRec, grp, sc.sum, rank, cluster);
+    else orderedSum<NT, true, DIAG>(mv, rv, p.w, p.r, ordRec, sc.blk, sc.sum, C, rank, cluster);
     // the residual test of the pending iteration, beta (a lane per component)
     if (t < 32) {
       int act = 0;
@@ -547,7 +730,6 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
     if (!go) break;
     phaseBarrier(cluster);
     // q = A p, p.q
-    Acc<T> pq[3];
     for (int i0 = t; i0 < R; i0 += kRows * NT) {
       int n[kRows];
       T dg[kRows], a[kRows][kResW];
@@ -585,18 +767,36 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
 #pragma unroll
           for (int k = 0; k < 3; ++k) {
             if (act[k]) qg[3 * i + k] = y[k];
-            if (ORD) wGlob[3 * (size_t)i + k] = mulT(y[k], v[k]);
-            else pq[k].add(mulT(y[k], v[k]));
+            if (!LOCAL) wGlob[3 * (size_t)i + k] = mulT(y[k], v[k]);
           }
         }
       }
     }
-    if constexpr (ORD) {
-      orderedSum<NT, false>(mv, rv, p.w, nullptr, ordRec, sc.blk, sc.sum, C, rank, cluster);
-    } else {
-      V v[4] = {P::of(pq[0]), P::of(pq[1]), P::of(pq[2]), P::zero()};
-      clusterSum<T, NT, 3>(v, wrec, rec1, sc.sum, C, rank, cluster);
-    }
+    if constexpr (LOCAL) {
+      // a row of another CTA: its product, as there
+      auto other = [&](int, T (&term)[3]) {
+        const int e0 = t & 31;
+        T v[3], y[3], x[kResW][3];
+        const uint32_t own = ext[32 * 2 * kResW + e0];
+        URow<T>::loadCluster(mapa(uBase + kU * (own & 0xffffffu), own >> 24), v);
+        const int n = (int)ext[32 * (2 * kResW + 2) + e0];
+#pragma unroll
+        for (int e = 0; e < kResW; ++e) {
+          const uint32_t cl = ext[32 * e + e0];
+          URow<T>::loadCluster(mapa(uBase + kU * (cl & 0xffffffu), cl >> 24), x[e]);
+        }
+#pragma unroll
+        for (int k = 0; k < 3; ++k) y[k] = mulT(extT[32 * (2 * kResW + 1) + e0], v[k]);
+#pragma unroll
+        for (int e = 0; e < kResW; ++e)
+          if (e < n)
+#pragma unroll
+            for (int k = 0; k < 3; ++k) y[k] = fmaT(extT[32 * (kResW + e) + e0], x[e][k], y[k]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) term[k] = mulT(y[k], v[k]);
+      };
+      localRowSum<NT>(mv, uBase, qg, base, R, posS, ordRec + 12 * (size_t)mv.nParts, sc.blk, sc.sum, cluster, other);
+    } else orderedSum<NT, false, DIAG>(mv, rv, p.w, p.r, ordRec, sc.blk, sc.sum, C, rank, cluster);
     if (t < 32) {
       int on = 0;
       unsigned bad = 0;
@@ -604,6 +804,7 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
         sc.pend[t] = 0;
         if (sc.active[t]) {
           const double s = sc.sum[t];
+          sc.wApA[t] = s;
           if (fabs(s) < 1e-300 * sc.norm[t]) {  // checkSingularity: stop this component
             sc.active[t] = 0;
           } else {
@@ -635,7 +836,7 @@ kResPcg(MeshView mv, Controls c, ResView rv, ResPtrs<T> rp, PcgPtrs<T> p, DevSta
   if (rank == 0 && t == 0) {
     for (int k = 0; k < 3; ++k) {
       st->nIter[k] = sc.nIter[k]; st->finalRes[k] = sc.last[k] / sc.norm[k]; st->active[k] = 0;
-      st->wArA[k] = sc.wArA[k]; st->alpha[k] = sc.alpha[k]; st->beta[k] = sc.beta[k];
+      st->wArA[k] = sc.wArA[k]; st->wApA[k] = sc.wApA[k]; st->alpha[k] = sc.alpha[k]; st->beta[k] = sc.beta[k];
     }
     if (sc.status) atomicOr(&st->status, sc.status);
     st->pcgIter += sc.iters;
@@ -740,9 +941,8 @@ int resMode(bool diag, const ResView& rv) {
 
 template <typename T>
 size_t resSmemBytes(const ResView& rv, int place) {
-  const size_t W = kResThreads / 32, mr = rv.maxRows;
-  size_t b = (size_t)URow<T>::kBytes * rv.uRows +
-             sizeof(typename Part<T>::V) * (6 * W + 9 * kResMaxCtas) +
+  const size_t mr = rv.maxRows;
+  size_t b = (size_t)URow<T>::kBytes * rv.uRows + (rv.local ? kResGroupBytes + 2 * ((mr + 7) / 8 * 8) : 0) +
              sizeof(int2) * (size_t)((rv.nLev + 5) / 2 * 2);
   if (place & 1) b += sizeof(T) * 12 * mr;
   b += (rv.more ? 2 : 1) * (sizeof(typename ResSweepTab<T>::Q) + sizeof(typename ResSweepTab<T>::R)) *

@@ -5,6 +5,7 @@
 
 #include "device_common.cuh"
 #include "pcg_common.cuh"
+#include "sweep.cuh"
 
 namespace s4g {
 
@@ -28,39 +29,42 @@ __device__ __forceinline__ bool locArrive(unsigned* gcnt, int part, int nParts) 
   return atomicAdd(&gcnt[g], 1u) + 1u == (unsigned)locGroupSize(g, nParts);
 }
 
-// One warp: the record (N values) of group g (lane j holds part g*32 + j),
-// and the group's counter back to zero for the next launch.
-template <int N = 6>
+// One warp: the record (six values) of group g (lane j holds part g*32 + j), and the
+// group's counter back to zero for the next launch.
 __device__ __forceinline__ void locGroupSum(const double* rec, double* grec, unsigned* gcnt, int g,
                                             int nParts) {
   const int lane = threadIdx.x & 31;
   const int part = g * kLocGroup + lane;
   __threadfence();
-  double v[N];
+  double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
-  for (int k = 0; k < N; ++k) v[k] = part < nParts ? __ldcg(rec + 8 * (size_t)part + k) : 0.0;
-#pragma unroll
-  for (int k = 0; k < N; ++k)
-    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < N; ++k) grec[8 * (size_t)g + k] = v[k];
-    gcnt[g] = 0;
-  }
+  for (int k = 0; k < 6; ++k) v[k] = part < nParts ? __ldcg(rec + 8 * (size_t)part + k) : 0.0;
+  const double s = warpSpreadSum<8>(v);
+  if (lane % 4 == 0 && lane < 24) grec[8 * (size_t)g + lane / 4] = s;
+  if (lane == 0) gcnt[g] = 0;
 }
 
 // The last CTA: the sum of the group records in group order -- lane v of
-// 64 sums groups v, v + 64, ..., then a fixed tree.  Result in thread 0.
-template <int N>
-__device__ __forceinline__ void locGroupsTotal(const double* grec, int nGroups, double (&S)[N],
-                                               double* red) {
+// 64 sums groups v, v + 64, ..., then a fixed tree (sum64's).  Value k in lane k of
+// warp 0.  red: 6 values.
+__device__ __forceinline__ double locGroupsTotal(const double* grec, int nGroups, double* red) {
+  const int t = (int)threadIdx.x, lane = t & 31;
+  double s = 0;
+  if (t < 64) {
+    double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    for (int g = t; g < nGroups; g += 64)
 #pragma unroll
-  for (int k = 0; k < N; ++k) S[k] = 0;
-  if (threadIdx.x < 64)
-    for (int g = threadIdx.x; g < nGroups; g += 64)
-#pragma unroll
-      for (int k = 0; k < N; ++k) S[k] += __ldcg(grec + 8 * (size_t)g + k);
-  sum64<N>(S, red);
+      for (int k = 0; k < 6; ++k) {
+        const double x = __ldcg(grec + 8 * (size_t)g + k);
+        v[k] = g == t ? x : v[k] + x;
+      }
+    s = warpSpreadSum<8>(v);
+    if (t >= 32 && lane % 4 == 0 && lane < 24) red[lane / 4] = s;
+  }
+  __syncthreads();
+  if (t >= 32) return 0;
+  if (lane % 4 == 0 && lane < 24) s += red[lane / 4];
+  return __shfl_sync(0xffffffffu, s, lane < 6 ? 4 * lane : 0);
 }
 
 // End of a preconditioner launch, after the CTA's last part: thread 0
@@ -80,15 +84,8 @@ __device__ __forceinline__ void locFinish(const MeshView& mv, const Controls& c,
   __syncthreads();
   if (*sGroup >= 0 && t < 32) locGroupSum(partials, grec, gcnt, *sGroup, mv.nParts);
   if (!lastBlockDone(&st->counter[5], gridDim.x)) return;
-  double S[6];
-  locGroupsTotal<6>(grec, mv.locGroups, S, red);
+  const double mine = locGroupsTotal(grec, mv.locGroups, red);
   if (t >= 32) return;
-  double mine = 0;
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    const double v = __shfl_sync(0xffffffffu, S[k], 0);
-    if (t == k) mine = v;
-  }
   if (t == 0) {
     st->counter[5] = 0;
     st->locTicket = 0;

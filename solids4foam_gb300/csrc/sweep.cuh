@@ -27,12 +27,6 @@ __device__ __forceinline__ unsigned mapa(unsigned addr, unsigned rank) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
   return r;
 }
-__device__ __forceinline__ void stRemote(unsigned addr, double v) {
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
-}
-__device__ __forceinline__ void stRemote(unsigned addr, float2 v) {
-  asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(addr), "f"(v.x), "f"(v.y) : "memory");
-}
 
 __device__ __forceinline__ float fmaT(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fmaT(double a, double b, double c) { return __fma_rn(a, b, c); }
@@ -359,71 +353,138 @@ __device__ __noinline__ void resSweep(const typename E::Tab tb, const typename E
 }
 
 // ---- sums ------------------------------------------------------------------------
-// A thread's partial sum and its addition: FP64, or (FP32 values) the
-// compensated pair s + c, added with the error of s (two-sum) kept in c.
-template <typename T> struct Part;
-template <> struct Part<double> {
-  using V = double;
-  static __device__ __forceinline__ V of(const Acc<double>& a) { return a.s; }
-  static __device__ __forceinline__ V zero() { return 0.0; }
-  static __device__ __forceinline__ V ldcg(const V* a) { return __ldcg(a); }
-  static __device__ __forceinline__ V add(V a, V b) { return a + b; }
-  static __device__ __forceinline__ V shfl(V a, int o) { return __shfl_xor_sync(0xffffffffu, a, o); }
-  static __device__ __forceinline__ double value(V a) { return a; }
-};
-template <> struct Part<float> {
-  using V = float2;
-  static __device__ __forceinline__ V of(const Acc<float>& a) { return make_float2(a.s, a.c); }
-  static __device__ __forceinline__ V zero() { return make_float2(0.0f, 0.0f); }
-  static __device__ __forceinline__ V ldcg(const V* a) { return __ldcg(a); }
-  static __device__ __forceinline__ V add(V a, V b) {
-    const float s = __fadd_rn(a.x, b.x), z = __fsub_rn(s, a.x);
-    const float e = __fadd_rn(__fsub_rn(a.x, __fsub_rn(s, z)), __fsub_rn(b.x, z));
-    return make_float2(s, __fadd_rn(__fadd_rn(a.y, b.y), e));
-  }
-  static __device__ __forceinline__ V shfl(V a, int o) {
-    return make_float2(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o));
-  }
-  static __device__ __forceinline__ double value(V a) { return (double)a.x + (double)a.y; }
-};
-
 // Sum of M values (a power of two) over a warp.  A lane adds M/2, M/4, ..., 1
 // values while the values are spread over the lanes, then one value per
 // remaining step: 9 (M = 8) or 6 (M = 4) additions per lane instead of 5 M --
 // an FP64 addition of a warp takes ~19 cycles of the SM's FP64 unit.  Value k
-// ends in the lanes k * 32 / M + (0 .. 32 / M - 1).
-template <typename T, int M>
-__device__ __forceinline__ typename Part<T>::V warpSpreadSum(typename Part<T>::V (&v)[M]) {
+// ends in the lanes k * 32 / M + (0 .. 32 / M - 1).  The pairs of lanes that are
+// added, and their order, are blockSum's and sum64's (16, 8, 4, 2, 1 apart).
+// N such sums side by side: their chains (some 130 cycles a step) overlap.
+template <int M, int N>
+__device__ __forceinline__ void warpSpreadSums(double (&v)[N][M], double (&s)[N]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int h = M / 2, o = 16; h >= 1; h /= 2, o /= 2) {
     const bool up = (lane & o) != 0;
 #pragma unroll
-    for (int k = 0; k < h; ++k) {
-      const typename Part<T>::V give = up ? v[k] : v[k + h];
-      const typename Part<T>::V keep = up ? v[k + h] : v[k];
-      v[k] = Part<T>::add(keep, Part<T>::shfl(give, o));
+    for (int n = 0; n < N; ++n)
+#pragma unroll
+      for (int k = 0; k < h; ++k) {
+        const double give = up ? v[n][k] : v[n][k + h];
+        const double keep = up ? v[n][k + h] : v[n][k];
+        v[n][k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+      }
+  }
+#pragma unroll
+  for (int n = 0; n < N; ++n) s[n] = v[n][0];
+#pragma unroll
+  for (int o = 32 / M / 2; o >= 1; o /= 2)
+#pragma unroll
+    for (int n = 0; n < N; ++n) s[n] += __shfl_xor_sync(0xffffffffu, s[n], o);
+}
+template <int M>
+__device__ __forceinline__ double warpSpreadSum(double (&v)[M]) {
+  double w[1][M], s[1];
+#pragma unroll
+  for (int k = 0; k < M; ++k) w[0][k] = v[k];
+  warpSpreadSums<M, 1>(w, s);
+  return s[0];
+}
+// warpSpreadSums<4, N> of N x 3 floats x (and their compensations c, added to them first:
+// PAIR), component k in the lanes 8 k ...; the same bits.  Where every float is a multiple
+// of 2^-46 of the largest one's power of two, the FP64 additions of that sum are exact,
+// whatever their order, and integer sums of the warp give it: some 70 instructions and 9
+// warp reductions instead of 6 FP64 additions, which take 114 cycles of the SM's FP64 unit
+// and 660 one after the other.  Else the additions are done.
+template <int N, bool PAIR>
+__device__ __forceinline__ void warpFloatSums(const float (&x)[N][3], const float (&c)[N][3], double (&s)[N]) {
+  constexpr int L = 23;  // bits below those of the largest: 24 + 23 + 5 < 53
+  const int comp = (int)(threadIdx.x & 31) >> 3;
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    int top[3], hi[3], lo[3];
+    bool exact = true;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      unsigned a = __float_as_uint(x[n][k]) & 0x7fffffffu;
+      if (PAIR) a = max(a, __float_as_uint(c[n][k]) & 0x7fffffffu);
+      top[k] = max(1, (int)(__reduce_max_sync(0xffffffffu, a) >> 23));
+      exact = exact && top[k] < 255;
+      hi[k] = lo[k] = 0;
+      auto add = [&](float f) {
+        const unsigned b = __float_as_uint(f), q = b & 0x7fffffffu;
+        const int e = max(1, (int)(q >> 23)), sh = top[k] - e;
+        const unsigned m = (q & 0x7fffffu) | (q >= 0x00800000u ? 0x800000u : 0u);
+        // m 2^L >> sh in two parts of L bits and the rest
+        const unsigned h = sh < 32 ? m >> sh : 0u;
+        unsigned l;
+        if (sh <= L) {
+          l = (m << (L - sh)) & ((1u << L) - 1);
+        } else {
+          const int d = sh - L;
+          l = d < 32 ? m >> d : 0u;
+          exact = exact && (d < 32 ? l << d : 0u) == m;
+        }
+        hi[k] += (b >> 31) ? -(int)h : (int)h;
+        lo[k] += (b >> 31) ? -(int)l : (int)l;
+      };
+      add(x[n][k]);
+      if (PAIR) add(c[n][k]);
+    }
+    if (__all_sync(0xffffffffu, exact)) {
+      long long sum = 0;
+      int e = 0;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        const long long t = ((long long)__reduce_add_sync(0xffffffffu, hi[k]) << L) +
+                            (long long)__reduce_add_sync(0xffffffffu, lo[k]);
+        if (comp == k) { sum = t; e = top[k]; }
+      }
+      // sum 2^(e - 150 - L)
+      const unsigned long long u = (unsigned long long)(sum < 0 ? -sum : sum);
+      const int z = __clzll((long long)u);
+      const unsigned long long m = (u << (z & 63)) >> 11 & 0xfffffffffffffull;
+      const unsigned long long ex = (unsigned long long)(1023 + 63 - z + e - 150 - L);
+      const unsigned long long r = u ? ex << 52 | m | (sum < 0 ? 1ull << 63 : 0ull) : 0ull;
+      s[n] = __longlong_as_double((long long)r);
+    } else {
+      double v[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        v[k] = toF64(x[n][k]);
+        if (PAIR) v[k] += toF64(c[n][k]);
+      }
+      s[n] = warpSpreadSum<4>(v);
     }
   }
-  typename Part<T>::V s = v[0];
-#pragma unroll
-  for (int o = 32 / M / 2; o >= 1; o /= 2) s = Part<T>::add(s, Part<T>::shfl(s, o));
-  return s;
+}
+template <int N>
+__device__ __forceinline__ void warpFloatSums(const float (&x)[N][3], double (&s)[N]) {
+  warpFloatSums<N, false>(x, x, s);
 }
 
-// Sum of the records rec[0..count) of N <= M values (stride N) by one warp:
-// lane = value * G + g sums records g, g + G, ..., then a fixed tree.  The sum
-// of value k is returned in the lanes k * G + (0 .. G-1).
-template <typename T, int N, int M>
-__device__ __forceinline__ typename Part<T>::V warpRecords(const typename Part<T>::V* rec, int count) {
-  constexpr int G = 32 / M;
-  const int lane = threadIdx.x & 31, k = lane / G, g = lane % G;
-  typename Part<T>::V a = Part<T>::zero();
-  if (k < N)
-    for (int j = g; j < count; j += G) a = Part<T>::add(a, rec[j * N + k]);
+// Sum over the lanes below n (the others hold zero), in lane 0: blockSum's tree without
+// its steps that add zeros.
+__device__ __forceinline__ double warpTree(double v, int n = 32) {
 #pragma unroll
-  for (int o = G / 2; o >= 1; o /= 2) a = Part<T>::add(a, Part<T>::shfl(a, o));
-  return a;
+  for (int o = 16; o > 0; o >>= 1) {
+    const double x = __shfl_down_sync(0xffffffffu, v, o);
+    if (o < n) v += x;
+  }
+  return v;
+}
+
+// locGroupsTotal's sums of six values over the part groups into out[0..5], by W warps:
+// grp holds them for 64 lanes (lane v: groups v, v + 64, ...).  The caller synchronises
+// the CTA before and after it.
+template <int W>
+__device__ __forceinline__ void groupTotal(const double* grp, int nGrp, double* out) {
+  const int lane = (int)threadIdx.x & 31, wid = (int)threadIdx.x >> 5;
+  for (int k = wid; k < 6; k += W) {
+    double s = warpTree(lane < nGrp ? grp[6 * lane + k] : 0.0, nGrp);
+    if (nGrp > 32) s += warpTree(32 + lane < nGrp ? grp[6 * (32 + lane) + k] : 0.0, nGrp - 32);
+    if (lane == 0) out[k] = s;
+  }
 }
 
 }  // namespace s4g

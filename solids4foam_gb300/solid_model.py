@@ -134,12 +134,14 @@ class SolidModel:
                  "linearGeometryTotalDisplacement", solver: dict | None = None,
                  outer: dict | None = None, precision: str = "FP64", renumber: str = "tiled",
                  part_size: int = 512, ls_boundary_delta: int = 0, dic_subdomains: bool = False,
-                 autotune: bool = True, empty_direction: int = 0, parts=None):
+                 autotune: bool = True, empty_direction: int = 0, parts=None,
+                 general_pcg: bool = False):
         """empty_direction: 1, 2 or 3 for a 2-D case whose empty patches'
         faces the mesh leaves out (x, y or z empty; plane strain); 0: 3-D.
         parts: the caller's decomposition into DIC subdomains (cell ->
         subdomain id, decomposePar's cellDecomposition); implies
-        renumber="none" and dic_subdomains=True.  outer may hold
+        renumber="none" and dic_subdomains=True.  general_pcg: the PCG's
+        general kernels on any mesh (the same results).  outer may hold
         fieldRelaxation (fvSolution relaxationFactors fields factor) and
         relaxationMethod ("fixed" or "Aitken")."""
         self.time_steps = None
@@ -157,7 +159,8 @@ class SolidModel:
             keep.append(parts)
             renumber, dic_subdomains = "none", True
         opts = _lib.MeshOpts(RENUMBER[renumber], part_size, ls_boundary_delta,
-                             1 if dic_subdomains else 0, 0 if autotune else 1, empty_direction,
+                             1 if dic_subdomains else 0,
+                             2 if general_pcg else 0 if autotune else 1, empty_direction,
                              None if parts is None else parts.ctypes.data)
         h = ct.c_void_p()
         _lib.check(self.L.s4g_mesh_upload(ctx.h, ct.byref(d), ct.byref(opts), ct.byref(h)),
@@ -309,6 +312,12 @@ class SolidModel:
         G = np.zeros((self.n_cells, 9))
         _lib.check(self.L.s4g_get_gradD(self.h, G.ctypes.data), "s4g_get_gradD")
         return G
+
+    def pcg_scalars(self):
+        """w.r, p.Ap, alpha and beta ([4][3]) of the last corrector's PCG."""
+        out = np.zeros((4, 3))
+        _lib.check(self.L.s4g_get_pcg_scalars(self.h, out.ctypes.data), "s4g_get_pcg_scalars")
+        return out
 
     def set_points(self, points, point_cell_start, point_cells):
         """The mesh's points and the cells of each point (s4g_point_cells)
