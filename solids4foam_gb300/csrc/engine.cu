@@ -838,7 +838,7 @@ struct Engine {
     // with others at the same time: room for a second CTA on the SM, if that
     // leaves the sweep tables in shared memory
     q.placeMany = resPlacement<T>(rv, limit / 2 - 1024);
-    if (!(q.placeMany & 2)) q.placeMany = rv.place;
+    if (q.placeMany < 0 || !(q.placeMany & 2)) q.placeMany = rv.place;
     int clusters = 0;
     const cudaError_t e = resPrepare<T>(rv, &clusters);
     if (e != cudaSuccess || clusters < 1) {
