@@ -685,7 +685,8 @@ struct Engine {
     cudaStream_t s = ctx->stream;
     if (!q.tried) {
       q.tried = true;
-      S4G_TRY(planResident<T>(q));
+      S4G_TRY(planResident<T>(q, true));
+      if (!q.ok) S4G_TRY(planResident<T>(q, false));
     }
     const int pre = lin.preconditioner == S4G_PRECOND_DIC ? 0 : 1;
     if (!q.ok || (q.valid && q.precond == pre)) return S4G_OK;
@@ -697,9 +698,12 @@ struct Engine {
     return S4G_OK;
   }
 
+  // one: exact DIC inside one CTA where its rows fit (they may, and the ring of its
+  // tables not: it is sized by the widest level); else across the cluster.
   template <typename T>
-  s4g_status planResident(Resident<T>& q) {
+  s4g_status planResident(Resident<T>& q, bool one) {
     const int nC = hp.nC;
+    if (!one && (mv.subdomains || !q.rv.single)) return S4G_OK;  // (planned so already)
     for (int r = 0; r < nC; ++r)
       if (hp.rowptr[r + 1] - hp.rowptr[r] > kResW) return S4G_OK;
     int maxSmem = 0;
@@ -716,7 +720,7 @@ struct Engine {
     // (a level costs the CTA's barrier, not the cluster's).  Rows per CTA: a
     // level's cost hardly depends on them, the other phases' time does, the sums'
     // above all (13 x 11 x 10 cells in blocks of 8: 91 ms with 1024 rows, 82 with 256).
-    rv.single = !rv.local && resSmemBytes<T>(rv, 0) <= limit;
+    rv.single = one && !rv.local && resSmemBytes<T>(rv, 0) <= limit;
     const int rows = 256;
     rv.C = std::max(1, std::min({kResMaxCtas, (nC + rows - 1) / rows,
                                  rv.local ? hp.nParts : kResMaxCtas}));

@@ -34,3 +34,20 @@ def test_batch_of_exact_dic_meshes_equals_the_single_solves(ctx, precision):
         assert np.array_equal(D, D1) and np.array_equal(sig, s1)
         assert perf["total_lin_iters"] == p1["total_lin_iters"] > 30
         m.close()
+
+
+@pytest.mark.parametrize("n", [20, 21, 22, 23])
+def test_exact_dic_runs_resident_where_one_cta_is_too_small(ctx, n):
+    """FP32: up to 20^3 the rows and the ring of the sweep tables fit one CTA, from 23^3
+    on not even the rows; 21^3 and 22^3 lie between and run across the cluster: one launch
+    per corrector (total_lin_iters counts three components, a general iteration is five
+    launches), with the general kernels' results."""
+    m = _model(ctx, n, "FP32_REFINE", "none")
+    D, sig, perf = m.evolve()
+    assert 3 * perf["kernel_launches"] < 2 * perf["total_lin_iters"]
+    m.close()
+    m = _model(ctx, n, "FP32_REFINE", "none", general_pcg=True)
+    D1, s1, p1 = m.evolve()
+    assert 3 * p1["kernel_launches"] > 2 * p1["total_lin_iters"] > 0
+    assert np.array_equal(D, D1) and np.array_equal(sig, s1)
+    m.close()
