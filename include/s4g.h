@@ -413,6 +413,13 @@ s4g_status s4g_get_pointD(s4g_mesh* mesh, double* pointD_out);
  * grad(D)_ij = dD_j/dx_i (the reference's gradD field). */
 s4g_status s4g_get_gradD(s4g_mesh* mesh, double* gradD_out);
 
+/* Limits of a mesh, by which the error paths can be tested.  value 0: the default. */
+typedef enum s4g_limit {
+  S4G_LIMIT_SWEEP_POLLS = 0   /* polls of the exact DIC sweeps' waits
+                                 (s4g_ctx_opts.spin_limit) */
+} s4g_limit;
+s4g_status s4g_mesh_set_limit(s4g_mesh* mesh, s4g_limit which, long long value);
+
 /* Scalars of the PCG in the last solve's last corrector (its first load case),
  * per component: out [4][3] = w.r, p.Ap, alpha, beta.  For diagnosis and tests:
  * every form of the PCG that a mesh may run gives the same bits. */

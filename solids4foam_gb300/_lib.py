@@ -20,6 +20,7 @@ LINEAR_ELASTIC, NEO_HOOKEAN = 0, 1
 FIXED_DISPLACEMENT, SOLID_TRACTION = 0, 1
 PRECOND_DIC, PRECOND_DIAGONAL = 0, 1
 FP64, FP32_REFINE = 0, 1
+LIMIT_SWEEP_POLLS = 0
 LIN_GEOM_TOTAL_DISP, NONLIN_GEOM_TOTAL_LAG, NONLIN_GEOM_TOTAL_LAG_TOTAL_DISP = 0, 1, 2
 
 
@@ -146,6 +147,7 @@ _SIGS = {
                                   ct.POINTER(Perf)]),
     "s4g_state_reset": (ct.c_int, [ct.c_void_p]),
     "s4g_get_gradD": (ct.c_int, [ct.c_void_p, ct.c_void_p]),
+    "s4g_mesh_set_limit": (ct.c_int, [ct.c_void_p, ct.c_int, ct.c_longlong]),
     "s4g_get_pcg_scalars": (ct.c_int, [ct.c_void_p, ct.c_void_p]),
     "s4g_solve_batch": (ct.c_int, [ct.c_void_p, ct.c_int, ct.c_void_p, ct.c_void_p, ct.c_void_p]),
     "s4g_mesh_set_points": (ct.c_int, [ct.c_void_p, ct.c_int, ct.c_void_p, ct.c_void_p,

@@ -1463,7 +1463,7 @@ struct Engine {
   //                       (or the cluster-resident PCG in one launch)
   //                     post-solve pass; cond(correctors)
   // Each loop is also bounded on the device (nCorrectors + 4 correctors,
-  // maxIter + 4 PCG iterations per corrector).
+  // maxIter + 4 PCG iterations per corrector, rounded up to whole passes).
   template <typename T>
   bool buildLoopGraph(cudaGraph_t g, const Controls& c, int tl, const PcgPtrs<T>& p, int grid) {
     cudaStream_t s = ctx->stream;
@@ -1474,7 +1474,8 @@ struct Engine {
     if (!runsResident<T>() && !runsPartLoop<T>() &&
         cudaGraphConditionalHandleCreate(&hPcg, g, 0, cudaGraphCondAssignDefault) != cudaSuccess)
       return false;
-    const unsigned outerLimit = (unsigned)c.nCorr + 4, pcgLimit = (unsigned)c.maxIter + 4;
+    const unsigned outerLimit = (unsigned)c.nCorr + 4;
+    const unsigned pcgLimit = ((unsigned)c.maxIter + 4 + kPcgUnroll - 1) / kPcgUnroll;  // passes
     cudaGraph_t outerBody = nullptr, pcgBody = nullptr, ended = nullptr;
     bool ok;
     if (cudaStreamBeginCaptureToGraph(s, g, nullptr, nullptr, 0, mode) != cudaSuccess) return false;
@@ -2025,6 +2026,14 @@ struct Engine {
     return S4G_OK;
   }
 
+  s4g_status setLimit(int which, long long value) {
+    if (value < 0 || value > INT_MAX) return setErr(S4G_BAD_ARG, "a limit must be >= 0");
+    if (which == S4G_LIMIT_SWEEP_POLLS) mv.spinLimit = value ? (int)value : ctx->spinLimit;
+    else return setErr(S4G_BAD_ARG, "unknown limit");
+    ++generation;  // captured graphs hold the old view of the mesh
+    return S4G_OK;
+  }
+
   s4g_status getPcgScalars(double* out) {
     if (lastModel < 0) return setErr(S4G_BAD_ARG, "no solve has run");
     if (!out) return setErr(S4G_BAD_ARG, "null output");
@@ -2289,6 +2298,11 @@ s4g_status s4g_state_reset(s4g_mesh* mesh) {
 s4g_status s4g_get_gradD(s4g_mesh* mesh, double* gradD_out) {
   if (!mesh || !gradD_out) return setErr(S4G_BAD_ARG, "null argument");
   return mesh->e.getGradD(gradD_out);
+}
+
+s4g_status s4g_mesh_set_limit(s4g_mesh* mesh, s4g_limit which, long long value) {
+  if (!mesh) return setErr(S4G_BAD_ARG, "null argument");
+  return mesh->e.setLimit((int)which, value);
 }
 
 s4g_status s4g_get_pcg_scalars(s4g_mesh* mesh, double* out) {

@@ -519,7 +519,7 @@ kUpdate(MeshView mv, Controls c, PcgPtrs<T> p, DevState* st, double* partials) {
   const unsigned any = __ballot_sync(0xffffffffu, act1 != 0);
   if (l == 0) {
     st->pcgIter += 1;
-    st->pcgContinue = any != 0;
+    st->pcgContinue = any != 0 && !pcgFailed(st);
   }
 }
 

@@ -70,6 +70,12 @@ __device__ __forceinline__ bool pcgConverged(double s, double norm, double lim) 
   return s / norm < lim;
 }
 
+// A wait that gave up or a value that is not finite ends the loop with its iteration (the
+// loop's own condition looks only once in kPcgUnroll of them).
+__device__ __forceinline__ bool pcgFailed(const DevState* st) {
+  return (*(const volatile unsigned*)&st->status & (kErrTimeout | kErrNaN)) != 0;
+}
+
 // End of a processor-local preconditioner launch, by warp 0 of its last CTA:
 // S = w.r of the components, then sum|r| (S[k] in lane k and k + 3 for lanes
 // 0 .. 5 of `mine`).  Per component the residual test of the pending iteration,
@@ -103,7 +109,7 @@ __device__ __forceinline__ void pcgDecideBeta(const Controls& c, DevState* st, d
   const unsigned any = __ballot_sync(0xffffffffu, act != 0);
   if (l == 0) {
     if (anyPend) st->pcgIter += 1;
-    st->pcgContinue = any != 0;
+    st->pcgContinue = any != 0 && !pcgFailed(st);
   }
 }
 

@@ -313,6 +313,11 @@ class SolidModel:
         _lib.check(self.L.s4g_get_gradD(self.h, G.ctypes.data), "s4g_get_gradD")
         return G
 
+    def set_limit(self, which: int, value: int):
+        """A limit of the mesh (_lib.LIMIT_*; 0: the default), for tests of the
+        error paths."""
+        _lib.check(self.L.s4g_mesh_set_limit(self.h, which, value), "s4g_mesh_set_limit")
+
     def pcg_scalars(self):
         """w.r, p.Ap, alpha and beta ([4][3]) of the last corrector's PCG."""
         out = np.zeros((4, 3))

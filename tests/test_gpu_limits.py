@@ -1,0 +1,46 @@
+"""Error paths of the solves, made on the host through a mesh's limits: waits that run
+out, tables that cannot be allocated."""
+import ctypes as ct
+
+import numpy as np
+import pytest
+
+import solids4foam_gb300 as sg
+from solids4foam_gb300 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(ctx, shape, precision, **kw):
+    m = sg.box_mesh(*shape, 1.0, 0.9, 0.8, 0.2, 4)
+    top = np.tile([1e5, 2e5, -3e5], (int(m["patch_size"][5]), 1))
+    return sg.SolidModel(ctx, m, dict(type="linearElastic", E=70e9, nu=0.3),
+                         {"zmin": ("fixedDisplacement", None, None),
+                          "zmax": ("solidTraction", top, None)},
+                         outer=dict(nCorrectors=3), precision=precision, **kw)
+
+
+def _solve(model):
+    """Status, displacement and perf of a solve, whatever its status."""
+    n = model.n_cells
+    D, sig, perf = np.zeros((n, 3)), np.zeros((n, 6)), _lib.Perf()
+    st = model.L.s4g_solve(model.h, _lib.LIN_GEOM_TOTAL_DISP, 1, D.ctypes.data, sig.ctypes.data,
+                           ct.byref(perf))
+    return st, D, perf.as_dict()
+
+
+@pytest.mark.parametrize("precision", ["FP64", "FP32_REFINE"])
+def test_a_timed_out_sweep_ends_the_loop_with_its_iteration(ctx, precision):
+    """The device loop runs several PCG iterations a pass; the iteration whose waits gave
+    up is its last (one iteration of three components)."""
+    model = _model(ctx, (16, 16, 16), precision, part_size=64, general_pcg=True)
+    st, D, p = _solve(model)
+    assert st == _lib.NOT_CONVERGED and p["device_loop"] == 1
+    model.set_limit(_lib.LIMIT_SWEEP_POLLS, 1)
+    st, _, q = _solve(model)
+    assert st == _lib.TIMEOUT and q["total_lin_iters"] <= 3
+    model.set_limit(_lib.LIMIT_SWEEP_POLLS, 0)
+    st, D2, r = _solve(model)
+    assert st == _lib.NOT_CONVERGED and r["total_lin_iters"] == p["total_lin_iters"]
+    assert np.array_equal(D, D2)
+    model.close()
