@@ -75,7 +75,10 @@ typedef struct s4g_ctx_opts {
                    wait for the parts they depend on) makes before it gives
                    up: the kernel then sets an error bit, returns, and the
                    call reports S4G_TIMEOUT with the context still usable.
-                   0: the default, 4,194,304 (seconds of waiting) */
+                   0: the default, 4,194,304 (seconds of waiting).  A smaller
+                   value does not bound the waits between the CTAs of a
+                   one-launch PCG loop (processor-local DIC, FP32), which make
+                   at least the default's polls: S4G_LIMIT_PACKET_POLLS */
 } s4g_ctx_opts;
 
 /* Kernel kinds of the per-kernel timers. */
@@ -415,8 +418,10 @@ s4g_status s4g_get_gradD(s4g_mesh* mesh, double* gradD_out);
 
 /* Limits of a mesh, by which the error paths can be tested.  value 0: the default. */
 typedef enum s4g_limit {
-  S4G_LIMIT_SWEEP_POLLS = 0   /* polls of the exact DIC sweeps' waits
+  S4G_LIMIT_SWEEP_POLLS = 0,  /* polls of the exact DIC sweeps' waits
                                  (s4g_ctx_opts.spin_limit) */
+  S4G_LIMIT_PACKET_POLLS = 1  /* polls of a wait between the CTAs of a one-launch PCG
+                                 loop (default 4,194,304, or spin_limit if larger) */
 } s4g_limit;
 s4g_status s4g_mesh_set_limit(s4g_mesh* mesh, s4g_limit which, long long value);
 

@@ -43,6 +43,7 @@ struct MeshView {
   int fvBlock, fvGrid, fvFaceGrid;
   const int* bcell;    // cell of each boundary face
   int spinLimit;       // polls of a bounded wait before it gives up (kErrTimeout)
+  int packetLimit;     // the same of the waits between the CTAs of kPartLoop
   // processor-local DIC tables (see HostPrep)
   const int* locEntStart; const int* locSrc; const uint16_t* locIdx;
   const int* locMetaStart; const uint32_t* locMeta;

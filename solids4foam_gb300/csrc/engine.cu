@@ -184,7 +184,8 @@ struct Engine {
   Parts<double> parts64;
   Parts<float> parts32;
   LoopPtrs lp;
-  size_t lpCount = 0;  // packets of lp
+  size_t lpCount = 0;    // packets of lp
+  bool lpStale = false;  // a launch that used them gave up
   int *dHaloCnt = nullptr, *dHalo = nullptr, haloCap = 0;
   unsigned short* dSlot = nullptr;
   template <typename T>
@@ -346,6 +347,7 @@ struct Engine {
     mv.fvGrid = std::max(1, std::min((nC + mv.fvBlock - 1) / mv.fvBlock, ctx->numSMs * kRowBlocksPerSM));
     mv.fvFaceGrid = ctx->numSMs * kRowBlocksPerSM * (kRowBlock / mv.fvBlock);
     mv.spinLimit = ctx->spinLimit;
+    mv.packetLimit = std::max(ctx->spinLimit, kSpinLimit);
     mv.rowptr = dRow; mv.col = dCol; mv.fidx = dFidx; mv.fown = dFown; mv.fnei = dFnei;
     mv.fS = geo.fS; mv.fmagS = geo.fmagS; mv.fw = geo.fw; mv.fdelta = geo.fdelta;
     mv.C = geo.C; mv.invDd = geo.invDd;
@@ -904,8 +906,8 @@ struct Engine {
       S4G_TRY(planParts<T>(q));
     }
     // packets of a launch whose waits gave up may carry the tags of the next one
-    if (q.loop && (hState->status & kErrTimeout))
-      S4G_CUDA(cudaMemsetAsync(lp.w, 0, sizeof(uint4) * lpCount, ctx->stream));
+    if (lpStale) S4G_CUDA(cudaMemsetAsync(lp.w, 0, sizeof(uint4) * lpCount, ctx->stream));
+    lpStale = false;
     if (!q.ok || q.valid) return S4G_OK;
     S4G_CUDA(launchPartTables<T>(mv, q.pv, dVal, dRDa, q.pt, ctx->stream));
     launches++;
@@ -1102,6 +1104,7 @@ struct Engine {
   s4g_status readState(bool inPcg = false) {
     S4G_CUDA(cudaMemcpyAsync(hState, dState, sizeof(DevState) * nRun, cudaMemcpyDeviceToHost, ctx->stream));
     S4G_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (lp.w && (hState->status & kErrTimeout)) lpStale = true;
     if (ctx->profile) {
       int keep = 1 << 30;
       if (inPcg) {
@@ -2029,6 +2032,8 @@ struct Engine {
   s4g_status setLimit(int which, long long value) {
     if (value < 0 || value > INT_MAX) return setErr(S4G_BAD_ARG, "a limit must be >= 0");
     if (which == S4G_LIMIT_SWEEP_POLLS) mv.spinLimit = value ? (int)value : ctx->spinLimit;
+    else if (which == S4G_LIMIT_PACKET_POLLS)
+      mv.packetLimit = value ? (int)value : std::max(ctx->spinLimit, kSpinLimit);
     else return setErr(S4G_BAD_ARG, "unknown limit");
     ++generation;  // captured graphs hold the old view of the mesh
     return S4G_OK;

@@ -664,8 +664,7 @@ kPartLoop(MeshView mv, Controls c, PartView pv, PartPtrs<float> pt, LoopPtrs lp,
   const int pLo = mv.partStart[part], nR = mv.partStart[part + 1] - pLo, nH = pv.haloCnt[part];
   const int l0 = mv.lvlOff[part], nL = mv.lvlOff[part + 1] - l0;
   const bool lead = part == 0;
-  // (a shorter limit is for the waits between parts of the exact DIC's sweeps)
-  const int limit = mv.spinLimit > kSpinLimit ? mv.spinLimit : kSpinLimit;
+  const int limit = mv.packetLimit;
   // the thread's rows: i0, i0 + 64, ..., nMine of them
   const int half = (nR + 127) / 128, i0 = (t & 63) + (t >> 6) * 64 * half;
   const int nMine = i0 < nR ? min(half, (nR - i0 + 63) / 64) : 0;

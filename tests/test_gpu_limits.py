@@ -7,6 +7,7 @@ import pytest
 
 import solids4foam_gb300 as sg
 from solids4foam_gb300 import _lib
+from solids4foam_gb300.cases import block_parts
 
 pytestmark = pytest.mark.gpu
 
@@ -43,4 +44,25 @@ def test_a_timed_out_sweep_ends_the_loop_with_its_iteration(ctx, precision):
     st, D2, r = _solve(model)
     assert st == _lib.NOT_CONVERGED and r["total_lin_iters"] == p["total_lin_iters"]
     assert np.array_equal(D, D2)
+    model.close()
+
+
+def test_a_timed_out_part_loop_leaves_the_mesh_usable(ctx):
+    """The one-launch part loop with a limit of one poll gives up (its CTAs return by
+    themselves) and reports S4G_TIMEOUT; the packets it left behind do not reach the
+    next launch, which has the first solve's bits."""
+    model = _model(ctx, (28, 27, 26), "FP32_REFINE", parts=block_parts(28, 27, 26, 8))
+    st, D, p = _solve(model)
+    assert st == _lib.NOT_CONVERGED
+    assert 3 * p["kernel_launches"] < 2 * p["total_lin_iters"]  # one launch per corrector
+    for again in range(5):
+        model.set_limit(_lib.LIMIT_PACKET_POLLS, 1)
+        st, _, _ = _solve(model)
+        assert st == _lib.TIMEOUT
+        model.set_limit(_lib.LIMIT_PACKET_POLLS, 0)
+        if again % 2:  # (a new matrix before the next solve)
+            model.set_law(dict(type="linearElastic", E=70e9, nu=0.3))
+        st, D2, q = _solve(model)
+        assert st == _lib.NOT_CONVERGED and q["total_lin_iters"] == p["total_lin_iters"]
+        assert np.array_equal(D, D2)
     model.close()
