@@ -420,8 +420,12 @@ s4g_status s4g_get_gradD(s4g_mesh* mesh, double* gradD_out);
 typedef enum s4g_limit {
   S4G_LIMIT_SWEEP_POLLS = 0,  /* polls of the exact DIC sweeps' waits
                                  (s4g_ctx_opts.spin_limit) */
-  S4G_LIMIT_PACKET_POLLS = 1  /* polls of a wait between the CTAs of a one-launch PCG
+  S4G_LIMIT_PACKET_POLLS = 1, /* polls of a wait between the CTAs of a one-launch PCG
                                  loop (default 4,194,304, or spin_limit if larger) */
+  S4G_LIMIT_TABLE_BYTES = 2   /* device bytes that the tables of one form of the PCG may
+                                 take (default: no limit); a form whose tables cannot
+                                 be allocated is not used.  Set before the mesh's first
+                                 solve */
 } s4g_limit;
 s4g_status s4g_mesh_set_limit(s4g_mesh* mesh, s4g_limit which, long long value);
 

@@ -261,6 +261,8 @@ struct Engine {
   template <class T>
   s4g_status alloc(T** p, size_t n) {
     if (n == 0) n = 1;
+    if (planning && tableLimit > 0 && bytes - planBytes + n * sizeof(T) > (size_t)tableLimit)
+      return setErr(S4G_OOM, "the PCG's tables exceed the mesh's limit");
     cudaError_t e = cudaMalloc((void**)p, n * sizeof(T));
     if (e != cudaSuccess) return setErr(S4G_OOM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     allocs.push_back(*p);
@@ -272,6 +274,27 @@ struct Engine {
     s4g_status st = alloc(p, h.size());
     if (st != S4G_OK) return st;
     if (!h.empty()) S4G_CUDA(cudaMemcpyAsync(*p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, ctx->stream));
+    return S4G_OK;
+  }
+  // Makes the plan of a form of the PCG.  Where its tables cannot be allocated, what it
+  // holds is freed (undo drops the plan) and the mesh runs the other forms.
+  long long tableLimit = 0;  // S4G_LIMIT_TABLE_BYTES
+  bool planning = false;
+  size_t planBytes = 0;
+  template <typename P, typename U>
+  s4g_status planTables(P plan, U undo) {
+    const size_t mark = allocs.size();
+    planBytes = bytes;
+    planning = true;
+    s4g_status st = plan();
+    planning = false;
+    if (st != S4G_OOM) return st;
+    cudaGetLastError();
+    S4G_CUDA(cudaStreamSynchronize(ctx->stream));
+    for (size_t i = mark; i < allocs.size(); ++i) cudaFree(allocs[i]);
+    allocs.resize(mark);
+    bytes = planBytes;
+    undo();
     return S4G_OK;
   }
 #define S4G_TRY(x)                      \
@@ -686,9 +709,12 @@ struct Engine {
     if (ctx->profile || generalPcg || !residentForm<T>()) return S4G_OK;
     cudaStream_t s = ctx->stream;
     if (!q.tried) {
+      auto plan = [&]() -> s4g_status {
+        S4G_TRY(planResident<T>(q, true));
+        return q.ok ? S4G_OK : planResident<T>(q, false);
+      };
+      S4G_TRY(planTables(plan, [&] { q = Resident<T>(); }));
       q.tried = true;
-      S4G_TRY(planResident<T>(q, true));
-      if (!q.ok) S4G_TRY(planResident<T>(q, false));
     }
     const int pre = lin.preconditioner == S4G_PRECOND_DIC ? 0 : 1;
     if (!q.ok || (q.valid && q.precond == pre)) return S4G_OK;
@@ -902,8 +928,15 @@ struct Engine {
         (runsResident<T>() && hp.nC <= kResAheadRows))
       return S4G_OK;
     if (!q.tried) {
+      S4G_TRY(planTables([&] { return planParts<T>(q); },
+                         [&] {
+                           q = Parts<T>();
+                           if (sizeof(T) == 8) return;
+                           dHaloCnt = dHalo = nullptr;
+                           dSlot = nullptr;
+                           lp = LoopPtrs();
+                         }));
       q.tried = true;
-      S4G_TRY(planParts<T>(q));
     }
     // packets of a launch whose waits gave up may carry the tags of the next one
     if (lpStale) S4G_CUDA(cudaMemsetAsync(lp.w, 0, sizeof(uint4) * lpCount, ctx->stream));
@@ -2030,10 +2063,12 @@ struct Engine {
   }
 
   s4g_status setLimit(int which, long long value) {
-    if (value < 0 || value > INT_MAX) return setErr(S4G_BAD_ARG, "a limit must be >= 0");
+    if (value < 0 || (which != S4G_LIMIT_TABLE_BYTES && value > INT_MAX))
+      return setErr(S4G_BAD_ARG, "limit out of range");
     if (which == S4G_LIMIT_SWEEP_POLLS) mv.spinLimit = value ? (int)value : ctx->spinLimit;
     else if (which == S4G_LIMIT_PACKET_POLLS)
       mv.packetLimit = value ? (int)value : std::max(ctx->spinLimit, kSpinLimit);
+    else if (which == S4G_LIMIT_TABLE_BYTES) tableLimit = value;
     else return setErr(S4G_BAD_ARG, "unknown limit");
     ++generation;  // captured graphs hold the old view of the mesh
     return S4G_OK;

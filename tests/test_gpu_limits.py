@@ -66,3 +66,31 @@ def test_a_timed_out_part_loop_leaves_the_mesh_usable(ctx):
         assert st == _lib.NOT_CONVERGED and q["total_lin_iters"] == p["total_lin_iters"]
         assert np.array_equal(D, D2)
     model.close()
+
+
+@pytest.mark.parametrize("shape,kw,precision", [
+    ((12, 11, 10), dict(renumber="tiled"), "FP64"),
+    ((12, 11, 10), dict(renumber="tiled"), "FP32_REFINE"),
+    ((13, 11, 10), dict(blocks=8), "FP32_REFINE"),
+    ((28, 27, 26), dict(blocks=8), "FP32_REFINE"),
+    ((28, 27, 26), dict(blocks=8), "FP64"),
+    ((34, 33, 33), dict(part_size=16, dic_subdomains=True), "FP32_REFINE"),
+])
+def test_a_form_whose_tables_do_not_fit_is_not_used(ctx, shape, kw, precision):
+    """Tables that cannot be allocated leave the solve to the general kernels, with the
+    same results and no memory kept."""
+    kw = dict(kw)
+    if "blocks" in kw:
+        kw["parts"] = block_parts(*shape, kw.pop("blocks"))
+    general = _model(ctx, shape, precision, general_pcg=True, **kw)
+    st0, D0, p0 = _solve(general)
+    for limit in (1, 100_000):  # the first allocation, a later one
+        model = _model(ctx, shape, precision, **kw)
+        model.set_limit(_lib.LIMIT_TABLE_BYTES, limit)
+        st, D, p = _solve(model)
+        assert st == st0 == _lib.NOT_CONVERGED and np.array_equal(D, D0)
+        assert p["total_lin_iters"] == p0["total_lin_iters"]
+        assert p["kernel_launches"] >= 2 * p["total_lin_iters"] // 3  # launches per iteration
+        assert model.info()["device_bytes"] == general.info()["device_bytes"]
+        model.close()
+    general.close()
