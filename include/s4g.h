@@ -319,14 +319,16 @@ typedef struct s4g_perf {
   long long kernel_launches;  /* kernels launched by the library */
   int enforce_linear;         /* TL: linear geometry was enforced */
   int device_status;          /* raw device status word (0 = clean) */
-  int part_threads;           /* processor-local PCG: threads per part of the
-                                 preconditioner kernel in use (autotuned) */
-  int spmv_unroll;            /* processor-local PCG: SpMV form in use: entries
-                                 unrolled in the fused p-update + SpMV (1 or
-                                 6), or 0 for the split form */
-  double tune_us[6];          /* autotuner timings (us): the two
+  int part_threads;           /* processor-local PCG: threads per part of the general
+                                 preconditioner kernel's variant (autotuned); a mesh
+                                 that runs another form of the PCG does not use it */
+  int spmv_unroll;            /* processor-local PCG: SpMV form of the general kernels and
+                                 of FP64: entries unrolled in the fused p-update + SpMV
+                                 (1 or 6), or 0 for the split form */
+  double tune_us[6];          /* autotuner timings (us): the two general
                                  preconditioner variants, then the SpMV
-                                 step plain/unrolled/split; the rest 0 */
+                                 step plain/unrolled/split; 0 for what the mesh
+                                 does not run, and the rest */
   /* per kernel kind (S4G_K_*), only with s4g_ctx_opts.profile: summed
    * CUDA-event time and number of launches that did work */
   double kernel_ms[S4G_K_KINDS];

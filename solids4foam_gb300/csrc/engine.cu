@@ -1366,7 +1366,7 @@ struct Engine {
   LocalTuning& tuning() { return sizeof(T) == 4 ? tune32 : tune64; }
 
   // Autotuner of the fused processor-local iteration: times every variant of
-  // its two kernels on this mesh and keeps the fastest.  Each timed launch
+  // those of its two kernels that this mesh runs and keeps the fastest.  Each timed launch
   // starts from the same state (a scratch DevState reset before it, all
   // components active, one pending update) on zeroed vectors, so every
   // launch does the full work.  The vectors are reset by the corrector's
@@ -1376,6 +1376,7 @@ struct Engine {
   s4g_status tuneLocal(const Controls& c, const PcgPtrs<T>& p) {
     bool& done = sizeof(T) == 4 ? tuned32 : tuned64;
     if (runsResident<T>() || (sizeof(T) == 4 && runsParts<T>())) return S4G_OK;  // nothing to choose
+    const bool precond = !runsParts<T>();  // (FP64 part kernels: the product's form only)
     if (done || !autotune) { done = true; return S4G_OK; }
     cudaStream_t s = ctx->stream;
     const size_t n3 = 3 * (size_t)hp.nC;
@@ -1410,7 +1411,7 @@ struct Engine {
     };
     LocalTuning cand = t;
     int bestNT = 0;
-    for (int k = 0; k < kLocNumNT; ++k) {
+    for (int k = 0; k < kLocNumNT && precond; ++k) {
       cand.ntIdx = k;
       us[k] = timeIt([&] { launchLocalPrecond<T>(mv, c, p, dTune, dPartials, cand, s); });
       launches += 7;

@@ -94,3 +94,20 @@ def test_a_form_whose_tables_do_not_fit_is_not_used(ctx, shape, kw, precision):
         assert model.info()["device_bytes"] == general.info()["device_bytes"]
         model.close()
     general.close()
+
+
+@pytest.mark.parametrize("precision,general,timed", [
+    ("FP64", True, [True, True, True, True, True]),
+    ("FP64", False, [False, False, True, True, True]),   # part kernels: the product's forms
+    ("FP32_REFINE", False, [False] * 5),
+])
+def test_the_autotuner_times_what_the_mesh_runs(ctx, precision, general, timed):
+    """(general_pcg switches the autotuner off; the general kernels run here because the
+    part kernels' tables may not be allocated.)"""
+    model = _model(ctx, (13, 11, 10), precision, parts=block_parts(13, 11, 10, 8))
+    if general:
+        model.set_limit(_lib.LIMIT_TABLE_BYTES, 1)
+    st, _, p = _solve(model)
+    assert st == _lib.NOT_CONVERGED
+    assert [t > 0 for t in p["tune_us"][:5]] == timed
+    model.close()
