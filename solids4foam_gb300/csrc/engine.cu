@@ -150,6 +150,7 @@ struct Engine {
   PcgPtrs<float> pc32{};   // FP32 inner solve of the mixed-precision path
   bool fp32Allocated = false;
   bool fp32Valid = false;  // FP32 copies match the FP64 matrix/factor
+  bool general64Valid = false, general32Valid = false;  // (ensureGeneral)
   int sweepGrid32 = 1;
   // processor-local DIC path (subdomain runs with DIC)
   int nLoc = 0;
@@ -502,9 +503,6 @@ struct Engine {
       grids(tune32, per);
       autotune = !(o && o->no_autotune);
       S4G_TRY(alloc(&pc.p2, 3 * (size_t)nC));
-      double* lc;
-      S4G_TRY(alloc(&lc, (size_t)nLoc));
-      pc.lcoef = lc;
     }
     S4G_CUDA(cudaStreamSynchronize(s));
     // caller geometry is no longer needed
@@ -679,10 +677,6 @@ struct Engine {
       S4G_CUDA(cudaMemcpyAsync(dRD, dDiag, sizeof(double) * hp.nC, cudaMemcpyDeviceToDevice, s));
       launchDicFactor(mv, dVal, dDiag, dRD, dRDa, pc.flags[0], dState, sweepGrid, s);
       launches += 2;
-      if (mv.subdomains) {
-        launchLocalGather<double>(nLoc, dLocSrc, dRDa, const_cast<double*>(pc.lcoef), s);
-        launches++;
-      }
     } else {
       launchReciprocal(hp.nC, dDiag, dRD, s);  // diagonalPreconditioner: rD = 1/diag
       launches++;
@@ -694,6 +688,7 @@ struct Engine {
     matrixValid = true;
     matrixPrecond = pre;
     fp32Valid = false;
+    general64Valid = general32Valid = false;
     res64.valid = res32.valid = false;
     parts64.valid = parts32.valid = false;
     return S4G_OK;
@@ -1095,41 +1090,83 @@ struct Engine {
   bool batched = false;    // capturing this mesh's loop into a batch's graph
   bool batchLoop = false;  // (runsPartLoop)
 
-  // FP32 copies of the matrix, factor and work vectors (mixed precision).
+  // FP32 copies of the matrix' diagonal, the factor and the work vectors (mixed
+  // precision).
   s4g_status ensureFp32() {
-    const size_t nC = hp.nC, nE = 2 * (size_t)hp.nI;
+    const size_t nC = hp.nC;
     if (!fp32Allocated) {
-      float *val, *diag, *rD, *rDa;
-      S4G_TRY(alloc(&val, nE)); S4G_TRY(alloc(&diag, nC)); S4G_TRY(alloc(&rD, nC)); S4G_TRY(alloc(&rDa, nE));
-      pc32.val = val; pc32.diag = diag; pc32.rD = rD; pc32.rDa = rDa;
+      float *diag, *rD;
+      S4G_TRY(alloc(&diag, nC)); S4G_TRY(alloc(&rD, nC));
+      pc32.diag = diag; pc32.rD = rD;
       const size_t nv = 3 * nC * (size_t)caseCap;  // one vector per load case
       S4G_TRY(alloc(&pc32.x, nv)); S4G_TRY(alloc(&pc32.r, nv)); S4G_TRY(alloc(&pc32.w, nv));
       S4G_TRY(alloc(&pc32.p, nv)); S4G_TRY(alloc(&pc32.q, nv));
       pc32.flags[0] = pc.flags[0]; pc32.flags[1] = pc.flags[1];
       ++generation;
-      if (mv.subdomains) {
-        float* lc;
-        S4G_TRY(alloc(&pc32.p2, 3 * nC * (size_t)caseCap));
-        S4G_TRY(alloc(&lc, (size_t)nLoc));
-        pc32.lcoef = lc;
-      }
+      if (mv.subdomains) S4G_TRY(alloc(&pc32.p2, nv));
       fp32Allocated = true;
     }
     if (!fp32Valid) {
       cudaStream_t s = ctx->stream;
-      launchToFloat(nE, dVal, const_cast<float*>(pc32.val), s);
       launchToFloat(nC, dDiag, const_cast<float*>(pc32.diag), s);
       launchToFloat(nC, dRD, const_cast<float*>(pc32.rD), s);
-      launchToFloat(nE, dRDa, const_cast<float*>(pc32.rDa), s);
-      launches += 4;
-      if (mv.subdomains) {
-        launchLocalGather<float>(nLoc, dLocSrc, dRDa, const_cast<float*>(pc32.lcoef), s);
-        launches++;
-      }
+      launches += 2;
       S4G_CUDA(cudaGetLastError());
       fp32Valid = true;
     }
     return S4G_OK;
+  }
+
+  // What the general kernels of type T read and the other forms do not: the coefficients
+  // of the processor-local substitutions, in FP32 also the product's and the sweeps'.
+  template <typename T>
+  s4g_status ensureGeneral() {
+    const bool local = mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC;
+    if ((resident<T>().ok && residentForm<T>()) || (local && parts<T>().ok)) return S4G_OK;
+    cudaStream_t s = ctx->stream;
+    const size_t nE = 2 * (size_t)hp.nI;
+    PcgPtrs<T>* p;
+    if constexpr (sizeof(T) == 4) p = &pc32;
+    else p = &pc;
+    bool& valid = sizeof(T) == 4 ? general32Valid : general64Valid;
+    if (sizeof(T) == 4 && !p->val) {
+      T *val, *rDa;
+      S4G_TRY(alloc(&val, nE)); S4G_TRY(alloc(&rDa, nE));
+      p->val = val; p->rDa = rDa;
+      ++generation;
+    }
+    if (local && !p->lcoef) {
+      T* lc;
+      S4G_TRY(alloc(&lc, (size_t)nLoc));
+      p->lcoef = lc;
+      valid = false;
+      ++generation;
+    }
+    if (valid) return S4G_OK;
+    if constexpr (sizeof(T) == 4) {
+      launchToFloat(nE, dVal, const_cast<T*>(p->val), s);
+      launchToFloat(nE, dRDa, const_cast<T*>(p->rDa), s);
+      launches += 2;
+    }
+    if (local) {
+      launchLocalGather<T>(nLoc, dLocSrc, dRDa, const_cast<T*>(p->lcoef), s);
+      launches++;
+    }
+    S4G_CUDA(cudaGetLastError());
+    valid = true;
+    return S4G_OK;
+  }
+  // The forms of the PCG that this mesh runs in its precision.
+  s4g_status ensureForms() {
+    if (precision == S4G_FP32_REFINE) {
+      S4G_TRY(ensureFp32());
+      S4G_TRY(ensureResident<float>());
+      S4G_TRY(ensureParts<float>());
+      return ensureGeneral<float>();
+    }
+    S4G_TRY(ensureResident<double>());
+    S4G_TRY(ensureParts<double>());
+    return ensureGeneral<double>();
   }
 
   // Reads the device state of the nRun cases.  In a PCG loop (inPcg), the
@@ -1267,9 +1304,7 @@ struct Engine {
     S4G_TRY(ensureAitken());
     S4G_TRY(ensureMatrix());
     const bool mixed = precision == S4G_FP32_REFINE;
-    if (mixed) S4G_TRY(ensureFp32());
-    S4G_TRY(mixed ? ensureResident<float>() : ensureResident<double>());
-    S4G_TRY(mixed ? ensureParts<float>() : ensureParts<double>());
+    S4G_TRY(ensureForms());
     {
       const Controls ct = controls(0);
       if (mixed) S4G_TRY(tuneLocal<float>(ct, pc32));
@@ -1708,9 +1743,7 @@ struct Engine {
     stepLive = false;
     S4G_TRY(ensureMatrix());
     const bool mixed = precision == S4G_FP32_REFINE;
-    if (mixed) S4G_TRY(ensureFp32());
-    S4G_TRY(mixed ? ensureResident<float>() : ensureResident<double>());
-    S4G_TRY(mixed ? ensureParts<float>() : ensureParts<double>());
+    S4G_TRY(ensureForms());
     cudaEvent_t e0, e1;
     S4G_CUDA(cudaEventCreate(&e0));
     S4G_CUDA(cudaEventCreate(&e1));
@@ -1840,9 +1873,7 @@ struct Engine {
     S4G_TRY(ensureAitken());
     S4G_TRY(ensureMatrix());
     const bool mixed = precision == S4G_FP32_REFINE;
-    if (mixed) S4G_TRY(ensureFp32());
-    S4G_TRY(mixed ? ensureResident<float>() : ensureResident<double>());
-    S4G_TRY(mixed ? ensureParts<float>() : ensureParts<double>());
+    S4G_TRY(ensureForms());
     if (mv.subdomains && lin.preconditioner == S4G_PRECOND_DIC) {
       const Controls ct = controls(0);
       if (mixed) S4G_TRY(tuneLocal<float>(ct, pc32));

@@ -94,7 +94,9 @@ namespace {
 // addressing and geometry, FP64 fields and matrix, PCG work vectors, the
 // FP32 copies of the mixed-precision path, the processor-local DIC tables
 // and the total Lagrangian fields -- the allocations of s4g_mesh_upload
-// and s4g_solve, rounded up.
+// and s4g_solve, rounded up.  (The tables of the PCG's forms take the place of those the
+// general kernels read; held against the device bytes of every form at 10^3 to 64^3
+// cells: 6 % too many at least, FP64 exact DIC inside one CTA, and 32 % at most.)
 long long estimateFootprint(const Request& r) {
   const double N = r.nCells, F = r.nInternal, B = (double)r.nFaces - r.nInternal;
   double b = 0;
@@ -102,7 +104,6 @@ long long estimateFootprint(const Request& r) {
   b += N * (8 * 3 + 24 * 3 + 72 + 48 + 72) + F * (48) + B * (24 + 72 + 48 + 24);
   b += N * 24 * 6;
   if (r.precision == S4G_FP32_REFINE) b += N * (8 + 12 * 6) + F * 16;
-  b += N * 240;  // the PCG's own tables (cluster-resident or by part)
   if (r.meshOpts.dic_subdomains) b += F * 2 * 18 + N * 8;
   if (r.model != S4G_LIN_GEOM_TOTAL_DISP) b += N * (72 * 6 + 48 + 8) + B * (72 * 6 + 48 + 8);
   return (long long)(b * 1.15) + (16ll << 20);

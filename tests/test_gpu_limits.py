@@ -1,6 +1,7 @@
 """Error paths of the solves, made on the host through a mesh's limits: waits that run
 out, tables that cannot be allocated."""
 import ctypes as ct
+import time
 
 import numpy as np
 import pytest
@@ -111,3 +112,34 @@ def test_the_autotuner_times_what_the_mesh_runs(ctx, precision, general, timed):
     assert st == _lib.NOT_CONVERGED
     assert [t > 0 for t in p["tune_us"][:5]] == timed
     model.close()
+
+
+@pytest.mark.parametrize("precision", ["FP64", "FP32_REFINE"])
+@pytest.mark.parametrize("n,kw", [
+    (24, dict(blocks=8)), (32, dict(blocks=8)), (24, dict(part_size=16, dic_subdomains=True)),
+    (20, dict(renumber="tiled")), (24, dict(renumber="tiled", diagonal=True)),
+])
+def test_a_request_is_booked_with_what_its_mesh_holds(ctx, n, kw, precision):
+    """The server's footprint covers the device bytes of the form that runs, and is not
+    more than 1.4 times them (and a fixed 16 MB)."""
+    kw = dict(kw)
+    solver = dict(preconditioner="diagonal") if kw.pop("diagonal", False) else {}
+    if "blocks" in kw:
+        kw["parts"] = block_parts(n, n, n, kw.pop("blocks"))
+    m = sg.box_mesh(n, n, n, 1.0, 0.9, 0.8, 0.2, 4)
+    law = dict(type="linearElastic", E=70e9, nu=0.3)
+    bcs = {"zmin": ("fixedDisplacement", None, None), "zmax": ("solidTraction", [0, 0, -1e5], None)}
+    args = dict(solver=solver, outer=dict(nCorrectors=2), precision=precision)
+    model = sg.SolidModel(ctx, m, law, {"zmin": bcs["zmin"]}, **args, **kw)
+    _solve(model)
+    held = model.info()["device_bytes"]
+    model.close()
+    srv = sg.Server(max_slots=1, memory_budget=1 << 36, dry_run=True, dry_run_us_per_kcell=2e4)
+    rid = srv.submit(m, law, bcs, **args, **kw)
+    t0 = time.time()
+    while srv.stats()["running"] == 0 and time.time() - t0 < 10:
+        time.sleep(0.001)
+    booked = srv.stats()["bytes_in_use"]
+    assert srv.result(rid)[0] == _lib.OK
+    srv.close()
+    assert held <= booked <= 1.4 * held + (16 << 20)
