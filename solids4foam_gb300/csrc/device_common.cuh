@@ -262,10 +262,12 @@ __device__ __forceinline__ double trS(const S6& s) { return s.xx + s.yy + s.zz; 
 __device__ __forceinline__ double trT(const T9& t) { return t.xx + t.yy + t.zz; }
 // x / 3, correctly rounded, in three operations instead of a division (some
 // fifteen FP64 ones): the product with the rounded reciprocal, corrected by its
-// exact remainder (Markstein 1990).
+// exact remainder (Markstein 1990).  Of a zero (the correction would lose its sign) and
+// of what is not finite: the product.
 __device__ __forceinline__ double third(double x) {
   const double y = 1.0 / 3.0, q = __dmul_rn(x, y), r = __fma_rn(-3.0, q, x);
-  return isfinite(x) ? __fma_rn(r, y, q) : q;
+  const bool zero = ((__double2hiint(x) & 0x7fffffff) | __double2loint(x)) == 0;
+  return isfinite(x) && !zero ? __fma_rn(r, y, q) : q;
 }
 __device__ __forceinline__ S6 devS(const S6& s) {
   double m = trS(s) / 3.0;

@@ -1,6 +1,6 @@
 """third() of the field kernels (x / 3 by a product and its remainder), compiled for the
 host from its source, against the division: the same bits for any x, subnormal,
-infinite and NaN ones among them."""
+infinite, NaN and negative zero among them."""
 import os
 import re
 import subprocess
@@ -16,6 +16,9 @@ MAIN = r"""
 #include <cstring>
 using std::isfinite;
 static double __dmul_rn(double a, double b) { return a * b; }
+static uint64_t bits(double x) { uint64_t b; std::memcpy(&b, &x, 8); return b; }
+static int __double2hiint(double x) { return (int)(bits(x) >> 32); }
+static int __double2loint(double x) { return (int)bits(x); }
 static double __fma_rn(double a, double b, double c) { return std::fma(a, b, c); }
 %s
 int main() {
