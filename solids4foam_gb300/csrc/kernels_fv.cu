@@ -192,6 +192,21 @@ __device__ __forceinline__ V3 tractionSnGrad(const MeshView& mv, const Controls&
   return c.rImpK * ((t - p * nc) - dotVS(nc, sb) + c.impK * dotVT(n, Gb));
 }
 
+// tractionSnGrad of the linear model in the pass over boundary faces.  Traction and pressure
+// load are explicitly rounded: t - (p n), p n rounded first.  (Left to the compiler, the
+// product is contracted with the subtraction in some kernels and not in others, and a last
+// bit of the gradient reaches 4e-9 of D after 60 correctors.)
+__device__ __forceinline__ V3 tractionSnGradLinear(const MeshView& mv, const Controls& c, int b,
+                                                   const S6& sb, const T9& Gb) {
+  const V3 v = ldV(mv.bval, b), n = ldV(mv.bn, b);
+  const double p = c.loadFactor * mv.bpress[b];
+  const V3 load = {__fma_rn(c.loadFactor, v.x, -__dmul_rn(p, n.x)),
+                   __fma_rn(c.loadFactor, v.y, -__dmul_rn(p, n.y)),
+                   __fma_rn(c.loadFactor, v.z, -__dmul_rn(p, n.z))};
+  T9 a = fromS(sb) - c.impK * Gb;
+  return c.rImpK * (load - dotVT(n, a));
+}
+
 // Relaxed update of the traction gradient (solidTraction...C:387-392):
 // g = f g_new + (1 - f) g_old; f = 1 leaves g_new as it is.
 __device__ __forceinline__ V3 relaxG(const MeshView& mv, int b, V3 gNew, V3 gOld) {
@@ -508,7 +523,7 @@ kPostFace(MeshView mv, Controls c, FieldPtrs f, DevState* st, double* partials, 
       if (mode == 1) stS(f.sigb, b, sb);
       if (mv.btype[b] == 1) {
         stV(f.gPrev, b, sg);
-        stV(f.g, b, relaxG(mv, b, tractionSnGrad(mv, c, b, sb, Gb, nullptr, 0), sg));
+        stV(f.g, b, relaxG(mv, b, tractionSnGradLinear(mv, c, b, sb, Gb), sg));
       }
     } else if (mode == 1) {
       T9 GDb = ldT(f.GD0b, b) + Gb;
