@@ -574,17 +574,22 @@ __device__ __forceinline__ bool loopPartTotal(const uint4* rec, int n, double* g
                return part < n ? rec + (size_t)(i % 4) * n + part : (const uint4*)nullptr;
              },
              tag, limit, x) && ok;
+    double v[A][8], s[A];
+#pragma unroll
+    for (int u = 0; u < A; ++u) {
+      const uint4 *const y = x + 4 * u;
+      const double d[6] = {wordsValue(y[0].x, y[0].y), wordsValue(y[0].z, y[1].x), wordsValue(y[1].y, y[1].z),
+                           wordsValue(y[2].x, y[2].y), wordsValue(y[2].z, y[3].x), wordsValue(y[3].y, y[3].z)};
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[u][k] = k < 6 ? d[k < 6 ? k : 0] : 0.0;
+    }
+    warpSpreadSums<8, A>(v, s);
 #pragma unroll
     for (int u = 0; u < A; ++u) {
       const int g = g0 + u * W;
-      if (g >= nGrp) break;
-      const uint4 *const y = x + 4 * u;
-      double v[8] = {wordsValue(y[0].x, y[0].y), wordsValue(y[0].z, y[1].x), wordsValue(y[1].y, y[1].z),
-                     wordsValue(y[2].x, y[2].y), wordsValue(y[2].z, y[3].x), wordsValue(y[3].y, y[3].z), 0, 0};
-      const double s = warpSpreadSum<8>(v);
-      if ((lane & 3) == 0 && lane < 24) {
+      if ((lane & 3) == 0 && lane < 24 && g < nGrp) {
         double* const o = grp + 6 * (g & 63) + (lane >> 2);
-        *o = g < 64 ? s : *o + s;
+        *o = g < 64 ? s[u] : *o + s[u];
       }
     }
   }

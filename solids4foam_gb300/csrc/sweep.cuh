@@ -464,13 +464,11 @@ __device__ __forceinline__ void warpFloatSums(const float (&x)[N][3], double (&s
 }
 
 // Sum over the lanes below n (the others hold zero), in lane 0: blockSum's tree without
-// its steps that add zeros.
+// its steps that add zeros (a loop: unrolled, they would be added and dropped).
 __device__ __forceinline__ double warpTree(double v, int n = 32) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const double x = __shfl_down_sync(0xffffffffu, v, o);
-    if (o < n) v += x;
-  }
+#pragma unroll 1
+  for (int o = n > 32 ? 16 : n > 1 ? 1 << (31 - __clz(n - 1)) : 0; o > 0; o >>= 1)
+    v += __shfl_down_sync(0xffffffffu, v, o);
   return v;
 }
 
