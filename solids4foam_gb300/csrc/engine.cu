@@ -1068,11 +1068,8 @@ struct Engine {
     if (sizeof(T) == 8 || !mv.subdomains || lin.preconditioner != S4G_PRECOND_DIC) return false;
     return hp.nC > kResAheadRows && (nRun > 1 || batched ? parts32.ok : parts32.loop);
   }
-  // The forms it has.  In FP64 the exact DIC only, whose sums it adds in the
-  // separate kernels' order: the corrector loop can amplify a last bit of a sum
-  // over many correctors.  (FP64 processor-local and diagonal runs of small meshes
-  // keep the separate kernels: their ordered sums in the cluster would take most
-  // of what its one launch saves.)
+  // The forms it has: in FP64 the exact DIC only.  (The others would need their ordered
+  // sums in FP64, as it has them in FP32; what they would give is not measured.)
   template <typename T>
   bool residentForm() const {
     const bool dic = lin.preconditioner == S4G_PRECOND_DIC;

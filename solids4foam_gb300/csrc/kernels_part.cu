@@ -40,8 +40,9 @@ namespace {
 template <typename T> struct PartCfg;
 template <> struct PartCfg<float> {
   using Ent = PartEnt;
-  // (8 resident CTAs at 123 registers; 6 at 139 before: 128^3 61.4 -> 60.1 us a
-  // launch, 16 cases of 40^3 39.4 -> 35.5; fewer rows a thread keeps: 65 and 70 us)
+  // (8 resident CTAs at 119 registers; with 6 at 139 a launch at 128^3 took 61.4 us for
+  // 60.1, 16 cases of 40^3 39.4 for 35.5; with fewer rows a thread keeps 65 and 70 us.
+  // The sums' order came after these: 128^3 68.1 us)
   static constexpr int kNT = 64, kKeep = 8, kOcc = 7;
   static constexpr bool kSplit = false;
 };
@@ -426,7 +427,8 @@ kPartSpmv(MeshView mv, PartView pv, PartPtrs<float> pt, PcgPtrs<float> p, const 
 
 // p.q of the product, in the order of kLocSpmv: a thread the storage rows of the row
 // kernels' grid, blocks of 256 threads, then the blocks.  (In the product itself the
-// rows are by part.)  Reads q and p_new, in good part from L2 right after the product.
+// rows are by part.)  Reads q and p_new.  128^3: 20 us, 50 MB from DRAM; 64^3: 11 us,
+// the latency of its chain (state, rows, block sums, the last block's total, alpha).
 __global__ void __launch_bounds__(kRowBlock)
 kPartDot(MeshView mv, PcgPtrs<float> p, DevState* st, double* partials) {
   p = casePcg(p, blockIdx.y, mv.nC);

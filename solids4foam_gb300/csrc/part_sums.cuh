@@ -1,6 +1,5 @@
 // Sums of the processor-local preconditioner over the parts, in an order that
-// depends on the part count only (kernels_local.cu, and kernels_part.cu in
-// FP64).
+// depends on the part count only (kernels_local.cu, kernels_part.cu).
 #pragma once
 
 #include "device_common.cuh"
